@@ -180,6 +180,14 @@ int64_t jja_plan_device_bytes(const jja_plan* p);
  * mx * my entries): the face (original order) at grid cell (ix, iy); mx + 1 and my + 1 powers of
  * two up to 1024. The caller checks that K has that form. jja_solve_static keeps the sweeps. */
 int jja_plan_set_fast_poisson(jja_plan* p, int mx, int my, const int32_t* grid_face, double kappa);
+
+/* The same solve with the sine transforms as tensor-core contractions (error-free digit products, FP64
+ * results) along one axis of the grid and tridiagonal solves along the other: for plans of many
+ * problems. K = kappa (4 I - adjacency) on an mx x my grid of faces of any size whose shorter side
+ * has at most 128 faces; grid_face[iy * mx + ix] is the face at (ix, iy) in the caller's order.
+ * Replaces the plan's triangular sweeps (jja_solve_static keeps them). Not on a plan that already solves
+ * by sine transforms. */
+int jja_plan_set_sine_solver(jja_plan* p, int mx, int my, const int32_t* grid_face, double kappa);
 /* Synchronises the device, then reads and clears the plan's device error flags: *flow_timeouts
  * = 1 if a wait of a dataflow sweep ran out of its bound since the last call (the results of
  * those steps are invalid), else 0. Returns JJA_ERR_NONFINITE when a time step of jja_run /

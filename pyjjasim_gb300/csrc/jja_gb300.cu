@@ -11,6 +11,7 @@
 #include "../../include/jja_gb300.h"
 #include "jja_internal.h"
 
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1598,6 +1599,12 @@ __global__ void k_permute_rows(const double* __restrict__ src, double* __restric
   }
 }
 
+}  // namespace
+
+#include "jja_sine.cuh"
+
+namespace {
+
 int grid_for(int64_t n, int threads) {
   int64_t g = (n + threads - 1) / threads;
   return (int)std::max<int64_t>(1, std::min<int64_t>(g, 152LL * 32));
@@ -2072,6 +2079,20 @@ struct FaceTables {
   int deg = 0;
 };
 
+// the fixed-degree copy of the face -> junction codes, when every face has at most kEllMax
+void fill_ell(FaceTables& ft, int Nf) {
+  ft.deg = 0;
+  for (int pn = 0; pn < Nf; ++pn) ft.deg = std::max<int>(ft.deg, (int)(ft.fj_ptr[pn + 1] - ft.fj_ptr[pn]));
+  if (ft.deg >= 1 && ft.deg <= kEllMax) {
+    ft.ell.assign((size_t)Nf * ft.deg, -1);
+    for (int pn = 0; pn < Nf; ++pn)
+      for (int64_t i = ft.fj_ptr[pn]; i < ft.fj_ptr[pn + 1]; ++i)
+        ft.ell[(size_t)pn * ft.deg + (i - ft.fj_ptr[pn])] = ft.fj_col[i];
+  } else {
+    ft.deg = 0;
+  }
+}
+
 FaceTables face_tables(int Nj, int Nf, const int64_t* a_rowptr, const int32_t* a_col, const double* a_val,
                        const std::vector<int>& perm) {
   if (Nj >= (1 << 30) || Nf >= (1 << 30)) throw Error(JJA_ERR_ARG, "too many junctions or faces");
@@ -2095,15 +2116,7 @@ FaceTables face_tables(int Nj, int Nf, const int64_t* a_rowptr, const int32_t* a
     }
     ft.fj_ptr[pn + 1] = (int64_t)ft.fj_col.size();
   }
-  for (int pn = 0; pn < Nf; ++pn) ft.deg = std::max<int>(ft.deg, (int)(ft.fj_ptr[pn + 1] - ft.fj_ptr[pn]));
-  if (ft.deg >= 1 && ft.deg <= kEllMax) {
-    ft.ell.assign((size_t)Nf * ft.deg, -1);
-    for (int pn = 0; pn < Nf; ++pn)
-      for (int64_t i = ft.fj_ptr[pn]; i < ft.fj_ptr[pn + 1]; ++i)
-        ft.ell[(size_t)pn * ft.deg + (i - ft.fj_ptr[pn])] = ft.fj_col[i];
-  } else {
-    ft.deg = 0;
-  }
+  fill_ell(ft, Nf);
   return ft;
 }
 
@@ -2242,6 +2255,11 @@ struct jja_plan {
   int dst = 0;
   int dst_lines = 0;   // grid lines per block of the sine-transform kernels (0: by grid size)
   DstArgs dst_args{};
+  // sine transforms on the tensor cores (jja_plan_set_sine_solver; dst == 2): first transform,
+  // tridiagonal solves, transform back; face vectors in grid order
+  SineArgs sine_fwd{}, sine_bwd{};
+  SineTri sine_tri{};
+  int32_t* perm_factor = nullptr;    // the factor's face order, when perm is the grid's
   std::vector<int32_t> iperm_host;   // original face -> factor's face order
   int64_t bytes = 0;
   // captured graphs of a fixed-length step sequence, keyed by the buffers they bake in (a few
@@ -2465,8 +2483,28 @@ void launch_levels(jja_plan* p, const Group& g, cudaStream_t st, bool forward) {
 }
 
 
-// x = K^-1 b for group g: the two triangular sweeps, or the three sine-transform kernels
+// the sine-transform solve on the tensor cores: b -> z (transform), in place (tridiagonal), -> x
+void launch_sine_solve(jja_plan* p, const Group& g, cudaStream_t st) {
+  auto lines = [&](SineArgs d, const double* in, double* out) {
+    const int64_t tiles = ((int64_t)d.lines * g.wn + kSineColumns - 1) / kSineColumns;
+    d.parts = sine_parts(d.kp, tiles);
+    const unsigned grid = (unsigned)(d.parts * std::min<int64_t>(tiles, kNumSMs / d.parts));
+    launch_smem(p->pdl, sine_kernel(d.kp), dim3(grid), kSineThreads, sine_smem_bytes(d.kp), st, d, in, out, g.w0, g.wn,
+                p->flow_err);
+  };
+  const SineTri& t = p->sine_tri;
+  const unsigned tri = (unsigned)(((int64_t)t.lines * g.wn + kTriColumns - 1) / kTriColumns);
+  lines(p->sine_fwd, p->b, p->z);
+  launch_smem(p->pdl, k_sine_tri, dim3(tri), 2 * kTriColumns, 0, st, t, p->z, g.w0, g.wn);
+  lines(p->sine_bwd, p->z, p->x);
+}
+
+// x = K^-1 b for group g: the two triangular sweeps, or sine transforms
 void launch_face_solve(jja_plan* p, const Group& g, cudaStream_t st) {
+  if (p->dst == 2) {
+    launch_sine_solve(p, g, st);
+    return;
+  }
   if (!p->dst) {
     launch_levels(p, g, st, true);
     launch_levels(p, g, st, false);
@@ -2995,6 +3033,7 @@ int jja_plan_set_fast_poisson(jja_plan* p, int mx, int my, const int32_t* grid_f
     if (!p || !grid_face || mx < 1 || my < 1) throw Error(JJA_ERR_ARG, "jja_plan_set_fast_poisson: bad arguments");
     if ((int64_t)mx * my != p->Nf) throw Error(JJA_ERR_ARG, "jja_plan_set_fast_poisson: mx * my != Nf");
     if (!(kappa > 0.0)) throw Error(JJA_ERR_ARG, "jja_plan_set_fast_poisson: kappa must be positive");
+    if (p->dst == 2) throw Error(JJA_ERR_ARG, "jja_plan_set_fast_poisson: the plan solves by jja_plan_set_sine_solver");
     auto log2_of = [](int n) {   // log2(2 n) for n a power of two (n = m + 1), else -1
       if (n < 2 || (n & (n - 1))) return -1;
       int l = 1;
@@ -3049,6 +3088,104 @@ int jja_plan_set_fast_poisson(jja_plan* p, int mx, int my, const int32_t* grid_f
     p->graphs.clear();
     p->adj_graphs.clear();
     p->dst = 1;
+  });
+}
+
+int jja_plan_set_sine_solver(jja_plan* p, int mx, int my, const int32_t* grid_face, double kappa) {
+  return guarded([&] {
+    if (!p || !grid_face || mx < 1 || my < 1) throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: bad arguments");
+    if ((int64_t)mx * my != p->Nf) throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: mx * my != Nf");
+    if (!(kappa > 0.0) || !std::isfinite(kappa))
+      throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: kappa must be positive and finite");
+    if (std::min(mx, my) > kSineMaxPoints)
+      throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: the shorter side must have at most 128 faces");
+    if (p->dst) throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: the plan already solves by sine transforms");
+    const int Nf = p->Nf, W = p->W;
+    // the tables again with the faces in grid order: cell iy * mx + ix
+    std::vector<int32_t> cell_of(Nf, -1);   // the factor's face -> grid cell
+    for (int c = 0; c < Nf; ++c) {
+      const int f = grid_face[c];
+      if (f < 0 || f >= Nf || cell_of[p->iperm_host[f]] >= 0)
+        throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: grid_face is not a permutation");
+      cell_of[p->iperm_host[f]] = c;
+    }
+    FaceTables ft;
+    {
+      std::vector<int64_t> ptr((size_t)Nf + 1);
+      JJA_CUDA(cudaMemcpy(ptr.data(), p->t.fj_ptr, ptr.size() * sizeof(int64_t), cudaMemcpyDeviceToHost));
+      std::vector<int32_t> col((size_t)ptr[Nf]);
+      JJA_CUDA(cudaMemcpy(col.data(), p->t.fj_col, col.size() * sizeof(int32_t), cudaMemcpyDeviceToHost));
+      ft.jf_face.resize(2 * (size_t)p->Nj);
+      JJA_CUDA(cudaMemcpy(ft.jf_face.data(), p->t.jf_face, ft.jf_face.size() * sizeof(int32_t), cudaMemcpyDeviceToHost));
+      for (int32_t& v : ft.jf_face)
+        if (v >= 0) v = (cell_of[v >> 1] << 1) | (v & 1);
+      ft.face_orig.assign(grid_face, grid_face + Nf);
+      std::vector<int32_t> face_at(Nf);
+      for (int f = 0; f < Nf; ++f) face_at[cell_of[f]] = f;
+      ft.fj_ptr.assign(1, 0);
+      for (int c = 0; c < Nf; ++c) {
+        const int f = face_at[c];
+        ft.fj_col.insert(ft.fj_col.end(), col.begin() + ptr[f], col.begin() + ptr[f + 1]);
+        ft.fj_ptr.push_back((int64_t)ft.fj_col.size());
+      }
+      fill_ell(ft, Nf);
+    }
+    // transforms along x (lines are grid rows) when the rows are the shorter side or both fit and
+    // rows keep the tridiagonal chains' loads contiguous for few problems; else along y
+    const bool along_x = mx <= my || mx <= kSineMaxPoints;
+    const int m = along_x ? mx : my, n = along_x ? my : mx;
+    const int kp = (m - m / 2 + 15) / 16 * 16;
+    const int64_t sx = W, sy = (int64_t)mx * W;
+    SineArgs d{};
+    d.m = m;
+    d.kp = kp;
+    d.lines = n;
+    d.s_t = along_x ? sx : sy;
+    d.s_c = along_x ? sy : sx;
+    int e = 0;
+    const long double scale = frexpl(2.0L / ((long double)(m + 1) * kappa), &e);   // in [1/2, 1) 2^e
+    const std::vector<uint16_t> plain = sine_matrix(m, kp, 1.0L), scaled = sine_matrix(m, kp, scale);
+    // the tridiagonal factors, eliminated from either end (the chain is symmetric)
+    SineTri t{};
+    t.n = n;
+    t.lines = m;
+    t.top = n / 2;
+    t.s_n = d.s_c;
+    t.s_c = d.s_t;
+    const int longest = n - t.top;
+    std::vector<double> c((size_t)longest * m), g(2 * (size_t)m);
+    const long double pi_l = 3.141592653589793238462643383279502884L;
+    for (int k = 0; k < m; ++k) {
+      const long double s = sinl(pi_l * (k + 1) / (2.0L * (m + 1)));
+      const long double diag = 2.0L + 4.0L * s * s;
+      long double r = 0.0L, ctop = 0.0L;
+      for (int i = 0; i < longest; ++i) {
+        r = 1.0L / (diag - r);
+        c[(size_t)i * m + k] = (double)r;
+        if (i == t.top - 1) ctop = r;
+      }
+      g[k] = (double)(ctop / (1.0L - ctop * r));
+      g[(size_t)m + k] = (double)(r / (1.0L - ctop * r));
+    }
+    set_face_tables(p->t, ft, [&](auto* h, size_t n) { return p->up(h, n); });
+    p->perm_factor = p->perm;
+    p->perm = p->up(grid_face, (size_t)Nf);
+    t.c = p->up(c.data(), c.size());
+    t.g = p->up(g.data(), g.size());
+    d.mat = reinterpret_cast<const unsigned char*>(p->up(plain.data(), plain.size()));
+    d.e_shift = 0;
+    p->sine_fwd = d;
+    d.mat = reinterpret_cast<const unsigned char*>(p->up(scaled.data(), scaled.size()));
+    d.e_shift = e;
+    p->sine_bwd = d;
+    p->sine_tri = t;
+    JJA_CUDA(cudaFuncSetAttribute(sine_kernel(kp), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sine_smem_bytes(kp)));
+    // graphs captured before bake in the sweeps: drop them
+    for (auto& g2 : p->graphs) cudaGraphExecDestroy(g2.exec);
+    for (auto& g2 : p->adj_graphs) cudaGraphExecDestroy(g2.exec);
+    p->graphs.clear();
+    p->adj_graphs.clear();
+    p->dst = 2;
   });
 }
 
@@ -3197,12 +3334,13 @@ int jja_solve_static(jja_plan* p, const double* b, double* x, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     double* bx = static_scratch_for_current_device(st);   // permuted right-hand side, later the solution
     double* z = bx + NfW;                                // forward-substitution result
+    const int32_t* perm = p->perm_factor ? p->perm_factor : p->perm;   // the sweeps' face order
     // every element of both work vectors is written before it is read: nothing to clear
-    k_permute_rows<<<grid_for(NfW, 256), 256, 0, st>>>(b, bx, p->perm, p->Nf, p->W, 1);
+    k_permute_rows<<<grid_for(NfW, 256), 256, 0, st>>>(b, bx, perm, p->Nf, p->W, 1);
     g_launches++;
     launch_levels_into(p, st, true, bx, z, nullptr);
     launch_levels_into(p, st, false, nullptr, z, bx);
-    k_permute_rows<<<grid_for(NfW, 256), 256, 0, st>>>(bx, x, p->perm, p->Nf, p->W, 0);
+    k_permute_rows<<<grid_for(NfW, 256), 256, 0, st>>>(bx, x, perm, p->Nf, p->W, 0);
     g_launches++;
     JJA_CUDA(cudaGetLastError());
   });

@@ -137,11 +137,24 @@ class HostFactor:
             self.handle = None
 
 
-def fast_poisson_grid(circuit, K):
+def poisson_grid(circuit, K):
     """(mx, my, grid_face, kappa) when the face-space matrix is K = kappa (4 I - adjacency) on an
-    mx x my grid of faces with mx + 1 and my + 1 powers of two (up to 1024): a square array with
-    equal R and C and a uniform self-inductance, whose K is kappa times the 5-point Laplacian with
-    Dirichlet boundaries. Checked entry by entry (relative 1e-12); None otherwise."""
+    mx x my grid of faces: a square array with equal R and C and a uniform self-inductance, whose K
+    is kappa times the 5-point Laplacian with Dirichlet boundaries. Checked entry by entry (relative
+    1e-12); None otherwise."""
+    # the diagonal and the entries first: most circuits fail there, without their geometry
+    diag = K.diagonal()
+    kappa = float(diag[0]) / 4.0
+    if not kappa > 0.0:
+        return None
+    tol = 1e-12 * kappa
+    if np.abs(diag - 4.0 * kappa).max() > tol:
+        return None
+    Kc = scipy.sparse.coo_matrix(K)
+    off = Kc.row != Kc.col
+    r, c, v = Kc.row[off], Kc.col[off], Kc.data[off]
+    if np.abs(v + kappa).max(initial=0.0) > tol:
+        return None
     try:
         cx, cy = circuit.get_face_centroids()
     except Exception:
@@ -150,27 +163,24 @@ def fast_poisson_grid(circuit, K):
     ux, ix = np.unique(np.round(np.asarray(cx, np.float64), 9), return_inverse=True)
     uy, iy = np.unique(np.round(np.asarray(cy, np.float64), 9), return_inverse=True)
     mx, my = len(ux), len(uy)
-    if mx * my != Nf or any(m + 1 > 1024 or (m + 1) & m for m in (mx, my)):
+    if mx * my != Nf:
         return None
     grid = np.full(mx * my, -1, np.int64)
     grid[iy * mx + ix] = np.arange(Nf)
     if np.any(grid < 0):
         return None
-    Kc = scipy.sparse.coo_matrix(K)
-    kappa = float(K.diagonal()[0]) / 4.0
-    if not kappa > 0.0:
-        return None
-    tol = 1e-12 * kappa
-    if np.abs(K.diagonal() - 4.0 * kappa).max() > tol:
-        return None
-    off = Kc.row != Kc.col
-    r, c, v = Kc.row[off], Kc.col[off], Kc.data[off]
     neighbour = (np.abs(ix[r] - ix[c]) + np.abs(iy[r] - iy[c])) == 1
-    if not np.all(neighbour) or np.abs(v + kappa).max(initial=0.0) > tol:
+    if not np.all(neighbour):
         return None
     if np.count_nonzero(np.abs(v) > tol) != 2 * (mx * (my - 1) + my * (mx - 1)):
         return None
     return mx, my, np.ascontiguousarray(grid, np.int32), kappa
+
+
+def fast_poisson_grid(circuit, K):
+    """``poisson_grid`` for the radix-2 transforms: mx + 1 and my + 1 powers of two, up to 1024."""
+    g = poisson_grid(circuit, K)
+    return None if g is None or any(m + 1 > 1024 or (m + 1) & m for m in g[:2]) else g
 
 
 # "auto" uses the sine transforms for at most this many problems and face-problems (W x Nf). Measured
@@ -181,10 +191,29 @@ FAST_POISSON_MAX_W = 8
 FAST_POISSON_MAX_WORK = 1 << 18
 
 
+# The tensor-core transforms work on tiles of 128 (grid line, problem) columns, one tile per SM at
+# a time, on grids whose shorter side has at most 128 faces (SINE_MAX_SIDE).
+SINE_MAX_SIDE = 128
+SINE_MIN_COLUMNS = 512
+
+
+def sine_solver_fits(grid, W):
+    """Whether "auto" takes the tensor-core sine transforms for W problems on this poisson_grid."""
+    mx, my = grid[:2]
+    return min(mx, my) <= SINE_MAX_SIDE and min(mx, my) >= 8 and max(mx, my) * W >= SINE_MIN_COLUMNS
+
+
+def untuned(tuning):
+    """True when ``tuning`` asks for nothing but the level schedule (the library's default)."""
+    t = dict(tuning or {})
+    return int(t.pop("schedule", 0)) in (0, 1) and not any(int(v) for v in t.values())
+
+
 class DevicePlan:
     """Circuit tables + factor uploaded for W problems (owned C object)."""
 
-    def __init__(self, circuit, factor, A, W, dt, stencil_width, stencil, Ic_w=None, tuning=None, fast_poisson=None):
+    def __init__(self, circuit, factor, A, W, dt, stencil_width, stencil, Ic_w=None, tuning=None, fast_poisson=None,
+                 sine=None):
         """``tuning``: dict with any of rhs_block, rows_per_lane, target_warps, min_piece (the
         launch shape of the triangular solves; missing or 0 = library default)."""
         Nj, Nf = circuit._Nj(), circuit._Nf()
@@ -222,6 +251,12 @@ class DevicePlan:
             self._keep["grid"] = grid
             N.check(N.lib().jja_plan_set_fast_poisson(h, int(mx), int(my), N.ptr(grid, ctypes.c_int32), float(kappa)))
             self.fast_poisson = True
+        self.sine = False
+        if sine is not None:
+            mx, my, grid, kappa = sine
+            self._keep["grid"] = grid
+            N.check(N.lib().jja_plan_set_sine_solver(h, int(mx), int(my), N.ptr(grid, ctypes.c_int32), float(kappa)))
+            self.sine = True
         self.device_bytes = N.lib().jja_plan_device_bytes(h)
 
     def solve(self, b_dev, x_dev, stream=0):
@@ -303,8 +338,9 @@ def fill_reducing_order(K, ordering, circuit=None):
     raise ValueError(f"ordering must be 'nd' or 'mmd', not {ordering!r}")
 
 
-def get_factor(circuit, dt, nd_leaf=8, ordering="nd", relax=(-1, -1.0)):
-    A, K = face_matrix(circuit, dt)
+def get_factor(circuit, dt, nd_leaf=8, ordering="nd", relax=(-1, -1.0), matrices=None):
+    """(factor, A, cache key); ``matrices``: face_matrix(circuit, dt) when the caller has it."""
+    A, K = face_matrix(circuit, dt) if matrices is None else matrices
     key = (_digest(K.indptr, K.indices, K.data), nd_leaf, ordering, tuple(relax))
     with _CACHE_LOCK:
         hit = _FACTORS.get(key)
@@ -326,27 +362,35 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
     ``ordering`` "nd", "mmd" or "auto" (see resolve_ordering); ``nd_leaf`` None: by the step's
     size (see resolve_factor_shape); ``tuning`` the launch shape of the triangular solves (see
     DevicePlan); ``fast_poisson``: solve with sine transforms when the face-space matrix allows it
-    (fast_poisson_grid): True, False, or "auto" (W <= 8 and W x Nf <= 2^18 face-problems)."""
+    (fast_poisson_grid): True, False, or "auto" (W <= 8 and W x Nf <= 2^18 face-problems; the
+    tensor-core transforms by sine_solver_fits)."""
     ordering = resolve_ordering(ordering, W, circuit._Nf())
     nd_leaf, relax = resolve_factor_shape(nd_leaf, relax, ordering, W, circuit._Nf())
     fp = None
+    matrices = face_matrix(circuit, dt)
     if fast_poisson is True or (fast_poisson == "auto" and W <= FAST_POISSON_MAX_W
                                 and W * circuit._Nf() <= FAST_POISSON_MAX_WORK):
-        fp = fast_poisson_grid(circuit, face_matrix(circuit, dt)[1])
-    factor, A, fkey = get_factor(circuit, dt, nd_leaf, ordering=ordering, relax=relax)
+        fp = fast_poisson_grid(circuit, matrices[1])
+    sine = None
+    if fp is None and fast_poisson == "auto" and W * circuit._Nf() >= SINE_MIN_COLUMNS and untuned(tuning):
+        sine = poisson_grid(circuit, matrices[1])
+        if sine is not None and not sine_solver_fits(sine, W):
+            sine = None
+    factor, A, fkey = get_factor(circuit, dt, nd_leaf, ordering=ordering, relax=relax, matrices=matrices)
     Rv, Cv, coef = coefficients(circuit, dt, stencil)
     if Ic_w is not None:
         Ic_w = np.ascontiguousarray(np.broadcast_to(np.asarray(Ic_w, np.float64), (circuit._Nj(), W)))
     ic = np.asarray(circuit._Ic(), np.float64) if Ic_w is None else Ic_w
     tkey = tuple(int((tuning or {}).get(f, 0)) for f in TUNING_FIELDS)
-    key = (fkey, W, stencil_width, Ic_w is None, tkey, fp is not None,
+    key = (fkey, W, stencil_width, Ic_w is None, tkey, fp is not None, sine is not None,
            _digest(ic, *coef, Rv, A.indptr, A.indices, A.data))
     with _CACHE_LOCK:
         p = _PLANS.get(key)
         if p is not None:
             _PLANS.move_to_end(key)
             return p
-    p = DevicePlan(circuit, factor, A, W, dt, stencil_width, stencil, Ic_w=Ic_w, tuning=tuning, fast_poisson=fp)
+    p = DevicePlan(circuit, factor, A, W, dt, stencil_width, stencil, Ic_w=Ic_w, tuning=tuning, fast_poisson=fp,
+                   sine=sine)
     with _CACHE_LOCK:
         _PLANS[key] = p
         while len(_PLANS) > MAX_PLANS:
