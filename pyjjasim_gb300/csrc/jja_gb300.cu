@@ -139,8 +139,30 @@ __device__ __forceinline__ double view_at(const jja_view& v, int64_t n, int64_t 
   return v.ptr ? __ldg(v.ptr + n * v.stride_n + w * v.stride_w + tt * v.stride_t) : 0.0;
 }
 
+// Division of an element index by a count fixed at launch: one multiplication below 2^31 (a 64-bit
+// division is about 100 integer instructions, as many as the rest of an elementwise kernel).
+struct FastDiv {
+  uint32_t d = 1, mul = 0;   // quotient = (i mul) >> (32 + shift), mul = ceil(2^(32 + shift) / d); mul = 0: d = 1
+  int shift = 0;
+  __device__ __forceinline__ int64_t operator()(int64_t i) const {
+    if (i < (1ll << 31)) return mul ? __umulhi((uint32_t)i, mul) >> shift : (uint32_t)i;
+    return i / d;
+  }
+};
+
+// 2^(shift) < d <= 2^(shift + 1): the multiplier has 32 bits and is exact for i < 2^31
+FastDiv fast_div(int d) {
+  FastDiv f;
+  f.d = (uint32_t)d;
+  if (d <= 1) return f;
+  while ((2ll << f.shift) < d) ++f.shift;
+  f.mul = (uint32_t)(((1ull << (32 + f.shift)) + f.d - 1) / f.d);
+  return f;
+}
+
 struct StepArgs {
   int Nj, Nf, W, width;
+  FastDiv by_wn;
   int w0, wn;          // the launch steps problems [w0, w0 + wn) of the W in the arrays (a group)
   const double* h[4];
   double* hout;
@@ -160,6 +182,7 @@ struct StepArgs {
   double e[4];
   double dt;
   jja_view Isq;        // Is / c0 for a time-independent Is (plan-owned, refreshed at the start of a run)
+  const double* amp;   // sqrt(2 T Rv) / c0 per junction, for a time-independent T equal for all problems (likewise)
   int resistive;       // width 3 and no capacitance anywhere: c1 / c0 = -1, c2 = 0
 };
 
@@ -177,7 +200,7 @@ struct Tables {
   const int32_t* fj_ell;   // faces of <= kEllMax junctions: Nf x face_deg codes, padded with -1
   int face_deg;            // 0 when some face has more than kEllMax junctions (CSR path)
   const int32_t* jf_face;  // 2 per junction: (permuted face << 1) | (A entry is -1), or -1
-  const longlong2* sincos; // per k < 65536: {S, C} = {sin, cos}(k pi/32768) in units of 2^-62
+  const longlong2* sincos; // per k < 65536: {S, C} = {sin, cos}(k pi/32768) in units of 2^-62, lower halves signed
   int* nonfinite;          // set to 1 by k_update when a new phase is NaN or +-inf (read by jja_plan_check)
 };
 
@@ -192,30 +215,32 @@ __device__ __forceinline__ double signed_by(double v, int neg) {
 }
 
 // ------------------------------------------------------------------------------------------
-// sin(x) and cos(x) to FP64 accuracy without FP64 instructions. GB300's FP64 pipe is ~60x
-// narrower than its FP32 and integer pipes, and the junction kernels are bound by it; this
-// evaluation runs on the integer pipe (64-bit fixed point) with an FP32 correction term.
+// sin(x) and cos(x) to FP64 accuracy without FP64 instructions. GB300's FP64 pipe does 2
+// operations per clock and SM (a warp's FP64 instruction takes 64 cycles of its scheduler, an
+// integer multiply-add or logic instruction 1-2), and the junction kernels are bound by it; this
+// evaluation runs on the integer pipes in fixed point, in 32 x 32-bit products.
 // Table-driven method (Tang, ACM TOMS 15(2), 1989) with an exact Payne-Hanek style reduction:
-// 1. |x| = M 2^(e-1075) exactly (M: the 53-bit significand). u = |x| 2^15/pi is formed as M times
-//    2^15/pi held to 128 bits (kInvPiHi:kInvPiLo = floor(2^129/pi), computed to 400 bits with
-//    mpmath), keeping 64 fractional bits of u and the low bits of its integer part (error
-//    < |x| 2^-114 in u: below 2^-70 for the phases' range, 2^-52 at |x| = 2^62). k = nearest
-//    integer to u, f = u - k in [-1/2, 1/2], t = f pi/2^15 (|t| <= 4.8e-5) as a signed 64-bit
-//    number in units of 2^-76 (kPi61 = round(pi 2^61)).
+// 1. |x| = M 2^(e-1075) exactly (M: the 53-bit significand). u = |x| 2^15/pi is formed from M times
+//    1/(2 pi) held to 96 bits (|x| < 2^20; to 128 bits in sin_reduce_wide), keeping 64
+//    fractional bits of u and the low 16 bits of its integer part (error below 2^-59 in u).
+//    k = nearest integer to u, f = u - k in [-1/2, 1/2], t = f pi/2^15 (|t| <= 4.8e-5) as a signed
+//    64-bit number in units of 2^-76 (kPi61 = round(pi 2^61)).
 // 2. With S, C = sin, cos(k pi/32768) from a 65536-entry table in units of 2^-62 (1 MB,
 //    L2-resident, computed on the host in extended precision):
 //      sin(|x|) = S + C t - S t^2/2 - C t^3/6,   cos(x) = C - S t - C t^2/2 + S t^3/6,
-//    remainder below 3e-19. S + C t and the quadratic term are formed in fixed point (64x64-bit
-//    products), the cubic term (< 1.9e-14) in FP32 (absolute error < 2e-21).
+//    remainder below 3e-19. C t is formed from 32-bit halves (the table's and t's lower halves
+//    are signed, so every product is a signed 32 x 32 one), and so is the quadratic term from t^2;
+//    the cubic term (< 1.9e-14) to 20 bits.
 // 3. The fixed-point sum (absolute error ~1e-18) is rounded to the nearest double with integer
-//    operations (count of leading zeros, shift, round half to even).
+//    operations (count of leading zeros, shift).
 // |x| < 2^-27 gives sin = x, cos = 1 (the next terms are below half an ulp); |x| >= 2^62, inf
-// and NaN give NaN. No library call: the kernels keep no stack frame for one. Host and device
-// share this code, so the library can check it on the CPU (jja_sin_host).
+// and NaN give NaN. Host and device share this code, so the library can check it on the CPU
+// (jja_sin_host).
 // ------------------------------------------------------------------------------------------
 constexpr int kSinTable = 65536;
 constexpr uint64_t kInvPiHi = 0xa2f9836e4e441529ull;   // floor(2^15/pi 2^114) = kInvPiHi 2^64 + kInvPiLo
 constexpr uint64_t kInvPiLo = 0xfc2757d1f534ddc0ull;
+constexpr uint32_t kTurn0 = 0x28be60dbu, kTurn1 = 0x9391054au, kTurn2 = 0x7f09d5f4u;   // 1/(2 pi) to 96 bits
 constexpr int64_t kPi61 = 0x6487ed5110b4611all;       // round(pi 2^61)
 
 __host__ __device__ __forceinline__ uint64_t umulhi64(uint64_t a, uint64_t b) {
@@ -223,14 +248,6 @@ __host__ __device__ __forceinline__ uint64_t umulhi64(uint64_t a, uint64_t b) {
   return __umul64hi(a, b);
 #else
   return (uint64_t)(((unsigned __int128)a * b) >> 64);
-#endif
-}
-
-__host__ __device__ __forceinline__ int64_t smulhi64(int64_t a, int64_t b) {
-#ifdef __CUDA_ARCH__
-  return __mul64hi(a, b);
-#else
-  return (int64_t)(((__int128)a * b) >> 64);
 #endif
 }
 
@@ -254,46 +271,35 @@ __host__ __device__ __forceinline__ double double_of(uint64_t b) {
 #endif
 }
 
-__host__ __device__ __forceinline__ float float_of_int(int v) {
-#ifdef __CUDA_ARCH__
-  return __int2float_rn(v);
-#else
-  return (float)v;
-#endif
-}
+__host__ __device__ __forceinline__ int mulhi32(int a, int b) { return (int)(((int64_t)a * b) >> 32); }
 
-// f 2^62 truncated to an integer, for |f| < 2^-28 (the cubic terms)
-__host__ __device__ __forceinline__ int64_t fixed62_of_float(float f) {
-  uint32_t b;
-#ifdef __CUDA_ARCH__
-  b = __float_as_uint(f);
-#else
-  memcpy(&b, &f, 4);
-#endif
-  const int E = (int)((b >> 23) & 0xffu);
-  const int64_t m = (int64_t)((b & 0x7fffffu) | 0x800000u);
-  const int sh = E - 88;   // f 2^62 = m 2^(E - 150 + 62)
-  const int64_t v = E == 0 ? 0 : sh >= 0 ? (m << sh) : (sh > -64 ? (m >> -sh) : 0);
-  return (b >> 31) ? -v : v;
-}
-
-// R 2^-62 rounded to the nearest double, negated when `neg`
+// R 2^-62 rounded to the nearest double (half up in magnitude), negated when `neg`; |R| < 2^63
 __host__ __device__ __forceinline__ double double_of_fixed62(int64_t R, bool neg) {
-  const bool sign = (R < 0) != neg;
-  const uint64_t a = R < 0 ? (uint64_t)0 - (uint64_t)R : (uint64_t)R;
-  if (a == 0) return double_of((uint64_t)neg << 63);
+  const int64_t m = R >> 63;
+  const uint64_t a = (uint64_t)((R ^ m) - m);
+  uint32_t h = (uint32_t)(a >> 32), l = (uint32_t)a;
+  int top = 1024 - 2;                   // biased exponent - 2 of a leading bit at position 62 + 1
+  if (h == 0) {                         // |value| < 2^-30
+    h = l >> 2;
+    l = l << 30;
+    top -= 30;
+  }
+  if (h == 0) {                         // |value| < 2^-60: at most two bits are left
+    h = l;
+    l = 0;
+    top -= 32;
+    if (h == 0) return double_of((uint64_t)neg << 63);
+  }
 #ifdef __CUDA_ARCH__
-  const int lz = __clzll((long long)a);
+  const int sh = __clz((int)h) - 1;
+  uint64_t n = ((uint64_t)__funnelshift_l(l, h, sh) << 32) | (l << sh);
 #else
-  const int lz = __builtin_clzll(a);
+  const int sh = __builtin_clz(h) - 1;
+  uint64_t n = (((uint64_t)h << 32) | l) << sh;
 #endif
-  const uint64_t n = a << lz;                     // leading one at bit 63
-  uint64_t mant = n >> 11;                        // 53 bits
-  const uint64_t rem = n & 0x7ffu;
-  mant += (rem > 0x400u) || (rem == 0x400u && (mant & 1u));
-  // value in [2^(1-lz), 2^(2-lz)): biased exponent 1024 - lz; a carry out of the rounding
-  // moves into the exponent field
-  return double_of((((uint64_t)(1023 - lz) << 52) + mant) | ((uint64_t)sign << 63));
+  n = (n + 0x200u) >> 10;               // leading bit at position 62: the rounding cannot overflow
+  // the leading one (or a carry beyond it) adds to the exponent field
+  return double_of((n + ((uint64_t)(uint32_t)((top - sh) * (1 << 20)) << 32)) | ((uint64_t)((m != 0) != neg) << 63));
 }
 
 struct SinReduced {
@@ -311,8 +317,19 @@ __host__ __device__ __forceinline__ uint64_t bits_at(uint64_t P0, uint64_t P1, u
   return (P0 >> pos) | (P1 << (64 - pos));
 }
 
+// the nearest table index and t, from u = kint + frac 2^-64
+__host__ __device__ __forceinline__ SinReduced sin_split(uint32_t kint, uint64_t frac) {
+  SinReduced r;
+  const int fh = (int)(frac >> 32);
+  r.idx = (kint + ((uint32_t)fh >> 31)) & (unsigned)(kSinTable - 1);   // round to nearest
+  // t 2^76 = f 2^64 pi 2^61 2^-64
+  const int low = mulhi32(fh, (int)(kPi61 & 0xffffffff)) + (int)(((frac & 0xffffffffu) * (uint64_t)(kPi61 >> 32)) >> 32);
+  r.t = (int64_t)fh * (int)(kPi61 >> 32) + low;
+  return r;
+}
+
 // step 1 for 2^-27 <= |x| < 2^62 (biased exponent e in [996, 1084])
-__host__ __device__ __forceinline__ SinReduced sin_reduce(uint64_t ax) {
+__host__ __device__ __forceinline__ SinReduced sin_reduce_wide(uint64_t ax) {
   const int e = (int)(ax >> 52);
   const uint64_t M = (ax & 0xfffffffffffffull) | (1ull << 52);
   // P = M (kInvPiHi 2^64 + kInvPiLo), 181 bits
@@ -323,32 +340,71 @@ __host__ __device__ __forceinline__ SinReduced sin_reduce(uint64_t ax) {
   // u 2^64 = P 2^(e - 1125): fraction = bits [sh, sh + 64) of P, integer part above (only its
   // low 16 bits index the table)
   const int sh = 1125 - e;   // 41 .. 129
-  const uint64_t frac = bits_at(P0, P1, P2, sh);
-  const uint64_t kint = bits_at(P0, P1, P2, sh + 64);
-  SinReduced r;
-  r.idx = (unsigned)(kint + (frac >> 63)) & (unsigned)(kSinTable - 1);   // round to nearest
-  r.t = smulhi64((int64_t)frac, kPi61);   // f 2^64 pi 2^61 2^-64 = t 2^76
-  return r;
+  return sin_split((uint32_t)bits_at(P0, P1, P2, sh + 64), bits_at(P0, P1, P2, sh));
 }
 
-// steps 2 and 3: sin(|x|) and cos(x) from the reduction and the table entry {S, C} (2^-62
-// units). t^2 is formed in units of 2^-88; the cubic term (< 1.9e-14) in FP32.
+// 2^-27 <= |x| < 2^20 (biased exponent in [996, 1042]), from the bits of x
+__host__ __device__ __forceinline__ bool sin_usual(uint64_t xb) {
+  return ((uint32_t)(xb >> 52) & 0x7ffu) - 996u <= 46u;
+}
+
+// step 1 for those, from the bits of x (the sign is ignored)
+__host__ __device__ __forceinline__ SinReduced sin_reduce(uint64_t xb) {
+  const int e = (int)((uint32_t)(xb >> 52) & 0x7ffu);
+  const uint32_t m0 = (uint32_t)xb, m1 = ((uint32_t)(xb >> 32) & 0xfffffu) | 0x100000u;
+  // P = M (kTurn0 2^64 + kTurn1 2^32 + kTurn2), words 1 to 4 (word 0 leaves a carry below 2^-60 of u)
+  const uint64_t t1 = (uint64_t)m0 * kTurn1 + (((uint64_t)m0 * kTurn2) >> 32);
+  const uint64_t s1 = (uint64_t)m1 * kTurn2 + (uint32_t)t1;
+  const uint64_t t2 = (uint64_t)m0 * kTurn0 + (t1 >> 32) + ((uint64_t)m1 * kTurn1 + (s1 >> 32));
+  const uint64_t t3 = (uint64_t)m1 * kTurn0 + (t2 >> 32);
+  // u 2^64 = |x| / (2 pi) 2^80 = P 2^(e - 1091)
+  const int sh = 1059 - e;   // 17 .. 63, from word 1
+  const bool up = sh >= 32;
+  const uint32_t w1 = up ? (uint32_t)t2 : (uint32_t)s1, w2 = up ? (uint32_t)t3 : (uint32_t)t2;
+  const uint32_t w3 = up ? (uint32_t)(t3 >> 32) : (uint32_t)t3, w4 = up ? 0u : (uint32_t)(t3 >> 32);
+#ifdef __CUDA_ARCH__
+  return sin_split(__funnelshift_r(w3, w4, sh), ((uint64_t)__funnelshift_r(w2, w3, sh) << 32) | __funnelshift_r(w1, w2, sh));
+#else
+  const int q = sh & 31;
+  auto fun = [&](uint32_t l, uint32_t h) { return (uint32_t)((((uint64_t)h << 32) | l) >> q); };
+  return sin_split(fun(w3, w4), ((uint64_t)fun(w2, w3) << 32) | fun(w1, w2));
+#endif
+}
+
+// hi 2^32 + lo with a signed lower half, so that products of halves are signed 32 x 32 ones. The
+// table's words are stored that way; split_word makes the halves of any other word.
+struct Halves {
+  int hi, lo;
+};
+__host__ __device__ __forceinline__ Halves table_word(long long v) { return {(int)(v >> 32), (int)v}; }
+__host__ __device__ __forceinline__ Halves split_word(int64_t v) {
+  return {(int)(v >> 32) + (int)((uint32_t)v >> 31), (int)v};
+}
+
+// a b 2^-64 to within 2^-31 (2^-32 of its last place), in 2^-32 units of it
+__host__ __device__ __forceinline__ int64_t mul_halves(Halves a, Halves b, int64_t round) {
+  const int64_t cross = (int64_t)a.hi * b.lo + (int64_t)a.lo * b.hi;
+  return (int64_t)a.hi * b.hi + ((cross >> 32) + round);
+}
+
+// steps 2 and 3: S + C t - S t^2/2 - C t^3/6 (2^-62 units) from table words S and C
+__host__ __device__ __forceinline__ int64_t sin_series(int64_t t, Halves S, Halves C) {
+  const Halves th = split_word(t);
+  const int64_t ct = mul_halves(C, th, 1 << 11) >> 12;          // 2^-74 units, rounded to 2^-62
+  const int64_t t2 = (int64_t)th.hi * th.hi + (((int64_t)(2 * th.hi) * th.lo) >> 32);   // 2^-88 units
+  const Halves q = split_word(t2);
+  const int64_t st2 = mul_halves(S, q, 1 << 24) >> 25;          // S t^2 / 2
+  const int c3 = mulhi32(mulhi32(mulhi32(q.hi, th.hi), C.hi), 715827883);   // C t^3 / 6 (2^32 / 6), 2^-66 units
+  return ((int64_t)S.hi * (1ll << 32) + S.lo) + ct - st2 - ((c3 + 8) >> 4);
+}
+
 __host__ __device__ __forceinline__ int64_t sin_fixed(const SinReduced& r, longlong2 sc) {
-  const int64_t ct = (smulhi64(sc.y, r.t) + (1 << 11)) >> 12;         // C t
-  const int64_t t2 = smulhi64(r.t, r.t);                               // t^2 2^88
-  const int64_t st2 = (smulhi64(sc.x, t2) + (1 << 24)) >> 25;          // S t^2 / 2
-  const float tf = float_of_int((int)(r.t >> 32)) * 0x1p-44f, cf = float_of_int((int)(sc.y >> 32)) * 0x1p-30f;
-  const float cubic = (-(1.0f / 6.0f) * cf) * (tf * tf * tf);          // -C t^3/6
-  return sc.x + ct - st2 + fixed62_of_float(cubic);
+  return sin_series(r.t, table_word(sc.x), table_word(sc.y));
 }
 
+// C - S t - C t^2/2 + S t^3/6: the same series of -t with the words exchanged
 __host__ __device__ __forceinline__ int64_t cos_fixed(const SinReduced& r, longlong2 sc) {
-  const int64_t st = (smulhi64(sc.x, r.t) + (1 << 11)) >> 12;         // S t
-  const int64_t t2 = smulhi64(r.t, r.t);
-  const int64_t ct2 = (smulhi64(sc.y, t2) + (1 << 24)) >> 25;          // C t^2 / 2
-  const float tf = float_of_int((int)(r.t >> 32)) * 0x1p-44f, sf = float_of_int((int)(sc.x >> 32)) * 0x1p-30f;
-  const float cubic = ((1.0f / 6.0f) * sf) * (tf * tf * tf);           // S t^3/6
-  return sc.y - st - ct2 + fixed62_of_float(cubic);
+  return sin_series(-r.t, table_word(sc.y), table_word(sc.x));
 }
 
 __host__ __device__ __forceinline__ longlong2 sin_table_entry(const longlong2* tab, unsigned idx) {
@@ -364,11 +420,19 @@ __host__ __device__ __forceinline__ bool sin_outside_range(uint64_t ax) { return
 __host__ __device__ __forceinline__ bool sin_tiny(uint64_t ax) { return ax < (996ull << 52); }   // |x| < 2^-27
 constexpr uint64_t kNaNBits = 0x7ff8000000000000ull;
 
-__host__ __device__ __forceinline__ double fast_sin(double x, const longlong2* __restrict__ tab) {
+// sine of the arguments outside [2^-27, 2^20) (rare: a call keeps it out of the kernels' registers)
+__host__ __device__ __noinline__ double sin_rare(double x, const longlong2* tab) {
   const uint64_t xb = bits_of(x), ax = xb & 0x7fffffffffffffffull;
   if (sin_outside_range(ax)) return double_of(kNaNBits);
   if (sin_tiny(ax)) return x;
-  const SinReduced r = sin_reduce(ax);
+  const SinReduced r = sin_reduce_wide(ax);
+  return double_of_fixed62(sin_fixed(r, sin_table_entry(tab, r.idx)), (xb >> 63) != 0);
+}
+
+__host__ __device__ __forceinline__ double fast_sin(double x, const longlong2* __restrict__ tab) {
+  const uint64_t xb = bits_of(x);
+  if (!sin_usual(xb)) return sin_rare(x, tab);
+  const SinReduced r = sin_reduce(xb);
   return double_of_fixed62(sin_fixed(r, sin_table_entry(tab, r.idx)), (xb >> 63) != 0);
 }
 
@@ -384,7 +448,7 @@ __host__ __device__ __forceinline__ void fast_sincos(double x, const longlong2* 
     c_out = 1.0;
     return;
   }
-  const SinReduced r = sin_reduce(ax);
+  const SinReduced r = sin_usual(xb) ? sin_reduce(xb) : sin_reduce_wide(ax);
   const longlong2 sc = sin_table_entry(tab, r.idx);
   s_out = double_of_fixed62(sin_fixed(r, sc), (xb >> 63) != 0);
   c_out = double_of_fixed62(cos_fixed(r, sc), false);
@@ -422,21 +486,30 @@ __device__ __forceinline__ double junction_q(const StepArgs& a, const Tables& t,
   const double isq = a.Isq.ptr ? view_at(a.Isq, j, w) : view_at(a.Is, j, w, tt) * __ldg(t.inv_c0 + j);
   if (a.noise_mode == JJA_NOISE_NONE)
     return a.Is.ptr ? X - isq : X;   // (0 - Is) + X in the reference
-  const double T = view_at(a.T, j, w, tt);
+  const double amp = a.amp ? __ldg(a.amp + j) : sqrt(2.0 * view_at(a.T, j, w, tt) * __ldg(t.Rvq + j));
   const double xi = a.noise_mode == JJA_NOISE_BUFFER ? a.noise[e] : philox_normal(a.seed, (uint64_t)e, (uint64_t)step);
-  const double fl = sqrt(2.0 * T * __ldg(t.Rvq + j)) * xi;
+  const double fl = amp * xi;
   return (fl - isq) + X;
 }
 
 // Isq = Is / c0 per junction, refreshed at the start of every run (and every host-driven step)
 __global__ void __launch_bounds__(256) k_scale_sources(jja_view Is, const double* __restrict__ inv_c0,
-                                                       double* __restrict__ Isq, int Nj, int W) {
+                                                       double* __restrict__ Isq, int Nj, int W, FastDiv by_W) {
   pdl_begin();
   const int64_t NjW = (int64_t)Nj * W;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < NjW; e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t j = e / W, w = e - j * W;
+    const int64_t j = by_W(e), w = e - j * W;
     Isq[e] = view_at(Is, j, w) * __ldg(inv_c0 + j);
   }
+}
+
+// noise amplitudes sqrt(2 T Rv) / c0 per junction (a square root is a dozen FP64 instructions, more
+// than the rest of a step's FP64 work per junction)
+__global__ void __launch_bounds__(256) k_noise_amp(jja_view T, const double* __restrict__ Rvq, double* __restrict__ amp,
+                                                   int Nj) {
+  pdl_begin();
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < Nj; j += gridDim.x * blockDim.x)
+    amp[j] = sqrt(2.0 * view_at(T, j, 0) * __ldg(Rvq + j));
 }
 
 // q for the first step of a run, from the stored phase history
@@ -445,7 +518,7 @@ __global__ void __launch_bounds__(256) k_junction(StepArgs a, Tables t, double* 
   const int64_t n = (int64_t)a.Nj * a.wn;
   const int64_t step = a.d_step[0], tt = step - a.d_step[2];
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t j = i / a.wn, w = a.w0 + (i - j * a.wn), e = j * a.W + w;
+    const int64_t j = a.by_wn(i), w = a.w0 + (i - j * a.wn), e = j * a.W + w;
     double th[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) th[k] = (k < a.width - 1) ? a.h[k][e] : 0.0;
@@ -471,7 +544,7 @@ __global__ void __launch_bounds__(256) k_face_rhs(StepArgs a, Tables t, const do
   const int64_t n = (int64_t)a.Nf * a.wn;
   const int64_t step = a.d_step[0], tt = step - a.d_step[2];
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = i / a.wn, w = a.w0 + (i - p * a.wn), e = p * a.W + w;
+    const int64_t p = a.by_wn(i), w = a.w0 + (i - p * a.wn), e = p * a.W + w;
     double acc = 0.0;
     if (t.face_deg) {
       // fixed-degree layout: all index loads, then all value loads, then the sum
@@ -520,7 +593,7 @@ __global__ void __launch_bounds__(256, JJA_UPDATE_MIN_BLOCKS) k_update(StepArgs 
   const int64_t next_step = a.d_step[1];            // published by this step's k_face_rhs
   const int64_t tt = next_step - 1 - a.d_step[2];   // source slot of the step being finished
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t j = i / a.wn, w = a.w0 + (i - j * a.wn), e = j * a.W + w;
+    const int64_t j = a.by_wn(i), w = a.w0 + (i - j * a.wn), e = j * a.W + w;
     // y = A^T J: a junction lies on one or two faces; the +-1 entries are sign flips
     const int p0 = __ldg(t.jf_face + 2 * j), p1 = __ldg(t.jf_face + 2 * j + 1);
     double y = p0 >= 0 ? signed_by(J[(int64_t)(p0 >> 1) * a.W + w], p0 & 1) : 0.0;
@@ -543,6 +616,108 @@ __global__ void __launch_bounds__(256, JJA_UPDATE_MIN_BLOCKS) k_update(StepArgs 
     if (kFuseNext) q[e] = junction_q(a, t, e, j, w, hist, next_step, tt + 1);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) a.d_step[0] = next_step;
+}
+
+// k_update<true> for the usual steps: stencil width 3, no voltage sources, time-independent
+// current sources, and no noise or Philox noise of an amplitude table; V adjacent problems per
+// thread. The general kernel spends 380 instructions per element, mostly on strided views and
+// 64-bit index arithmetic; this one shares them between the V problems (two 16-byte loads per
+// array). Measured per step: 128x128 x 512 0.301 -> 0.193 ms, 1024x1024 x 8 with C, L and noise
+// 0.721 -> 0.290 ms (there the amplitude table saves the FP64 square root). Bound by the latency of
+// three dependent reads (face numbers, face currents, sine table) at 32 warps per SM, with the FP64
+// pipe 75 % busy; 5 or 6 blocks per SM (fewer registers) and a thread per pair without the grid
+// loop measured the same.
+template <bool kCap, bool kNoise, int V>
+__global__ void __launch_bounds__(256, V == 1 ? 6 : 4) k_update_fast(StepArgs a, Tables t, double* __restrict__ q,
+                                                                    const double* __restrict__ J) {
+  pdl_begin();
+  struct alignas(8 * V) Vec {
+    double v[V];
+  };
+  const int64_t n = (int64_t)a.Nj * (a.wn / V);
+  const int64_t next_step = a.d_step[1];   // published by this step's k_face_rhs
+  double* th_out = a.store_all && a.th_out ? a.th_out + (next_step - 1 - a.d_step[3]) * ((int64_t)a.Nj * a.W) : nullptr;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t j = a.by_wn(i);   // divides by wn / V
+    const int w = a.w0 + (int)(i - j * (a.wn / V)) * V;
+    const int64_t e = j * a.W + w;
+    const int2 p = __ldg(reinterpret_cast<const int2*>(t.jf_face) + j);
+    const Vec qv = *reinterpret_cast<const Vec*>(q + e), h0 = *reinterpret_cast<const Vec*>(a.h[0] + e);
+    Vec y{}, J1{}, isq{};
+    if (p.x >= 0) y = *reinterpret_cast<const Vec*>(J + (int64_t)(p.x >> 1) * a.W + w);
+    if (p.y >= 0) J1 = *reinterpret_cast<const Vec*>(J + (int64_t)(p.y >> 1) * a.W + w);
+    if (a.Isq.ptr) isq = *reinterpret_cast<const Vec*>(a.Isq.ptr + e);
+    const double ic0 = __ldg(t.inv_c0 + j);
+    double icq[V], c0 = 0.0, c1 = 0.0, amp = 0.0;
+#pragma unroll
+    for (int u = 0; u < V; ++u) icq[u] = __ldg(t.Icq + (t.ic_per_w ? e + u : j));
+    if (kCap) {
+      c0 = __ldg(t.coefq + j);
+      c1 = __ldg(t.coefq + a.Nj + j);
+    }
+    if (kNoise) amp = __ldg(a.amp + j);
+    Vec th, qn;
+#pragma unroll
+    for (int u = 0; u < V; ++u) {
+      double s = p.x >= 0 ? signed_by(y.v[u], p.x & 1) : 0.0;
+      if (p.y >= 0) s += signed_by(J1.v[u], p.y & 1);
+      th.v[u] = fma(s, ic0, -qv.v[u]);
+      if (non_finite(th.v[u])) *t.nonfinite = 1;
+      const double sn = fast_sin(fma(2.0, th.v[u], -h0.v[u]), t.sincos);
+      double X;
+      if (kCap) X = fma(c1, h0.v[u], fma(c0, th.v[u], icq[u] * sn));
+      else X = fma(icq[u], sn, -th.v[u]);
+      if (kNoise) {
+        const double xi = philox_normal(a.seed, (uint64_t)(e + u), (uint64_t)next_step);
+        qn.v[u] = fma(amp, xi, -isq.v[u]) + X;
+      } else {
+        qn.v[u] = a.Isq.ptr ? X - isq.v[u] : X;
+      }
+    }
+    *reinterpret_cast<Vec*>(a.hout + e) = th;
+    *reinterpret_cast<Vec*>(q + e) = qn;
+    if (th_out) *reinterpret_cast<Vec*>(th_out + e) = th;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.d_step[0] = next_step;
+}
+
+// b = A q - 2 pi f for faces of at most kEllMax junctions without voltage sources and with a flux
+// that does not change with time, V adjacent problems per thread (see k_face_rhs, k_update_fast)
+template <int V>
+__global__ void __launch_bounds__(256) k_face_rhs_fast(StepArgs a, Tables t, const double* __restrict__ q,
+                                                       double* __restrict__ b) {
+  pdl_begin();
+  struct alignas(8 * V) Vec {
+    double v[V];
+  };
+  const int64_t n = (int64_t)a.Nf * (a.wn / V);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t p = a.by_wn(i);
+    const int w = a.w0 + (int)(i - p * (a.wn / V)) * V;
+    int code[kEllMax];
+    Vec v[kEllMax], acc;
+#pragma unroll
+    for (int d = 0; d < kEllMax; ++d) code[d] = d < t.face_deg ? __ldg(t.fj_ell + (int)p * t.face_deg + d) : -1;
+#pragma unroll
+    for (int d = 0; d < kEllMax; ++d) {
+      if (code[d] >= 0) v[d] = *reinterpret_cast<const Vec*>(q + (int64_t)(code[d] >> 1) * a.W + w);
+      else v[d] = Vec{};
+    }
+#pragma unroll
+    for (int u = 0; u < V; ++u) acc.v[u] = signed_by(v[0].v[u], code[0] & 1);
+#pragma unroll
+    for (int d = 1; d < kEllMax; ++d)
+      if (code[d] >= 0)
+#pragma unroll
+        for (int u = 0; u < V; ++u) acc.v[u] += signed_by(v[d].v[u], code[d] & 1);
+    if (a.f.ptr) {
+      const double* f = a.f.ptr + (a.f.stride_n ? __ldg(t.face_orig + p) * a.f.stride_n : 0) + w * a.f.stride_w;
+#pragma unroll
+      for (int u = 0; u < V; ++u) acc.v[u] = fma(-kTwoPi, __ldg(f + u * a.f.stride_w), acc.v[u]);
+    }
+    *reinterpret_cast<Vec*>(b + p * a.W + w) = acc;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.d_step[1] = a.d_step[0] + 1;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -574,12 +749,12 @@ __device__ __forceinline__ Item unpack_item(int4 v) {
 // zero the listed rows (columns [w0, w0 + wn)) of an (Nf x W) vector before a sweep whose partial items accumulate
 // there, and the sweep's dataflow counters (n_ctr of them, none for level-synchronous sweeps)
 __global__ void k_zero_rows(double* __restrict__ v, const int32_t* __restrict__ rows, int n_rows, int W, int w0,
-                            int wn, unsigned* __restrict__ ctr, int n_ctr) {
+                            int wn, FastDiv by_wn, unsigned* __restrict__ ctr, int n_ctr) {
   pdl_begin();
   const int64_t n = (int64_t)n_rows * wn;
   const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nth = (int64_t)gridDim.x * blockDim.x;
   for (int64_t e = tid; e < n; e += nth) {
-    const int64_t i = e / wn, w = w0 + (e - i * wn);
+    const int64_t i = by_wn(e), w = w0 + (e - i * wn);
     v[(int64_t)__ldg(rows + i) * W + w] = 0.0;
   }
   for (int64_t e = tid; e < n_ctr; e += nth) ctr[e] = 0u;
@@ -1497,6 +1672,7 @@ __global__ void k_dst_cols(DstArgs d, int w0, int lines) {
 // ------------------------------------------------------------------------------------------
 struct AdjArgs {
   int Nj, W;
+  FastDiv by_W;
   jja_view G;
   const double* th_m1;
   const double* th_m2;
@@ -1514,7 +1690,7 @@ struct AdjArgs {
 __global__ void __launch_bounds__(256) k_adj_a(AdjArgs a, Tables t, double* __restrict__ u) {
   const int64_t NjW = (int64_t)a.Nj * a.W;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < NjW; e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t j = e / a.W, w = e - j * a.W;
+    const int64_t j = a.by_W(e), w = e - j * a.W;
     double v = view_at(a.G, j, w);
     const double ic = __ldg(t.Ic + (t.ic_per_w ? e : j));
     if (a.mu_p1) v = fma(fma(2.0 * ic, a.cos_p1[e], __ldg(t.coef + j)), a.mu_p1[e], v);
@@ -1529,7 +1705,7 @@ __global__ void __launch_bounds__(256) k_adj_mu(AdjArgs a, Tables t, const doubl
                                                 const double* __restrict__ nu) {
   const int64_t NjW = (int64_t)a.Nj * a.W;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < NjW; e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t j = e / a.W, w = e - j * a.W;
+    const int64_t j = a.by_W(e), w = e - j * a.W;
     const int p0 = __ldg(t.jf_face + 2 * j), p1 = __ldg(t.jf_face + 2 * j + 1);
     double y = p0 >= 0 ? signed_by(nu[(int64_t)(p0 >> 1) * a.W + w], p0 & 1) : 0.0;
     if (p1 >= 0) y += signed_by(nu[(int64_t)(p1 >> 1) * a.W + w], p1 & 1);
@@ -1574,10 +1750,10 @@ __global__ void __launch_bounds__(256) k_vortex(const double* __restrict__ theta
 }
 
 __global__ void k_unpermute_scaled(const double* __restrict__ src, double* __restrict__ dst,
-                                   const int32_t* __restrict__ perm, int n, int W, double scale) {
+                                   const int32_t* __restrict__ perm, int n, int W, FastDiv by_W, double scale) {
   const int64_t nW = (int64_t)n * W;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nW; e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = e / W, w = e - i * W;
+    const int64_t i = by_W(e), w = e - i * W;
     dst[(int64_t)__ldg(perm + i) * W + w] = scale * src[e];
   }
 }
@@ -1589,10 +1765,10 @@ __global__ void k_eval_sin(const double* __restrict__ x, double* __restrict__ ou
 }
 
 __global__ void k_permute_rows(const double* __restrict__ src, double* __restrict__ dst, const int32_t* __restrict__ map,
-                               int n, int W, int gather) {
+                               int n, int W, FastDiv by_W, int gather) {
   const int64_t nW = (int64_t)n * W;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nW; e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = e / W, w = e - i * W;
+    const int64_t i = by_W(e), w = e - i * W;
     const int64_t o = __ldg(map + i);
     if (gather) dst[e] = src[o * W + w];
     else dst[o * W + w] = src[e];
@@ -2183,7 +2359,11 @@ std::vector<longlong2> build_sin_table() {
     const long double ang = (long double)r * pi_l / (long double)(kSinTable / 2);
     const long long s0 = llroundl(sinl(ang) * scale), c0 = llroundl(cosl(ang) * scale);
     const long long sv[4] = {s0, c0, -s0, -c0}, cv[4] = {c0, -s0, -c0, s0};
-    tab[(size_t)k] = make_longlong2(sv[q], cv[q]);
+    // hi 2^32 + lo with a signed lower half
+    auto word = [](long long v) {
+      return (long long)((((unsigned long long)(v + (1ll << 31)) >> 32) << 32) | ((unsigned long long)v & 0xffffffffull));
+    };
+    tab[(size_t)k] = make_longlong2(word(sv[q]), word(cv[q]));
   }
   return tab;
 }
@@ -2229,6 +2409,7 @@ struct jja_plan {
   double *b = nullptr, *z = nullptr, *x = nullptr, *xj = nullptr;
   int32_t* perm = nullptr;   // new -> old face
   double* isq = nullptr;        // Is / c0 (Nj x W)
+  double* amp = nullptr;        // noise amplitude over c0 (Nj)
   int resistive = 0;
   // dataflow sweeps (schedule 2): dependency tables per supernode, counters, error flag
   int flow = 0, ns = 0;
@@ -2358,7 +2539,7 @@ void launch_zero_rows(jja_plan* p, const Group& g, cudaStream_t st, bool forward
   if (!n && !n_ctr) return;
   unsigned* ctr = p->flow ? p->counters + (forward ? 0 : p->ns + 1) : nullptr;
   launch(p->pdl, k_zero_rows, grid_for(std::max<int64_t>((int64_t)n * g.wn, n_ctr), 256), 256, st, v,
-         (const int32_t*)(forward ? g.zrows_f : g.zrows_b), n, p->W, g.w0, g.wn, ctr, n_ctr);
+         (const int32_t*)(forward ? g.zrows_f : g.zrows_b), n, p->W, g.w0, g.wn, fast_div(g.wn), ctr, n_ctr);
 }
 
 void launch_zero_rows(jja_plan* p, cudaStream_t st, bool forward, double* v) { launch_zero_rows(p, p->all, st, forward, v); }
@@ -2490,12 +2671,12 @@ void launch_sine_solve(jja_plan* p, const Group& g, cudaStream_t st) {
     d.parts = sine_parts(d.kp, tiles);
     const unsigned grid = (unsigned)(d.parts * std::min<int64_t>(tiles, kNumSMs / d.parts));
     launch_smem(p->pdl, sine_kernel(d.kp), dim3(grid), kSineThreads, sine_smem_bytes(d.kp), st, d, in, out, g.w0, g.wn,
-                p->flow_err);
+                fast_div(g.wn), p->flow_err);
   };
   const SineTri& t = p->sine_tri;
   const unsigned tri = (unsigned)(((int64_t)t.lines * g.wn + kTriColumns - 1) / kTriColumns);
   lines(p->sine_fwd, p->b, p->z);
-  launch_smem(p->pdl, k_sine_tri, dim3(tri), 2 * kTriColumns, 0, st, t, p->z, g.w0, g.wn);
+  launch_smem(p->pdl, k_sine_tri, dim3(tri), 2 * kTriColumns, 0, st, t, p->z, g.w0, g.wn, fast_div(g.wn));
   lines(p->sine_bwd, p->z, p->x);
 }
 
@@ -2533,14 +2714,61 @@ void launch_junction(jja_plan* p, StepArgs& a, cudaStream_t st) {
   launch(p->pdl, k_junction, grid_for((int64_t)p->Nj * a.wn, 256), 256, st, a, p->t, p->xj);
 }
 
+// two problems per thread: even problem ranges and 16-byte aligned arrays
+bool pairs_fit(const StepArgs& a) {
+  auto aligned = [](const void* p) { return ((uintptr_t)p & 15u) == 0; };
+  return a.W % 2 == 0 && a.w0 % 2 == 0 && a.wn % 2 == 0 && aligned(a.h[0]) && aligned(a.hout) && aligned(a.th_out);
+}
+
+void launch_face_rhs(jja_plan* p, const StepArgs& a, cudaStream_t st) {
+  const int64_t nf = (int64_t)p->Nf * a.wn;
+  const double* q = p->xj;
+  if (!p->t.face_deg || a.theta_s || a.f.stride_t || (int64_t)p->Nf * p->t.face_deg >= INT_MAX) {
+    launch(p->pdl, k_face_rhs, grid_for(nf, 256), 256, st, a, p->t, q, p->b);
+    return;
+  }
+  StepArgs f = a;
+  if (a.W % 2 == 0 && a.w0 % 2 == 0 && a.wn % 2 == 0) {
+    f.by_wn = fast_div(a.wn / 2);
+    launch(p->pdl, k_face_rhs_fast<2>, grid_for(nf / 2, 256), 256, st, f, p->t, q, p->b);
+  } else {
+    launch(p->pdl, k_face_rhs_fast<1>, grid_for(nf, 256), 256, st, f, p->t, q, p->b);
+  }
+}
+
+void launch_update(jja_plan* p, const StepArgs& a, cudaStream_t st, bool fuse_next) {
+  const int64_t nj = (int64_t)p->Nj * a.wn;
+  const double* J = p->x;
+  const bool noise = a.noise_mode != JJA_NOISE_NONE;
+  const bool fast = fuse_next && a.width == 3 && !a.theta_s && (!a.Is.ptr || a.Isq.ptr) &&
+                    (a.store_all ? !a.I_out : a.th_slot < 0 && a.I_slot < 0) &&
+                    (!noise || (a.noise_mode == JJA_NOISE_PHILOX && a.amp));
+  if (!fast) {
+    if (fuse_next) launch(p->pdl, k_update<true>, grid_for(nj, 256), 256, st, a, p->t, p->xj, J);
+    else launch(p->pdl, k_update<false>, grid_for(nj, 256), 256, st, a, p->t, p->xj, J);
+    return;
+  }
+  StepArgs f = a;
+  const bool cap = !a.resistive;
+  if (pairs_fit(a)) {
+    f.by_wn = fast_div(a.wn / 2);
+    auto kern = cap ? (noise ? k_update_fast<true, true, 2> : k_update_fast<true, false, 2>)
+                    : (noise ? k_update_fast<false, true, 2> : k_update_fast<false, false, 2>);
+    launch(p->pdl, kern, grid_for(nj / 2, 256), 256, st, f, p->t, p->xj, J);
+  } else {
+    auto kern = cap ? (noise ? k_update_fast<true, true, 1> : k_update_fast<true, false, 1>)
+                    : (noise ? k_update_fast<false, true, 1> : k_update_fast<false, false, 1>);
+    launch(p->pdl, kern, grid_for(nj, 256), 256, st, f, p->t, p->xj, J);
+  }
+}
+
 // one time step of group g whose q is already in p->xj; `fuse_next` also leaves the next step's
 // q there. With `ev` (5 events) the boundaries face rhs | forward | backward | update(+next q)
 // are recorded.
 void launch_step(jja_plan* p, const Group& g, StepArgs& a, cudaStream_t st, bool fuse_next,
                  cudaEvent_t* ev = nullptr) {
-  const int64_t nj = (int64_t)p->Nj * g.wn, nf = (int64_t)p->Nf * g.wn;
   if (ev) JJA_CUDA(cudaEventRecord(ev[0], st));
-  launch(p->pdl, k_face_rhs, grid_for(nf, 256), 256, st, a, p->t, (const double*)p->xj, p->b);
+  launch_face_rhs(p, a, st);
   if (ev) JJA_CUDA(cudaEventRecord(ev[1], st));
   if (p->dst) {
     launch_face_solve(p, g, st);
@@ -2551,8 +2779,7 @@ void launch_step(jja_plan* p, const Group& g, StepArgs& a, cudaStream_t st, bool
     launch_levels(p, g, st, false);
   }
   if (ev) JJA_CUDA(cudaEventRecord(ev[3], st));
-  if (fuse_next) launch(p->pdl, k_update<true>, grid_for(nj, 256), 256, st, a, p->t, p->xj, (const double*)p->x);
-  else launch(p->pdl, k_update<false>, grid_for(nj, 256), 256, st, a, p->t, p->xj, (const double*)p->x);
+  launch_update(p, a, st, fuse_next);
   if (ev) JJA_CUDA(cudaEventRecord(ev[4], st));
 }
 
@@ -2560,6 +2787,7 @@ StepArgs make_args(jja_plan* p, jja_state* s, const Group& g) {
   StepArgs a{};
   a.Nj = p->Nj; a.Nf = p->Nf; a.W = p->W; a.width = p->width;
   a.w0 = g.w0; a.wn = g.wn;
+  a.by_wn = fast_div(g.wn);
   for (int k = 0; k < 4; ++k) { a.h[k] = s->hist[k]; a.e[k] = p->extrap[k]; }
   a.theta_s = s->theta_s;
   a.Is = s->Is; a.f = s->f; a.Vs = s->Vs; a.T = s->T;
@@ -2573,14 +2801,17 @@ StepArgs make_args(jja_plan* p, jja_state* s, const Group& g) {
   a.dt = p->dt;
   a.Isq = (s->Is.ptr && !s->Is.stride_t) ? jja_view{p->isq, p->W, 1, 0} : jja_view{nullptr, 0, 0, 0};
   a.resistive = p->resistive;
+  a.amp = (s->noise_mode != JJA_NOISE_NONE && s->T.ptr && !s->T.stride_t && !s->T.stride_w) ? p->amp : nullptr;
   return a;
 }
 
-// refresh Is / c0 from a time-independent current-source view (before the first step of a run)
+// refresh Is / c0 and the noise amplitudes from time-independent views (before the first step of a run)
 void launch_scale_sources(jja_plan* p, jja_state* s, cudaStream_t st) {
+  if (s->noise_mode != JJA_NOISE_NONE && s->T.ptr && !s->T.stride_t && !s->T.stride_w)
+    launch(p->pdl, k_noise_amp, grid_for(p->Nj, 256), 256, st, s->T, p->t.Rvq, p->amp, p->Nj);
   if (!s->Is.ptr || s->Is.stride_t) return;
   launch(p->pdl, k_scale_sources, grid_for((int64_t)p->Nj * p->W, 256), 256, st, s->Is, p->t.inv_c0, p->isq, p->Nj,
-         p->W);
+         p->W, fast_div(p->W));
 }
 
 // rotate the history: the oldest buffer receives theta_next
@@ -3019,6 +3250,7 @@ int jja_plan_create(const jja_plan_desc* d, const jja_factor* fac, jja_plan** ou
     p->x = p->up<double>(nullptr, NfW);
     p->xj = p->up<double>(nullptr, NjW);
     p->isq = p->up<double>(nullptr, NjW);
+    p->amp = p->up<double>(nullptr, Nj);
     JJA_CUDA(cudaDeviceSynchronize());
     *out = p.release();
   });
@@ -3180,6 +3412,13 @@ int jja_plan_set_sine_solver(jja_plan* p, int mx, int my, const int32_t* grid_fa
     p->sine_bwd = d;
     p->sine_tri = t;
     JJA_CUDA(cudaFuncSetAttribute(sine_kernel(kp), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sine_smem_bytes(kp)));
+    // the step runs as one chain: its kernels fill the GPU (128x128 x 512: 0.477 ms per step, 0.519
+    // as the three concurrent groups that the sweeps' levels want)
+    for (Group& gr : p->groups) {
+      if (gr.stream) cudaStreamDestroy(gr.stream);
+      if (gr.done) cudaEventDestroy(gr.done);
+    }
+    p->groups.clear();
     // graphs captured before bake in the sweeps: drop them
     for (auto& g2 : p->graphs) cudaGraphExecDestroy(g2.exec);
     for (auto& g2 : p->adj_graphs) cudaGraphExecDestroy(g2.exec);
@@ -3240,10 +3479,10 @@ int jja_solve(jja_plan* p, const double* b, double* x, void* stream) {
     if (!p || !b || !x) throw Error(JJA_ERR_ARG, "jja_solve: null argument");
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t NfW = (int64_t)p->Nf * p->W;
-    k_permute_rows<<<grid_for(NfW, 256), 256, 0, st>>>(b, p->b, p->perm, p->Nf, p->W, 1);
+    k_permute_rows<<<grid_for(NfW, 256), 256, 0, st>>>(b, p->b, p->perm, p->Nf, p->W, fast_div(p->W), 1);
     g_launches++;
     launch_face_solve(p, st);
-    k_permute_rows<<<grid_for(NfW, 256), 256, 0, st>>>(p->x, x, p->perm, p->Nf, p->W, 0);
+    k_permute_rows<<<grid_for(NfW, 256), 256, 0, st>>>(p->x, x, p->perm, p->Nf, p->W, fast_div(p->W), 0);
     g_launches++;
     JJA_CUDA(cudaGetLastError());
   });
@@ -3336,11 +3575,11 @@ int jja_solve_static(jja_plan* p, const double* b, double* x, void* stream) {
     double* z = bx + NfW;                                // forward-substitution result
     const int32_t* perm = p->perm_factor ? p->perm_factor : p->perm;   // the sweeps' face order
     // every element of both work vectors is written before it is read: nothing to clear
-    k_permute_rows<<<grid_for(NfW, 256), 256, 0, st>>>(b, bx, perm, p->Nf, p->W, 1);
+    k_permute_rows<<<grid_for(NfW, 256), 256, 0, st>>>(b, bx, perm, p->Nf, p->W, fast_div(p->W), 1);
     g_launches++;
     launch_levels_into(p, st, true, bx, z, nullptr);
     launch_levels_into(p, st, false, nullptr, z, bx);
-    k_permute_rows<<<grid_for(NfW, 256), 256, 0, st>>>(bx, x, perm, p->Nf, p->W, 0);
+    k_permute_rows<<<grid_for(NfW, 256), 256, 0, st>>>(bx, x, perm, p->Nf, p->W, fast_div(p->W), 0);
     g_launches++;
     JJA_CUDA(cudaGetLastError());
   });
@@ -3348,12 +3587,12 @@ int jja_solve_static(jja_plan* p, const double* b, double* x, void* stream) {
 
 // one backward-through-time step: a_n -> u = D a_n, b = A u, both sweeps, mu_n and accumulations
 static void launch_adjoint_step(jja_plan* p, const AdjArgs& a, cudaStream_t st) {
-  const int64_t NjW = (int64_t)p->Nj * p->W, NfW = (int64_t)p->Nf * p->W;
+  const int64_t NjW = (int64_t)p->Nj * p->W;
   k_adj_a<<<grid_for(NjW, 256), 256, 0, st>>>(a, p->t, p->xj);
   StepArgs s{};
-  s.Nj = p->Nj; s.Nf = p->Nf; s.W = p->W; s.width = p->width; s.w0 = 0; s.wn = p->W; s.d_step = p->all.d_step;
-  k_face_rhs<<<grid_for(NfW, 256), 256, 0, st>>>(s, p->t, p->xj, p->b);
-  g_launches += 2;
+  s.Nj = p->Nj; s.Nf = p->Nf; s.W = p->W; s.width = p->width; s.w0 = 0; s.wn = p->W; s.by_wn = fast_div(p->W); s.d_step = p->all.d_step;
+  launch_face_rhs(p, s, st);
+  g_launches++;
   launch_face_solve(p, st);
   k_adj_mu<<<grid_for(NjW, 256), 256, 0, st>>>(a, p->t, p->xj, p->x);
   g_launches++;
@@ -3368,7 +3607,7 @@ int jja_adjoint_step(jja_plan* p, const jja_adjoint_args* g, void* stream) {
     if ((g->mu_p1 && !g->cos_p1) || (g->mu_p2 && !g->cos_p2))
       throw Error(JJA_ERR_ARG, "jja_adjoint_step: mu of a later step given without its cos(phi)");
     AdjArgs a{};
-    a.Nj = p->Nj; a.W = p->W; a.G = g->G;
+    a.Nj = p->Nj; a.W = p->W; a.by_W = fast_div(p->W); a.G = g->G;
     a.th_m1 = g->th_m1; a.th_m2 = g->th_m2;
     a.mu_p1 = g->mu_p1; a.mu_p2 = g->mu_p2; a.cos_p1 = g->cos_p1; a.cos_p2 = g->cos_p2;
     a.mu_out = g->mu_out; a.cos_out = g->cos_out; a.usum = g->usum; a.musum = g->musum; a.gIc = g->gIc;
@@ -3391,7 +3630,7 @@ int jja_adjoint_segment(jja_plan* p, const jja_adjoint_segment_args* g, void* st
       for (int64_t i = g->L - 1; i >= 0; --i) {    // steps s0 + L - 1 down to s0
         const int64_t n = g->s0 + i;
         AdjArgs a{};
-        a.Nj = p->Nj; a.W = p->W;
+        a.Nj = p->Nj; a.W = p->W; a.by_W = fast_div(p->W);
         const double* Gn = g->G ? g->G[i] : nullptr;
         a.G = jja_view{Gn, Gn ? p->W : 0, Gn ? 1 : 0, 0};
         a.th_m1 = g->seg + (i + 1) * NjW;          // theta_{n-1}
@@ -3448,11 +3687,11 @@ int jja_adjoint_flux(jja_plan* p, const double* usum, double* gf, void* stream) 
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t NfW = (int64_t)p->Nf * p->W;
     StepArgs s{};
-    s.Nj = p->Nj; s.Nf = p->Nf; s.W = p->W; s.width = p->width; s.w0 = 0; s.wn = p->W; s.d_step = p->all.d_step;
+    s.Nj = p->Nj; s.Nf = p->Nf; s.W = p->W; s.width = p->width; s.w0 = 0; s.wn = p->W; s.by_wn = fast_div(p->W); s.d_step = p->all.d_step;
     k_face_rhs<<<grid_for(NfW, 256), 256, 0, st>>>(s, p->t, usum, p->b);
     g_launches++;
     launch_face_solve(p, st);
-    k_unpermute_scaled<<<grid_for(NfW, 256), 256, 0, st>>>(p->x, gf, p->perm, p->Nf, p->W, -kTwoPi);
+    k_unpermute_scaled<<<grid_for(NfW, 256), 256, 0, st>>>(p->x, gf, p->perm, p->Nf, p->W, fast_div(p->W), -kTwoPi);
     g_launches++;
     JJA_CUDA(cudaGetLastError());
   });
@@ -3599,8 +3838,7 @@ int jja_run_timed(jja_plan* p, jja_state* s, int nsteps, double* stage_ms, void*
       };
       JJA_CUDA(cudaEventRecord(e[0], st));
       stage(1, [&](size_t q, cudaStream_t gst) {
-        launch(p->pdl, k_face_rhs, grid_for((int64_t)p->Nf * gs[q]->wn, 256), 256, gst, args[q], p->t,
-               (const double*)p->xj, p->b);
+        launch_face_rhs(p, args[q], gst);
       });
       // (a fast Poisson plan solves in the "forward" stage; its "backward" stage is empty)
       stage(2, [&](size_t q, cudaStream_t gst) {
@@ -3611,11 +3849,7 @@ int jja_run_timed(jja_plan* p, jja_state* s, int nsteps, double* stage_ms, void*
         if (!p->dst) launch_levels(p, *gs[q], gst, false);
       });
       stage(4, [&](size_t q, cudaStream_t gst) {
-        const int64_t nj = (int64_t)p->Nj * gs[q]->wn;
-        if (i + 1 < nsteps)
-          launch(p->pdl, k_update<true>, grid_for(nj, 256), 256, gst, args[q], p->t, p->xj, (const double*)p->x);
-        else
-          launch(p->pdl, k_update<false>, grid_for(nj, 256), 256, gst, args[q], p->t, p->xj, (const double*)p->x);
+        launch_update(p, args[q], gst, i + 1 < nsteps);
       });
       rotate(s, p->width);
     }

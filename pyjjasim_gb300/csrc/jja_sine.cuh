@@ -197,7 +197,7 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 template <int kp>
 __global__ void __launch_bounds__(kSineThreads, 1) k_sine_lines(SineArgs d, const double* __restrict__ in,
                                                                double* __restrict__ out, int w0, int wn,
-                                                               int* __restrict__ err) {
+                                                               FastDiv by_wn, int* __restrict__ err) {
   pdl_begin();
   extern __shared__ __align__(128) unsigned char sine_sh[];
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), m = d.m, half = m >> 1;
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kSineThreads, 1) k_sine_lines(SineArgs d, cons
   auto load = [&](int tl) {
     const int64_t c = (int64_t)tl * kSineColumns + col;
     const bool live = c < ncols;
-    const int64_t line = live ? c / wn : 0;
+    const int64_t line = live ? by_wn(c) : 0;
     const double* src = in + line * d.s_c + (live ? w0 + (c - line * wn) : 0);
 #pragma unroll
     for (int r = 0; r < 2; ++r)
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kSineThreads, 1) k_sine_lines(SineArgs d, cons
   for (; tile < tiles; tile += tile_step) {
     const int64_t c = (int64_t)tile * kSineColumns + col;
     const bool live = c < ncols;
-    const int64_t line = live ? c / wn : 0;
+    const int64_t line = live ? by_wn(c) : 0;
     double* dst = out + line * d.s_c + (live ? w0 + (c - line * wn) : 0);
     uint32_t top = 0;   // the line's largest magnitude (high words without the sign)
 #pragma unroll
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kSineThreads, 1) k_sine_lines(SineArgs d, cons
   }
 }
 
-using SineKernel = void (*)(SineArgs, const double*, double*, int, int, int*);
+using SineKernel = void (*)(SineArgs, const double*, double*, int, int, FastDiv, int*);
 SineKernel sine_kernel(int kp) {
   return kp == 16 ? k_sine_lines<16> : kp == 32 ? k_sine_lines<32> : kp == 48 ? k_sine_lines<48> : k_sine_lines<64>;
 }
@@ -400,13 +400,13 @@ size_t sine_smem_bytes(int kp) {
 // eliminated from both ends towards the middle by two threads (half the chain each), joined
 // there, and substituted back outwards. 3 FP64 operations per element.
 constexpr int kTriColumns = 64;
-__global__ void __launch_bounds__(2 * kTriColumns) k_sine_tri(SineTri t, double* v, int w0, int wn) {
+__global__ void __launch_bounds__(2 * kTriColumns) k_sine_tri(SineTri t, double* v, int w0, int wn, FastDiv by_wn) {
   pdl_begin();
   __shared__ double join_z[2][kTriColumns];
   const int side = threadIdx.x / kTriColumns, lc = threadIdx.x - side * kTriColumns;   // 0: from the first point
   const int64_t c = (int64_t)blockIdx.x * kTriColumns + lc, ncols = (int64_t)t.lines * wn;
   const bool live = c < ncols;
-  const int mode = live ? (int)(c / wn) : 0;
+  const int mode = live ? (int)by_wn(c) : 0;
   const int cnt = side ? t.n - t.top : t.top;
   const int64_t step = side ? -t.s_n : t.s_n;
   double* p0 = v + (int64_t)mode * t.s_c + (live ? w0 + (c - (int64_t)mode * wn) : 0) + (side ? (int64_t)(t.n - 1) * t.s_n : 0);
