@@ -188,6 +188,13 @@ int jja_plan_set_fast_poisson(jja_plan* p, int mx, int my, const int32_t* grid_f
  * Replaces the plan's triangular sweeps (jja_solve_static keeps them). Not on a plan that already solves
  * by sine transforms. */
 int jja_plan_set_sine_solver(jja_plan* p, int mx, int my, const int32_t* grid_face, double kappa);
+
+/* Steps of a small circuit (at most 160 faces and 1024 junctions, and their state and the inverse of
+ * the face-space matrix within one SM's shared memory) run whole inside one launch per call of jja_run
+ * with use_graph (one block per problem), from the inverse of the factored matrix. Calls without
+ * use_graph, with a host noise buffer, jja_run_timed, jja_solve and the adjoint keep the sweeps. The
+ * history buffers keep their places in jja_state over such a call (no rotation). */
+int jja_plan_set_resident(jja_plan* p, const jja_factor* f);
 /* Synchronises the device, then reads and clears the plan's device error flags: *flow_timeouts
  * = 1 if a wait of a dataflow sweep ran out of its bound since the last call (the results of
  * those steps are invalid), else 0. Returns JJA_ERR_NONFINITE when a time step of jja_run /

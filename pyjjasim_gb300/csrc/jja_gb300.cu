@@ -1778,6 +1778,7 @@ __global__ void k_permute_rows(const double* __restrict__ src, double* __restric
 }  // namespace
 
 #include "jja_sine.cuh"
+#include "jja_resident.cuh"
 
 namespace {
 
@@ -2440,6 +2441,10 @@ struct jja_plan {
   // tridiagonal solves, transform back; face vectors in grid order
   SineArgs sine_fwd{}, sine_bwd{};
   SineTri sine_tri{};
+  // whole runs of a small circuit in one launch (jja_plan_set_resident; inv null: not)
+  ResidentArgs res{};
+  int64_t* res_slots = nullptr;      // output slots of a call's steps (phases, then currents)
+  size_t res_slots_cap = 0;
   int32_t* perm_factor = nullptr;    // the factor's face order, when perm is the grid's
   std::vector<int32_t> iperm_host;   // original face -> factor's face order
   int64_t bytes = 0;
@@ -2460,6 +2465,7 @@ struct jja_plan {
       if (g.done) cudaEventDestroy(g.done);
     }
     if (fork) cudaEventDestroy(fork);
+    if (res_slots) cudaFree(res_slots);
     for (void* p : allocs) cudaFree(p);
   }
   template <class T>
@@ -2866,6 +2872,38 @@ void join_groups(jja_plan* p, cudaStream_t st) {
 
 void set_counters(jja_plan* p, const jja_state* s, cudaStream_t st) {
   for (Group* g : step_groups(p)) launch(p->pdl, k_set_counters, 1, 1, st, g->d_step, s->step, s->src_t0);
+}
+
+// all steps of a call of a resident plan: one launch per kResChunk steps, the phase history read
+// from and left in the state's buffers (no rotation)
+void run_resident(jja_plan* p, jja_state* s, int nsteps, const int64_t* th_slot, const int64_t* I_slot,
+                  cudaStream_t st) {
+  StepArgs a = make_args(p, s, p->all);
+  if (th_slot || I_slot) {
+    if (p->res_slots_cap < 2 * (size_t)nsteps) {
+      JJA_CUDA(cudaDeviceSynchronize());   // an earlier call may still read the smaller buffer
+      if (p->res_slots) JJA_CUDA(cudaFree(p->res_slots));
+      p->res_slots = nullptr;
+      p->res_slots_cap = 0;
+      JJA_CUDA(cudaMalloc(&p->res_slots, 2 * (size_t)nsteps * sizeof(int64_t)));
+      p->res_slots_cap = 2 * (size_t)nsteps;
+    }
+    if (th_slot)
+      JJA_CUDA(cudaMemcpyAsync(p->res_slots, th_slot, nsteps * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+    if (I_slot)
+      JJA_CUDA(cudaMemcpyAsync(p->res_slots + nsteps, I_slot, nsteps * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+  }
+  for (int i = 0; i < nsteps; i += kResChunk) {
+    ResidentArgs g = p->res;
+    g.nsteps = std::min(kResChunk, nsteps - i);
+    g.step0 = s->step + i;
+    g.src_t0 = s->src_t0;
+    g.th_slots = th_slot ? p->res_slots + i : nullptr;
+    g.I_slots = I_slot ? p->res_slots + nsteps + i : nullptr;
+    g.slot0 = i;
+    launch_smem(false, k_resident, dim3((unsigned)p->W), kResThreads,
+                resident_smem_bytes(g.n, g.nj, p->width - 1), st, a, p->t, g);
+  }
 }
 
 // graph of G fused steps for the state's current buffers (captured on first use, then cached);
@@ -3428,6 +3466,42 @@ int jja_plan_set_sine_solver(jja_plan* p, int mx, int my, const int32_t* grid_fa
   });
 }
 
+int jja_plan_set_resident(jja_plan* p, const jja_factor* fac) {
+  return guarded([&] {
+    if (!p || !fac) throw Error(JJA_ERR_ARG, "jja_plan_set_resident: null argument");
+    const jja::Factor& F = *fac->f;
+    const int n = p->Nf, nh = p->width - 1;
+    if (F.n != n) throw Error(JJA_ERR_ARG, "jja_plan_set_resident: factor order != Nf");
+    if (p->dst) throw Error(JJA_ERR_ARG, "jja_plan_set_resident: the plan solves by sine transforms");
+    const size_t smem = n <= kResMaxFaces ? resident_smem_bytes(n, p->Nj, nh) : SIZE_MAX;
+    if (p->Nj > kResMaxJunctions || smem > (size_t)227 * 1024)
+      throw Error(JJA_ERR_ARG, "jja_plan_set_resident: the circuit does not fit one SM");
+    // the inverse, in the factor's face order, column by column in fixed point
+    std::vector<double> inv((size_t)n * n, 0.0);   // row-major right-hand sides
+    for (int i = 0; i < n; ++i) inv[(size_t)i * n + i] = 1.0;
+    jja::factor_solve_host(F, inv.data(), n);
+    double top = 0.0;
+    for (double v : inv) top = std::max(top, std::fabs(v));
+    if (!(top > 0.0) || !std::isfinite(top)) throw Error(JJA_ERR_NOT_SPD, "jja_plan_set_resident: no finite inverse");
+    int e = 0;
+    std::frexp(top, &e);   // |inv| < 2^e
+    std::vector<int2> fixed((size_t)n * n);
+    for (int c = 0; c < n; ++c)
+      for (int r = 0; r < n; ++r) {
+        const int64_t v = (int64_t)std::llround(std::ldexp(inv[(size_t)F.perm[r] * n + F.perm[c]], 55 - e));
+        const int lo = (int)((uint32_t)v << (32 - kResHalf)) >> (32 - kResHalf);
+        fixed[(size_t)c * n + r] = make_int2((int)((v - lo) >> kResHalf), lo);
+      }
+    JJA_CUDA(cudaFuncSetAttribute(k_resident, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    ResidentArgs g{};
+    g.inv = p->up(fixed.data(), fixed.size());
+    g.e_inv = e;
+    g.n = n;
+    g.nj = p->Nj;
+    p->res = g;
+  });
+}
+
 int jja_plan_test_wait_limit(jja_plan* p, void* stream) {
   return guarded([&] {
     if (!p) throw Error(JJA_ERR_ARG, "jja_plan_test_wait_limit: null plan");
@@ -3747,6 +3821,12 @@ int jja_run(jja_plan* p, jja_state* s, int nsteps, const int64_t* th_slot, const
     const std::vector<Group*> gs = step_groups(p);
     set_counters(p, s, st);
     launch_scale_sources(p, s, st);
+    if (p->res.inv && use_graph && s->noise_mode != JJA_NOISE_BUFFER) {
+      run_resident(p, s, nsteps, th_slot, I_slot, st);
+      JJA_CUDA(cudaGetLastError());
+      s->step += nsteps;
+      return;
+    }
     fork_groups(p, st);
     for (Group* g : gs) {
       StepArgs a = make_args(p, s, *g);

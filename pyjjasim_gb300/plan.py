@@ -203,6 +203,20 @@ def sine_solver_fits(grid, W):
     return min(mx, my) <= SINE_MAX_SIDE and min(mx, my) >= 8 and max(mx, my) * W >= SINE_MIN_COLUMNS
 
 
+# Circuits whose state and inverse fit one SM run whole calls in one launch, a block per problem, while
+# the problems need at most a few rounds of blocks. Measured on GB300 (us per step, one launch per call /
+# launches per step): 5x5 nodes W = 1 2.4 / 12.2; 10x10 W = 64 3.2 / 24.8, W = 512 8.2 / 25.7, W = 1024
+# 14.5 / 27.0; 13x13 W = 152 5.0 / 25.5, W = 512 19.4 / 27.2, W = 1024 34.1 / 32.6
+RESIDENT_MAX_FACES = 160
+RESIDENT_MAX_JUNCTIONS = 512
+RESIDENT_MAX_W = 512
+
+
+def resident_fits(circuit, W):
+    """Whether the default plan steps W problems of this circuit in one launch per call."""
+    return circuit._Nf() <= RESIDENT_MAX_FACES and circuit._Nj() <= RESIDENT_MAX_JUNCTIONS and W <= RESIDENT_MAX_W
+
+
 def untuned(tuning):
     """True when ``tuning`` asks for nothing but the level schedule (the library's default)."""
     t = dict(tuning or {})
@@ -213,7 +227,7 @@ class DevicePlan:
     """Circuit tables + factor uploaded for W problems (owned C object)."""
 
     def __init__(self, circuit, factor, A, W, dt, stencil_width, stencil, Ic_w=None, tuning=None, fast_poisson=None,
-                 sine=None):
+                 sine=None, resident=False):
         """``tuning``: dict with any of rhs_block, rows_per_lane, target_warps, min_piece (the
         launch shape of the triangular solves; missing or 0 = library default)."""
         Nj, Nf = circuit._Nj(), circuit._Nf()
@@ -257,6 +271,10 @@ class DevicePlan:
             self._keep["grid"] = grid
             N.check(N.lib().jja_plan_set_sine_solver(h, int(mx), int(my), N.ptr(grid, ctypes.c_int32), float(kappa)))
             self.sine = True
+        self.resident = False
+        if resident:
+            N.check(N.lib().jja_plan_set_resident(h, factor.handle))
+            self.resident = True
         self.device_bytes = N.lib().jja_plan_device_bytes(h)
 
     def solve(self, b_dev, x_dev, stream=0):
@@ -368,11 +386,12 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
     nd_leaf, relax = resolve_factor_shape(nd_leaf, relax, ordering, W, circuit._Nf())
     fp = None
     matrices = face_matrix(circuit, dt)
-    if fast_poisson is True or (fast_poisson == "auto" and W <= FAST_POISSON_MAX_W
+    resident = fast_poisson == "auto" and untuned(tuning) and resident_fits(circuit, W)
+    if fast_poisson is True or (fast_poisson == "auto" and not resident and W <= FAST_POISSON_MAX_W
                                 and W * circuit._Nf() <= FAST_POISSON_MAX_WORK):
         fp = fast_poisson_grid(circuit, matrices[1])
     sine = None
-    if fp is None and fast_poisson == "auto" and W * circuit._Nf() >= SINE_MIN_COLUMNS and untuned(tuning):
+    if fp is None and not resident and fast_poisson == "auto" and W * circuit._Nf() >= SINE_MIN_COLUMNS and untuned(tuning):
         sine = poisson_grid(circuit, matrices[1])
         if sine is not None and not sine_solver_fits(sine, W):
             sine = None
@@ -382,7 +401,7 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
         Ic_w = np.ascontiguousarray(np.broadcast_to(np.asarray(Ic_w, np.float64), (circuit._Nj(), W)))
     ic = np.asarray(circuit._Ic(), np.float64) if Ic_w is None else Ic_w
     tkey = tuple(int((tuning or {}).get(f, 0)) for f in TUNING_FIELDS)
-    key = (fkey, W, stencil_width, Ic_w is None, tkey, fp is not None, sine is not None,
+    key = (fkey, W, stencil_width, Ic_w is None, tkey, fp is not None, sine is not None, resident,
            _digest(ic, *coef, Rv, A.indptr, A.indices, A.data))
     with _CACHE_LOCK:
         p = _PLANS.get(key)
@@ -390,7 +409,7 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
             _PLANS.move_to_end(key)
             return p
     p = DevicePlan(circuit, factor, A, W, dt, stencil_width, stencil, Ic_w=Ic_w, tuning=tuning, fast_poisson=fp,
-                   sine=sine)
+                   sine=sine, resident=resident)
     with _CACHE_LOCK:
         _PLANS[key] = p
         while len(_PLANS) > MAX_PLANS:

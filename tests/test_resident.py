@@ -1,0 +1,94 @@
+"""Whole runs of small circuits in one launch (jja_plan_set_resident) against the oracle and the sweeps.
+
+The trajectory bars are those of the other paths (1e-9 relative against the oracle, 1e-10 between
+solvers): one face-space product is off by at most n 2^-55 of max|K^-1| max|b|, below an FP64 dot
+product's bound for n <= 160 terms."""
+import numpy as np
+import pytest
+
+from oracle import rcsj_oracle
+from pyjjasim_gb300 import TimeEvolutionProblem, backend
+from pyjjasim_gb300 import plan as P
+from pyjjasim_gb300.circuit import HoneycombArray, SquareArray, TriangularArray
+
+
+def test_rule():
+    assert P.resident_fits(SquareArray(10, 10), 1) and P.resident_fits(SquareArray(13, 13), P.RESIDENT_MAX_W)
+    assert not P.resident_fits(SquareArray(10, 10), P.RESIDENT_MAX_W + 1)
+    assert not P.resident_fits(SquareArray(14, 14), 1)
+
+
+CASES = [(SquareArray, 2, 2, 1, 3), (SquareArray, 2, 5, 3, 4), (SquareArray, 9, 5, 1, 3),    # 1, 4 and 32 faces
+         (SquareArray, 12, 4, 2, 5), (SquareArray, 10, 10, 5, 3), (SquareArray, 9, 17, 2, 4),  # 33, 81, 128 faces
+         (SquareArray, 9, 21, 1, 3), (HoneycombArray, 4, 4, 7, 3), (TriangularArray, 5, 4, 3, 5)]   # 160 faces
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lattice,nx,ny,W,width", CASES)
+@pytest.mark.parametrize("sources", ["constant", "timedep"])
+def test_trajectory(lattice, nx, ny, W, width, sources):
+    c = lattice(nx, ny)
+    rng = np.random.default_rng(nx * ny + W)
+    c.set_resistance(rng.uniform(0.8, 1.3, c._Nj()))
+    c.set_critical_current(rng.uniform(0.5, 1.5, c._Nj()))
+    if width > 3:
+        c.set_capacitance(0.6)
+    c.set_inductance(0.1)
+    Nt = 60
+    Is = rng.uniform(-0.6, 0.6, (c._Nj(), W, 1))
+    f, kw = rng.uniform(-0.4, 0.4, (c._Nf(), W, 1)), {}
+    if sources == "timedep":
+        Is = Is * np.sin(0.1 * np.arange(Nt))
+        f = lambda i: 0.01 * i
+        kw = dict(voltage_sources=rng.uniform(-0.2, 0.2, (c._Nj(), 1, 1)))
+    prob = TimeEvolutionProblem(c, time_step=0.05, time_step_count=Nt, current_sources=Is, external_flux=f,
+                                store_time_steps=[0, 7, 8, 9, 30, Nt - 1], stencil_width=width,
+                                config_at_minus_1=rng.uniform(-1, 1, (c._Nj(), W)), **kw)
+    m, mI = prob.store_time_steps, np.arange(Nt) % 3 == 0
+    sim = backend.GpuSimulation(prob)
+    assert sim.plan.resident
+    th, I = backend.time_evolution_core(prob, m, mI, sim=sim)
+    th_s, I_s = backend.time_evolution_core(prob, m, mI, fast_poisson=False)
+    th_o, I_o = rcsj_oracle.evolve(prob, m, mI)
+    scale = max(1.0, float(np.abs(th_o).max()))
+    assert float(np.abs(th - th_s).max()) <= 1e-10 * scale and float(np.abs(I - I_s).max()) <= 1e-9
+    assert float(np.abs(th - th_o).max()) <= 1e-9 * scale and float(np.abs(I - I_o).max()) <= 1e-9
+
+
+@pytest.mark.gpu
+def test_calls_chain_and_noise_is_the_same_as_step_by_step():
+    c = SquareArray(8, 7)
+    W, Nt = 4, 50
+    Is = c.current_base(0.0)[:, None, None] * np.linspace(0.3, 1.4, W)[None, :, None]
+    prob = TimeEvolutionProblem(c, time_step=0.05, time_step_count=Nt, current_sources=Is, external_flux=0.1,
+                                temperature=0.05)
+    import torch
+    a, b = backend.GpuSimulation(prob, seed=5), backend.GpuSimulation(prob, seed=5, fast_poisson=False)
+    assert a.plan.resident and not b.plan.resident
+    for n in (1, 7, 20, 3):
+        a.run(n)
+        b.run(n)
+    all_a = torch.empty((19, c._Nj(), W), dtype=torch.float64, device="cuda")
+    all_b = torch.empty_like(all_a)
+    a.run(19, None, None, all_a, None, store_all=True)
+    b.run(19, None, None, all_b, None, store_all=True)
+    a.synchronize()
+    b.synchronize()
+    assert float((all_a - all_b).abs().max()) <= 1e-10
+    for x, y in zip(a.history(), b.history()):
+        assert float((x - y).abs().max()) <= 1e-10
+
+
+@pytest.mark.gpu
+def test_non_finite_phases_are_reported():
+    from pyjjasim_gb300 import _native as N
+    c = SquareArray(6, 6)
+    Is = np.zeros((c._Nj(), 2, 1))
+    Is[3, 1] = np.nan
+    prob = TimeEvolutionProblem(c, time_step=0.05, time_step_count=5, current_sources=Is, external_flux=0.1)
+    sim = backend.GpuSimulation(prob)
+    assert sim.plan.resident
+    sim.run(5)
+    with pytest.raises(N.JJAError):
+        sim.synchronize()
+    sim.synchronize()   # reported once
