@@ -195,6 +195,13 @@ int jja_plan_set_sine_solver(jja_plan* p, int mx, int my, const int32_t* grid_fa
  * use_graph, with a host noise buffer, jja_run_timed, jja_solve and the adjoint keep the sweeps. The
  * history buffers keep their places in jja_state over such a call (no rotation). */
 int jja_plan_set_resident(jja_plan* p, const jja_factor* f);
+
+/* Face-space solves by products with dense blocks on the tensor cores (error-free digit products,
+ * FP64 results) instead of the triangular sweeps: leaf_faces = 0, the whole inverse (one launch per
+ * solve); else the inverses of the largest subtrees of at most leaf_faces faces of the factor's elimination tree,
+ * of the Schur complement of the other faces, and the couplings (three launches per solve). 12 bytes per
+ * matrix entry; at most 32768 blocks of 128 x 64. jja_solve_static keeps the sweeps. */
+int jja_plan_set_blocks(jja_plan* p, const jja_factor* f, int leaf_faces);
 /* Synchronises the device, then reads and clears the plan's device error flags: *flow_timeouts
  * = 1 if a wait of a dataflow sweep ran out of its bound since the last call (the results of
  * those steps are invalid), else 0. Returns JJA_ERR_NONFINITE when a time step of jja_run /

@@ -233,7 +233,7 @@ class GpuSimulation:
             self.relax, self.tuning = tuple(relax), dict(tuning or {})
             self.stream = stream if stream is not None else torch.cuda.Stream(device=self.dev)
             self.plan = P.get_plan(c, stage.dt, self.W, self.width, stage.stencil, nd_leaf=nd_leaf,
-                                   ordering=self.ordering, relax=relax, Ic_w=Ic, tuning=tuning,
+                                   ordering=ordering, relax=relax, Ic_w=Ic, tuning=tuning,
                                    fast_poisson=fast_poisson)
             self.hist0, self.hist0_zero = stage.hist0, stage.hist0_zero
             self.hist = []

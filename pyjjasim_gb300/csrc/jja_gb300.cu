@@ -184,6 +184,7 @@ struct StepArgs {
   jja_view Isq;        // Is / c0 for a time-independent Is (plan-owned, refreshed at the start of a run)
   const double* amp;   // sqrt(2 T Rv) / c0 per junction, for a time-independent T equal for all problems (likewise)
   int resistive;       // width 3 and no capacitance anywhere: c1 / c0 = -1, c2 = 0
+  double* zero_x;      // the face kernel also zeroes the solution here (the block solver accumulates into it)
 };
 
 struct Tables {
@@ -575,6 +576,7 @@ __global__ void __launch_bounds__(256) k_face_rhs(StepArgs a, Tables t, const do
     }
     if (a.f.ptr) acc = fma(-kTwoPi, view_at(a.f, __ldg(t.face_orig + p), w, tt), acc);
     b[e] = acc;
+    if (a.zero_x) a.zero_x[e] = 0.0;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) a.d_step[1] = step + 1;
 }
@@ -716,6 +718,7 @@ __global__ void __launch_bounds__(256) k_face_rhs_fast(StepArgs a, Tables t, con
       for (int u = 0; u < V; ++u) acc.v[u] = fma(-kTwoPi, __ldg(f + u * a.f.stride_w), acc.v[u]);
     }
     *reinterpret_cast<Vec*>(b + p * a.W + w) = acc;
+    if (a.zero_x) *reinterpret_cast<Vec*>(a.zero_x + p * a.W + w) = Vec{};
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) a.d_step[1] = a.d_step[0] + 1;
 }
@@ -1778,6 +1781,7 @@ __global__ void k_permute_rows(const double* __restrict__ src, double* __restric
 }  // namespace
 
 #include "jja_sine.cuh"
+#include "jja_block.cuh"
 #include "jja_resident.cuh"
 
 namespace {
@@ -2047,8 +2051,10 @@ void build_subtree_packs(const jja::Factor& F, Schedule& S, int WB, int w_lo, in
   S.sub_max_rows = S.sub_max_f = S.sub_max_n = S.sub_max_l = 0;
 }
 
-// the work items of problems [w_lo, w_hi) (w_hi < 0: all W); w_lo a multiple of the RHS block
-Schedule build_schedule(const jja::Factor& F, int W, const jja_solve_tuning& tu, int w_lo = 0, int w_hi = -1) {
+// the work items of problems [w_lo, w_hi) (w_hi < 0: all W); w_lo a multiple of the RHS block; without the
+// supernodes marked in `skip`
+Schedule build_schedule(const jja::Factor& F, int W, const jja_solve_tuning& tu, int w_lo = 0, int w_hi = -1,
+                        const std::vector<char>* skip = nullptr) {
   if (W <= 0 || W >= (1 << 30)) throw Error(JJA_ERR_ARG, "W must be in [1, 2^30)");
   for (int v : {tu.rows_per_lane, tu.rows_per_lane_fwd})
     if (v && v != 1 && v != 2 && v != 4 && v != 8)
@@ -2120,7 +2126,7 @@ Schedule build_schedule(const jja::Factor& F, int W, const jja_solve_tuning& tu,
   }
   std::vector<std::vector<int>> by_level(S.n_levels);
   for (int s = 0; s < F.ns; ++s)
-    if (!inside[s]) by_level[level[s]].push_back(s);
+    if (!inside[s] && !(skip && (*skip)[s])) by_level[level[s]].push_back(s);
   auto pack = [](int s, int r0, int r1, int w0, bool partial, int c_lo, int c_hi) {
     return make_int4(s, r0 | (r1 << 16), w0 | ((int)partial << 30), c_lo | (c_hi << 16));
   };
@@ -2441,6 +2447,7 @@ struct jja_plan {
   // tridiagonal solves, transform back; face vectors in grid order
   SineArgs sine_fwd{}, sine_bwd{};
   SineTri sine_tri{};
+  BlockList blocks[3];               // launches of the block solver (jja_plan_set_blocks; dst == 3)
   // whole runs of a small circuit in one launch (jja_plan_set_resident; inv null: not)
   ResidentArgs res{};
   int64_t* res_slots = nullptr;      // output slots of a call's steps (phases, then currents)
@@ -2686,8 +2693,25 @@ void launch_sine_solve(jja_plan* p, const Group& g, cudaStream_t st) {
   lines(p->sine_bwd, p->z, p->x);
 }
 
-// x = K^-1 b for group g: the two triangular sweeps, or sine transforms
-void launch_face_solve(jja_plan* p, const Group& g, cudaStream_t st) {
+// x = K^-1 b by products with dense blocks, accumulated into a zeroed x (b is changed); `zeroed`: the
+// face kernel has zeroed it
+void launch_block_solve(jja_plan* p, const Group& g, cudaStream_t st, bool zeroed) {
+  if (!zeroed) JJA_CUDA(cudaMemsetAsync(p->x, 0, (size_t)p->Nf * p->W * sizeof(double), st));
+  for (const BlockList& L : p->blocks) {
+    if (!L.n) continue;
+    const int wp = block_width(L.n, g.wn), ty = (g.wn + wp - 1) / wp;
+    const dim3 grid((unsigned)std::max(1, std::min(L.n, kNumSMs / ty)), (unsigned)ty);
+    launch_smem(p->pdl, block_kernel(wp), grid, kBlockThreads, block_smem_bytes(wp), st, L, p->b, p->x, p->W, g.w0, g.wn,
+                p->flow_err);
+  }
+}
+
+// x = K^-1 b for group g: the two triangular sweeps, sine transforms, or dense blocks
+void launch_face_solve(jja_plan* p, const Group& g, cudaStream_t st, bool zeroed = false) {
+  if (p->dst == 3) {
+    launch_block_solve(p, g, st, zeroed);
+    return;
+  }
   if (p->dst == 2) {
     launch_sine_solve(p, g, st);
     return;
@@ -2777,7 +2801,7 @@ void launch_step(jja_plan* p, const Group& g, StepArgs& a, cudaStream_t st, bool
   launch_face_rhs(p, a, st);
   if (ev) JJA_CUDA(cudaEventRecord(ev[1], st));
   if (p->dst) {
-    launch_face_solve(p, g, st);
+    launch_face_solve(p, g, st, true);
     if (ev) JJA_CUDA(cudaEventRecord(ev[2], st));
   } else {
     launch_levels(p, g, st, true);
@@ -2807,6 +2831,7 @@ StepArgs make_args(jja_plan* p, jja_state* s, const Group& g) {
   a.dt = p->dt;
   a.Isq = (s->Is.ptr && !s->Is.stride_t) ? jja_view{p->isq, p->W, 1, 0} : jja_view{nullptr, 0, 0, 0};
   a.resistive = p->resistive;
+  a.zero_x = p->dst == 3 ? p->x : nullptr;
   a.amp = (s->noise_mode != JJA_NOISE_NONE && s->T.ptr && !s->T.stride_t && !s->T.stride_w) ? p->amp : nullptr;
   return a;
 }
@@ -2905,6 +2930,187 @@ void run_resident(jja_plan* p, jja_state* s, int nsteps, const int64_t* th_slot,
                 resident_smem_bytes(g.n, g.nj, p->width - 1), st, a, p->t, g);
   }
 }
+
+// a plan whose solver changed: its step as one chain, no graphs that bake in the sweeps
+void one_chain(jja_plan* p) {
+  for (Group& g : p->groups) {
+    if (g.stream) cudaStreamDestroy(g.stream);
+    if (g.done) cudaEventDestroy(g.done);
+  }
+  p->groups.clear();
+  for (auto& g : p->graphs) cudaGraphExecDestroy(g.exec);
+  for (auto& g : p->adj_graphs) cudaGraphExecDestroy(g.exec);
+  p->graphs.clear();
+  p->adj_graphs.clear();
+}
+
+// The blocks of jja_plan_set_blocks and how they are computed. Leaves: the largest subtrees of the
+// elimination tree of at most leaf_faces columns (contiguous in the factor's order; every row outside
+// that a leaf touches is an off-diagonal row of its root); leaf_faces = 0: none, one block matrix.
+// Row lists: per leaf its columns and its root's rows, then the separators of every tree.
+// Columns of K_ll^-1 come 64 at a time from sweeps over the leaves alone: a batch holds leaves that
+// share no separator, so one set of columns serves them all and the forward sweep leaves each one's
+// -G_l^T in the separators' rows. S^-1 comes from sweeps over the separators alone.
+struct BlockSetup {
+  struct Chunk {
+    int c0, own0, n_own, couple0, n_couple;   // into jobs
+  };
+  struct Batch {
+    std::vector<int32_t> rows, pos;
+    std::vector<Chunk> chunks;
+  };
+  std::vector<int> leaf_of;               // per supernode: its leaf, or -1
+  std::vector<int32_t> lists;
+  std::vector<Batch> leaf_batches, top_batches;
+  std::vector<BlockUnit> units[3];
+  std::vector<BlockSource> sources;
+  std::vector<StoreRows> jobs;
+  int64_t store_size = 0, n_blocks = 0;
+
+  // blocks of a rows x cols matrix at `base` of the store with the given strides
+  void add_blocks(int launch, int from, int64_t base, int64_t s_r, int64_t s_c, int out_off, int rows, int in_off,
+                  int cols) {
+    for (int c = 0; c < cols; c += kBlockCols)
+      for (int r = 0; r < rows; r += kBlockRows) {
+        const int nr = std::min(kBlockRows, rows - r), nc = std::min(kBlockCols, cols - c);
+        units[launch].push_back({in_off + c, nc, out_off + r, nr, (int)n_blocks, from});
+        sources.push_back({base + r * s_r + c * s_c, s_r, s_c, nr, nc});
+        ++n_blocks;
+      }
+  }
+
+  BlockSetup(const jja::Factor& F, int leaf_faces) {
+    const int ns = F.ns;
+    std::vector<int> cols(ns), cnt(ns, 1);
+    for (int s = 0; s < ns; ++s) cols[s] = F.sn_k[s];
+    for (int s = 0; s < ns; ++s) {
+      const int q = F.sn_parent[s];
+      if (q < 0) continue;
+      if (q <= s || q >= ns) throw Error(JJA_ERR_INTERNAL, "supernodes are not in postorder");
+      cols[q] += cols[s];
+      cnt[q] += cnt[s];
+    }
+    struct Leaf {
+      int c0, n, m, root, cols_off, rows_off;
+      int64_t inv, gt;    // K_ll^-1 (n x n) and -G_l^T (m x n) in the store
+    };
+    std::vector<Leaf> leaves;
+    leaf_of.assign(ns, -1);
+    std::vector<char> sep(F.n, 1);
+    for (int t = 0; t < ns && leaf_faces > 0; ++t) {
+      const int q = F.sn_parent[t];
+      if (cols[t] > leaf_faces || (q >= 0 && cols[q] <= leaf_faces)) continue;
+      Leaf l{};
+      l.c0 = F.sn_col0[t - cnt[t] + 1];
+      l.n = cols[t];
+      l.m = F.sn_m[t];
+      l.root = t;
+      for (int s = t - cnt[t] + 1; s <= t; ++s) leaf_of[s] = (int)leaves.size();
+      for (int i = 0; i < l.n; ++i) sep[l.c0 + i] = 0;
+      leaves.push_back(l);
+    }
+    // the separators, tree by tree (the circuits of a ragged batch are trees of a forest: their Schur
+    // complements are independent)
+    std::vector<std::vector<int32_t>> trees(ns);
+    {
+      std::vector<int> root(ns);
+      for (int s = ns - 1; s >= 0; --s) {
+        root[s] = F.sn_parent[s] < 0 ? s : root[F.sn_parent[s]];
+        if (leaf_of[s] >= 0) continue;
+        for (int i = 0; i < F.sn_k[s]; ++i) trees[root[s]].push_back(F.sn_col0[s] + i);
+      }
+      trees.erase(std::remove_if(trees.begin(), trees.end(), [](const auto& t) { return t.empty(); }), trees.end());
+    }
+    for (Leaf& l : leaves) {
+      l.cols_off = (int)lists.size();
+      for (int i = 0; i < l.n; ++i) lists.push_back(l.c0 + i);
+      l.rows_off = (int)lists.size();
+      const int* R = F.rows.data() + F.sn_rowptr[l.root];
+      for (int i = 0; i < l.m; ++i) {
+        if (!sep[R[i]]) throw Error(JJA_ERR_INTERNAL, "a leaf's outside row is not a separator");
+        lists.push_back(R[i]);
+      }
+      l.inv = store_size;
+      l.gt = l.inv + (int64_t)l.n * l.n;
+      store_size = l.gt + (int64_t)l.m * l.n;
+      add_blocks(0, 1, l.gt, l.n, 1, l.rows_off, l.m, l.cols_off, l.n);        // b_s += (-G^T) b_l
+      add_blocks(0, 0, l.inv, l.n, 1, l.cols_off, l.n, l.cols_off, l.n);       // x_l += K_ll^-1 b_l
+      add_blocks(2, 2, l.gt, 1, l.n, l.cols_off, l.n, l.rows_off, l.m);        // x_l += (-G) x_s
+    }
+    Batch top;
+    int longest_top = 0;
+    std::vector<int64_t> sinv;
+    std::vector<int> sep_off;
+    for (const auto& t : trees) {
+      const int m = (int)t.size();
+      sep_off.push_back((int)lists.size());
+      sinv.push_back(store_size);
+      store_size += (int64_t)m * m;
+      lists.insert(lists.end(), t.begin(), t.end());
+      add_blocks(1, 0, sinv.back(), m, 1, sep_off.back(), m, sep_off.back(), m);   // x_s += S^-1 b_s
+      for (int i = 0; i < m; ++i) {
+        top.rows.push_back(t[i]);
+        top.pos.push_back(i);
+      }
+      longest_top = std::max(longest_top, m);
+    }
+    // leaves that share no separator into the same batch (greedy)
+    std::vector<std::vector<char>> used;
+    std::vector<std::vector<int>> members;
+    for (int i = 0; i < (int)leaves.size(); ++i) {
+      const int* R = F.rows.data() + F.sn_rowptr[leaves[i].root];
+      size_t c = 0;
+      for (;; ++c) {
+        if (c == used.size()) {
+          used.emplace_back(F.n, 0);
+          members.emplace_back();
+        }
+        bool free_of = true;
+        for (int k = 0; k < leaves[i].m && free_of; ++k) free_of = !used[c][R[k]];
+        if (free_of) break;
+      }
+      for (int k = 0; k < leaves[i].m; ++k) used[c][R[k]] = 1;
+      members[c].push_back(i);
+    }
+    for (const auto& mem : members) {
+      Batch t;
+      int longest = 0;
+      for (int i : mem) {
+        for (int k = 0; k < leaves[i].n; ++k) {
+          t.rows.push_back(leaves[i].c0 + k);
+          t.pos.push_back(k);
+        }
+        longest = std::max(longest, leaves[i].n);
+      }
+      for (int c0 = 0; c0 < longest; c0 += kBlockCols) {
+        Chunk c{c0, (int)jobs.size(), 0, 0, 0};
+        for (int i : mem)
+          if (leaves[i].n > c0)
+            jobs.push_back({leaves[i].inv + c0, leaves[i].n, 1, leaves[i].cols_off, leaves[i].n,
+                            std::min(kBlockCols, leaves[i].n - c0)});
+        c.n_own = (int)jobs.size() - c.own0;
+        c.couple0 = (int)jobs.size();
+        for (int i : mem)
+          if (leaves[i].n > c0 && leaves[i].m)
+            jobs.push_back({leaves[i].gt + c0, leaves[i].n, 1, leaves[i].rows_off, leaves[i].m,
+                            std::min(kBlockCols, leaves[i].n - c0)});
+        c.n_couple = (int)jobs.size() - c.couple0;
+        t.chunks.push_back(c);
+      }
+      leaf_batches.push_back(std::move(t));
+    }
+    for (int c0 = 0; c0 < longest_top; c0 += kBlockCols) {
+      Chunk c{c0, (int)jobs.size(), 0, 0, 0};
+      for (size_t i = 0; i < trees.size(); ++i) {
+        const int m = (int)trees[i].size();
+        if (m > c0) jobs.push_back({sinv[i] + c0, m, 1, sep_off[i], m, std::min(kBlockCols, m - c0)});
+      }
+      c.n_own = (int)jobs.size() - c.own0;
+      top.chunks.push_back(c);
+    }
+    if (longest_top) top_batches.push_back(std::move(top));
+  }
+};
 
 // graph of G fused steps for the state's current buffers (captured on first use, then cached);
 // with several groups the graph forks into their streams and joins back
@@ -3303,7 +3509,7 @@ int jja_plan_set_fast_poisson(jja_plan* p, int mx, int my, const int32_t* grid_f
     if (!p || !grid_face || mx < 1 || my < 1) throw Error(JJA_ERR_ARG, "jja_plan_set_fast_poisson: bad arguments");
     if ((int64_t)mx * my != p->Nf) throw Error(JJA_ERR_ARG, "jja_plan_set_fast_poisson: mx * my != Nf");
     if (!(kappa > 0.0)) throw Error(JJA_ERR_ARG, "jja_plan_set_fast_poisson: kappa must be positive");
-    if (p->dst == 2) throw Error(JJA_ERR_ARG, "jja_plan_set_fast_poisson: the plan solves by jja_plan_set_sine_solver");
+    if (p->dst > 1) throw Error(JJA_ERR_ARG, "jja_plan_set_fast_poisson: the plan already has another solver");
     auto log2_of = [](int n) {   // log2(2 n) for n a power of two (n = m + 1), else -1
       if (n < 2 || (n & (n - 1))) return -1;
       int l = 1;
@@ -3452,17 +3658,130 @@ int jja_plan_set_sine_solver(jja_plan* p, int mx, int my, const int32_t* grid_fa
     JJA_CUDA(cudaFuncSetAttribute(sine_kernel(kp), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sine_smem_bytes(kp)));
     // the step runs as one chain: its kernels fill the GPU (128x128 x 512: 0.477 ms per step, 0.519
     // as the three concurrent groups that the sweeps' levels want)
-    for (Group& gr : p->groups) {
-      if (gr.stream) cudaStreamDestroy(gr.stream);
-      if (gr.done) cudaEventDestroy(gr.done);
-    }
-    p->groups.clear();
-    // graphs captured before bake in the sweeps: drop them
-    for (auto& g2 : p->graphs) cudaGraphExecDestroy(g2.exec);
-    for (auto& g2 : p->adj_graphs) cudaGraphExecDestroy(g2.exec);
-    p->graphs.clear();
-    p->adj_graphs.clear();
+    one_chain(p);
     p->dst = 2;
+  });
+}
+
+int jja_plan_set_blocks(jja_plan* p, const jja_factor* fac, int leaf_faces) {
+  return guarded([&] {
+    if (!p || !fac || leaf_faces < 0) throw Error(JJA_ERR_ARG, "jja_plan_set_blocks: bad arguments");
+    const jja::Factor& F = *fac->f;
+    const int n = p->Nf, ns = F.ns;
+    if (F.n != n) throw Error(JJA_ERR_ARG, "jja_plan_set_blocks: factor order != Nf");
+    if (p->dst || p->res.inv) throw Error(JJA_ERR_ARG, "jja_plan_set_blocks: the plan already has another solver");
+    BlockSetup B(F, leaf_faces);
+    if (B.n_blocks > kBlocksMax)
+      throw Error(JJA_ERR_ARG, "jja_plan_set_blocks: " + std::to_string(B.n_blocks) + " blocks of the matrix, more than " +
+                                   std::to_string(kBlocksMax));
+    // device scratch of the setup
+    struct Scratch {
+      std::vector<void*> mem;
+      cudaStream_t st = nullptr;
+      ~Scratch() {
+        if (st) cudaStreamDestroy(st);
+        for (void* m : mem) cudaFree(m);
+      }
+    } tmp;
+    int64_t ignored = 0;
+    auto scratch = [&](auto* h, size_t count) {
+      auto* d = upload(h, count, ignored);
+      tmp.mem.push_back((void*)d);
+      return d;
+    };
+    const int64_t nW = (int64_t)n * kBlockCols;
+    double* b = scratch((const double*)nullptr, (size_t)nW);
+    double* z = scratch((const double*)nullptr, (size_t)nW);
+    double* x = scratch((const double*)nullptr, (size_t)nW);
+    double* store = scratch((const double*)nullptr, (size_t)B.store_size);
+    JJA_CUDA(cudaStreamCreateWithFlags(&tmp.st, cudaStreamNonBlocking));
+    cudaStream_t st = tmp.st;
+    JJA_CUDA(cudaDeviceSynchronize());
+    // level sweeps over the supernodes of one part of the tree, 64 columns at a time
+    jja_solve_tuning tu{};
+    tu.subtree_rows = tu.pack_rows = -1;
+    tu.rows_per_lane = tu.rows_per_lane_fwd = 1;
+    constexpr int kW = kBlockCols, kWB = 32;
+    struct Part {
+      Schedule S;
+      int4 *fi, *bi;
+      int32_t *zf, *zb;
+    };
+    auto make_part = [&](const std::vector<char>& skip) {
+      Part P{build_schedule(F, kW, tu, 0, -1, &skip), nullptr, nullptr, nullptr, nullptr};
+      P.fi = scratch(P.S.fi.data(), P.S.fi.size());
+      P.bi = scratch(P.S.bi.data(), P.S.bi.size());
+      P.zf = scratch(P.S.zf.data(), P.S.zf.size());
+      P.zb = scratch(P.S.zb.data(), P.S.zb.size());
+      return P;
+    };
+    auto zero_rows = [&](double* v, const int32_t* rows, size_t count) {
+      if (count)
+        launch(false, k_zero_rows, grid_for((int64_t)count * kW, 256), 256, st, v, rows, (int)count, kW, 0, kW,
+               fast_div(kW), (unsigned*)nullptr, 0);
+    };
+    auto forward = [&](const Part& P) {
+      zero_rows(z, P.zf, P.S.zf.size());
+      for (int l = 0; l < P.S.n_levels; ++l)
+        if (const int m = (int)(P.S.fwd_ptr[l + 1] - P.S.fwd_ptr[l]))
+          launch(false, k_fwd_level<1, false>, (m + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, st, p->F,
+                 (const int4*)(P.fi + P.S.fwd_ptr[l]), m, kW, kWB, b, z);
+    };
+    auto backward = [&](const Part& P) {
+      zero_rows(x, P.zb, P.S.zb.size());
+      for (int l = P.S.n_levels - 1; l >= 0; --l)
+        if (const int m = (int)(P.S.bwd_ptr[l + 1] - P.S.bwd_ptr[l]))
+          launch(false, k_bwd_level<1, false>, (m + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, st, p->F,
+                 (const int4*)(P.bi + P.S.bwd_ptr[l]), m, kW, kWB, (const double*)z, x);
+    };
+    auto clear = [&](double* v) { JJA_CUDA(cudaMemsetAsync(v, 0, nW * sizeof(double), st)); };
+    std::vector<char> leaf_only(ns), top_only(ns);
+    for (int s = 0; s < ns; ++s) {
+      leaf_only[s] = B.leaf_of[s] < 0;    // skip the separators
+      top_only[s] = B.leaf_of[s] >= 0;    // skip the leaves
+    }
+    int32_t* lists = p->up(B.lists.data(), B.lists.size());
+    const StoreRows* jobs = scratch(B.jobs.data(), B.jobs.size());
+    auto store_rows = [&](const double* v, int first, int count) {
+      if (count)
+        launch(false, k_store_rows, count, 256, st, v, (const int32_t*)lists, (const StoreRows*)(jobs + first), store);
+    };
+    auto run = [&](const std::vector<BlockSetup::Batch>& batches, const Part& P, bool leaves) {
+      for (const BlockSetup::Batch& t : batches) {
+        const int32_t* rows = scratch(t.rows.data(), t.rows.size());
+        const int32_t* pos = scratch(t.pos.data(), t.pos.size());
+        for (const BlockSetup::Chunk& c : t.chunks) {
+          clear(b);
+          launch(false, k_unit_columns, grid_for((int64_t)t.rows.size(), 256), 256, st, b, rows, pos, (int)t.rows.size(),
+                 c.c0);
+          forward(P);
+          store_rows(b, c.couple0, c.n_couple);   // the separators' rows of b now hold -G_l^T
+          if (leaves) clear(x);                   // zero at the separators
+          backward(P);
+          store_rows(x, c.own0, c.n_own);
+        }
+      }
+    };
+    if (!B.leaf_batches.empty()) run(B.leaf_batches, make_part(leaf_only), true);
+    run(B.top_batches, make_part(top_only), false);
+    unsigned char* mats = p->up<unsigned char>(nullptr, (size_t)B.n_blocks * kBlockMatBytes);
+    int* e_mat = p->up<int>(nullptr, (size_t)B.n_blocks);
+    BlockSource* src = scratch(B.sources.data(), B.sources.size());
+    launch(false, k_block_digits, (int)B.n_blocks, 256, st, (const double*)store, (const BlockSource*)src, mats, e_mat);
+    JJA_CUDA(cudaStreamSynchronize(st));
+    for (int k = 0; k < 3; ++k) {
+      BlockList L{};
+      L.n = (int)B.units[k].size();
+      if (L.n) L.units = p->up(B.units[k].data(), B.units[k].size());
+      L.in_rows = L.out_rows = lists;
+      L.mats = mats;
+      L.e_mat = e_mat;
+      p->blocks[k] = L;
+    }
+    for (int wp : {16, 32, 48, 64})
+      JJA_CUDA(cudaFuncSetAttribute(block_kernel(wp), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem_bytes(wp)));
+    one_chain(p);
+    p->dst = 3;
   });
 }
 
@@ -3922,7 +4241,7 @@ int jja_run_timed(jja_plan* p, jja_state* s, int nsteps, double* stage_ms, void*
       });
       // (a fast Poisson plan solves in the "forward" stage; its "backward" stage is empty)
       stage(2, [&](size_t q, cudaStream_t gst) {
-        if (p->dst) launch_face_solve(p, *gs[q], gst);
+        if (p->dst) launch_face_solve(p, *gs[q], gst, true);
         else launch_levels(p, *gs[q], gst, true);
       });
       stage(3, [&](size_t q, cudaStream_t gst) {

@@ -217,6 +217,32 @@ def resident_fits(circuit, W):
     return circuit._Nf() <= RESIDENT_MAX_FACES and circuit._Nj() <= RESIDENT_MAX_JUNCTIONS and W <= RESIDENT_MAX_W
 
 
+# Other circuits solve by products with dense blocks on the tensor cores: the whole inverse (leaf 0),
+# or the inverses of subtrees of up to `leaf` faces with the separators' Schur complement (3 launches).
+# Measured on GB300 (us per step, W problems; sweeps / inverse / leaves of 256):
+#   honeycomb 24x24 (1081 faces)   W = 1  48 / 14 / 20    W = 24  58 / 20 / 25    W = 96  103 / 34 / 31
+#   honeycomb 31x31 (1830 faces)   W = 1  55 / 17 / 21    W = 24  70 / 27 / 28    W = 96  115 / 63 / 40
+#   triangular 64x48 (11970 faces) W = 1  89 / - / 33     W = 24  145 / - / 61    W = 96  240 / - / 145
+#   triangular 80x80 (25122 faces) W = 1  97 / - / 66     W = 24  188 / - / 111   W = 256 906 / - / 734
+# and with leaves of 384:
+#   square 230x200, R spread (45571) W = 1  141 / 139     W = 4  157 / 154        W = 24  380 / 247
+#   square 300x300, R spread (89401) W = 1  204 / 317     W = 4  254 / 362        W = 24  670 / 588
+INVERSE_MAX_FACES = 2048
+INVERSE_MAX_WORK = 11000    # 128 x 64 blocks of the inverse x problems
+
+
+def block_leaf(circuit, W):
+    """The leaf size of the block solver that the default plan takes for W problems, or None."""
+    n = circuit._Nf()
+    if n <= INVERSE_MAX_FACES and -(-n // 128) * -(-n // 64) * W <= INVERSE_MAX_WORK:
+        return 0
+    if n <= 1 << 15:
+        return 256
+    if W >= 8 and n <= 1 << 16 or W >= 24 and n <= 92000:
+        return 384
+    return None
+
+
 def untuned(tuning):
     """True when ``tuning`` asks for nothing but the level schedule (the library's default)."""
     t = dict(tuning or {})
@@ -227,7 +253,7 @@ class DevicePlan:
     """Circuit tables + factor uploaded for W problems (owned C object)."""
 
     def __init__(self, circuit, factor, A, W, dt, stencil_width, stencil, Ic_w=None, tuning=None, fast_poisson=None,
-                 sine=None, resident=False):
+                 sine=None, resident=False, blocks=None):
         """``tuning``: dict with any of rhs_block, rows_per_lane, target_warps, min_piece (the
         launch shape of the triangular solves; missing or 0 = library default)."""
         Nj, Nf = circuit._Nj(), circuit._Nf()
@@ -275,6 +301,9 @@ class DevicePlan:
         if resident:
             N.check(N.lib().jja_plan_set_resident(h, factor.handle))
             self.resident = True
+        self.blocks = blocks
+        if blocks is not None:
+            N.check(N.lib().jja_plan_set_blocks(h, factor.handle, int(blocks)))
         self.device_bytes = N.lib().jja_plan_device_bytes(h)
 
     def solve(self, b_dev, x_dev, stream=0):
@@ -382,8 +411,6 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
     DevicePlan); ``fast_poisson``: solve with sine transforms when the face-space matrix allows it
     (fast_poisson_grid): True, False, or "auto" (W <= 8 and W x Nf <= 2^18 face-problems; the
     tensor-core transforms by sine_solver_fits)."""
-    ordering = resolve_ordering(ordering, W, circuit._Nf())
-    nd_leaf, relax = resolve_factor_shape(nd_leaf, relax, ordering, W, circuit._Nf())
     fp = None
     matrices = face_matrix(circuit, dt)
     resident = fast_poisson == "auto" and untuned(tuning) and resident_fits(circuit, W)
@@ -395,13 +422,21 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
         sine = poisson_grid(circuit, matrices[1])
         if sine is not None and not sine_solver_fits(sine, W):
             sine = None
+    blocks = None
+    if fp is None and sine is None and not resident and fast_poisson == "auto" and untuned(tuning):
+        blocks = block_leaf(circuit, W)
+    if blocks is not None:     # the block solver cuts the tree itself: nested dissection with small leaves
+        nd_leaf = 8 if nd_leaf is None else nd_leaf
+        ordering = "nd" if ordering == "auto" else ordering
+    ordering = resolve_ordering(ordering, W, circuit._Nf())
+    nd_leaf, relax = resolve_factor_shape(nd_leaf, relax, ordering, W, circuit._Nf())
     factor, A, fkey = get_factor(circuit, dt, nd_leaf, ordering=ordering, relax=relax, matrices=matrices)
     Rv, Cv, coef = coefficients(circuit, dt, stencil)
     if Ic_w is not None:
         Ic_w = np.ascontiguousarray(np.broadcast_to(np.asarray(Ic_w, np.float64), (circuit._Nj(), W)))
     ic = np.asarray(circuit._Ic(), np.float64) if Ic_w is None else Ic_w
     tkey = tuple(int((tuning or {}).get(f, 0)) for f in TUNING_FIELDS)
-    key = (fkey, W, stencil_width, Ic_w is None, tkey, fp is not None, sine is not None, resident,
+    key = (fkey, W, stencil_width, Ic_w is None, tkey, fp is not None, sine is not None, resident, blocks,
            _digest(ic, *coef, Rv, A.indptr, A.indices, A.data))
     with _CACHE_LOCK:
         p = _PLANS.get(key)
@@ -409,7 +444,7 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
             _PLANS.move_to_end(key)
             return p
     p = DevicePlan(circuit, factor, A, W, dt, stencil_width, stencil, Ic_w=Ic_w, tuning=tuning, fast_poisson=fp,
-                   sine=sine, resident=resident)
+                   sine=sine, resident=resident, blocks=blocks)
     with _CACHE_LOCK:
         _PLANS[key] = p
         while len(_PLANS) > MAX_PLANS:

@@ -1,0 +1,92 @@
+"""Face solves by dense blocks on the tensor cores (jja_plan_set_blocks) against scipy and the sweeps.
+
+Sizes around its blocks of 128 x 64 entries and tiles of 16 to 64 problems. The bar against scipy is
+the one of the other face solves (1e-11 of the largest value per problem); residuals are compared with
+the triangular sweeps', which the blocks stand in for."""
+import numpy as np
+import pytest
+import scipy.sparse.linalg
+
+from oracle import rcsj_oracle
+from pyjjasim_gb300 import TimeEvolutionProblem, backend
+from pyjjasim_gb300 import plan as P
+from pyjjasim_gb300.circuit import HoneycombArray, SquareArray, TriangularArray
+
+
+def test_rule():
+    assert P.block_leaf(HoneycombArray(24, 24), 61) == 0
+    assert P.block_leaf(HoneycombArray(24, 24), 700) == 256
+    assert P.block_leaf(SquareArray(301, 301), 24) == 384 and P.block_leaf(SquareArray(301, 301), 8) is None
+
+
+def _solve(c, b, leaf):
+    import torch
+    A, K = P.face_matrix(c, 0.05)
+    factor, A, _ = P.get_factor(c, 0.05)
+    pl = P.DevicePlan(c, factor, A, b.shape[1], 0.05, 3, ((1.0, -1.0, 0.0), (1.0, -2.0, 1.0)), blocks=leaf)
+    bd = torch.from_numpy(b).cuda()
+    xd = torch.empty_like(bd)
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    pl.solve(bd.data_ptr(), xd.data_ptr(), s.cuda_stream)
+    s.synchronize()
+    pl.check()
+    return xd.cpu().numpy(), K
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lattice,nx,ny,W,leaf", [
+    (SquareArray, 2, 2, 1, 0), (SquareArray, 9, 9, 16, 0), (SquareArray, 14, 6, 17, 0), (SquareArray, 17, 9, 48, 0),
+    (SquareArray, 44, 4, 49, 0), (SquareArray, 14, 15, 64, 0), (HoneycombArray, 12, 12, 65, 0),
+    (TriangularArray, 10, 9, 15, 0), (TriangularArray, 24, 21, 130, 0), (HoneycombArray, 40, 40, 3, 0),
+    (SquareArray, 9, 9, 5, 8), (SquareArray, 40, 33, 33, 64), (HoneycombArray, 30, 24, 61, 200),
+    (TriangularArray, 40, 30, 20, 448), (SquareArray, 90, 70, 2, 300), (SquareArray, 12, 12, 3, 4000)])
+def test_solve_matches_scipy(lattice, nx, ny, W, leaf):
+    c = lattice(nx, ny)
+    rng = np.random.default_rng(nx * ny + W)
+    c.set_resistance(rng.lognormal(0.0, 0.4, c._Nj()))
+    c.set_inductance(0.05)
+    Nf = c._Nf()
+    b = rng.standard_normal((Nf, W)) * 10.0 ** rng.uniform(-12, 12, (1, W))
+    b[:, 0] = 1.0
+    if W > 1:
+        b[:, 1] = 0.0
+    x, K = _solve(c, b, leaf)
+    ref = scipy.sparse.linalg.spsolve(K.tocsc(), b).reshape(x.shape)
+    err = np.abs(x - ref).max(0) / np.maximum(np.abs(ref).max(0), 1e-300)
+    assert float(err.max()) <= 1e-11, err.argmax()
+    y, _ = _solve(c, b, None)
+    rx, ry = (np.linalg.norm(K @ v - b, axis=0) / np.maximum(np.linalg.norm(b, axis=0), 1e-300) for v in (x, y))
+    print(f"Nf={Nf} W={W}: residual {rx.max():.2e}, sweeps {ry.max():.2e}")
+    assert rx.max() <= max(4.0 * ry.max(), 1e-13)
+
+
+@pytest.mark.gpu
+def test_non_finite_values_stay_in_their_problem():
+    c = HoneycombArray(14, 13)
+    b = np.random.default_rng(1).standard_normal((c._Nf(), 20))
+    good = _solve(c, b, 0)[0]
+    b[17, 2], b[200, 4] = np.nan, np.inf
+    x = _solve(c, b, 0)[0]
+    rest = [w for w in range(20) if w not in (2, 4)]
+    assert np.isnan(x[:, [2, 4]]).all()
+    np.testing.assert_allclose(x[:, rest], good[:, rest], rtol=1e-13, atol=1e-15 * np.abs(good).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lattice,nx,ny,W,width", [(HoneycombArray, 16, 12, 33, 3), (TriangularArray, 15, 14, 5, 4)])
+def test_trajectory_matches_sweeps_and_oracle(lattice, nx, ny, W, width):
+    c = lattice(nx, ny)
+    c.set_capacitance(0.4)
+    Is = c.current_base(0.0)[:, None, None] * np.linspace(0.4, 1.4, W)[None, :, None]
+    prob = TimeEvolutionProblem(c, time_step=0.05, time_step_count=120, current_sources=Is, external_flux=0.13,
+                                store_time_steps=np.arange(0, 120, 25), stencil_width=width)
+    m = prob.store_time_steps
+    assert backend.GpuSimulation(prob).plan.blocks is not None
+    th, I = backend.time_evolution_core(prob, m, m)
+    th_s, I_s = backend.time_evolution_core(prob, m, m, fast_poisson=False)
+    th_o, I_o = rcsj_oracle.evolve(prob, m, m)
+    scale = max(1.0, float(np.abs(th_o).max()))
+    assert float(np.abs(th - th_s).max()) <= 1e-10 * scale
+    assert float(np.abs(th - th_o).max()) <= 1e-9 * scale
+    assert float(np.abs(I - I_o).max()) <= 1e-9
