@@ -182,11 +182,11 @@ int64_t jja_plan_device_bytes(const jja_plan* p);
 int jja_plan_set_fast_poisson(jja_plan* p, int mx, int my, const int32_t* grid_face, double kappa);
 
 /* The same solve with the sine transforms as tensor-core contractions (error-free digit products, FP64
- * results) along one axis of the grid and tridiagonal solves along the other: for plans of many
- * problems. K = kappa (4 I - adjacency) on an mx x my grid of faces of any size whose shorter side
- * has at most 128 faces; grid_face[iy * mx + ix] is the face at (ix, iy) in the caller's order.
- * Replaces the plan's triangular sweeps (jja_solve_static keeps them). Not on a plan that already solves
- * by sine transforms. */
+ * results) along one axis of the grid and tridiagonal solves along the other: K = kappa (4 I - adjacency)
+ * on an mx x my grid of faces of any size up to 4096 a side (grids longer than 128 faces both ways are cut
+ * into strips, joined by a direct solve on the lines between them); grid_face[iy * mx + ix] is the
+ * face at (ix, iy) in the caller's order. Replaces the plan's triangular sweeps (jja_solve_static keeps
+ * them). Not on a plan that already has another solver. */
 int jja_plan_set_sine_solver(jja_plan* p, int mx, int my, const int32_t* grid_face, double kappa);
 
 /* Steps of a small circuit (at most 160 faces and 1024 junctions, and their state and the inverse of

@@ -2445,8 +2445,15 @@ struct jja_plan {
   DstArgs dst_args{};
   // sine transforms on the tensor cores (jja_plan_set_sine_solver; dst == 2): first transform,
   // tridiagonal solves, transform back; face vectors in grid order
-  SineArgs sine_fwd{}, sine_bwd{};
-  SineTri sine_tri{};
+  struct SineClass {                 // the strips of one width (one class, one strip: the whole grid)
+    SineArgs fwd{}, bwd{};
+    SineTri tri{};
+    const double* es = nullptr;      // weights of u0 at the strips' edges
+    int strip0 = 0, strips = 1;
+  };
+  std::vector<SineClass> sine;
+  SineStrips strips{};
+  BlockList sep_dst{};               // the dense sine matrix along the separators
   BlockList blocks[3];               // launches of the block solver (jja_plan_set_blocks; dst == 3)
   // whole runs of a small circuit in one launch (jja_plan_set_resident; inv null: not)
   ResidentArgs res{};
@@ -2677,7 +2684,15 @@ void launch_levels(jja_plan* p, const Group& g, cudaStream_t st, bool forward) {
 }
 
 
-// the sine-transform solve on the tensor cores: b -> z (transform), in place (tridiagonal), -> x
+void launch_block_list(jja_plan* p, const BlockList& L, double* b, double* x, int W, int w0, int wn, cudaStream_t st) {
+  if (!L.n) return;
+  const int wp = block_width(L.n, wn), ty = (wn + wp - 1) / wp;
+  const dim3 grid((unsigned)std::max(1, std::min(L.n, kNumSMs / ty)), (unsigned)ty);
+  launch_smem(p->pdl, block_kernel(wp), grid, kBlockThreads, block_smem_bytes(wp), st, L, b, x, W, w0, wn, p->flow_err);
+}
+
+// the sine-transform solve on the tensor cores: b -> z (transform), chains, -> x (transform back);
+// with strips z keeps the transformed right-hand side for the second pass over the chains
 void launch_sine_solve(jja_plan* p, const Group& g, cudaStream_t st) {
   auto lines = [&](SineArgs d, const double* in, double* out) {
     const int64_t tiles = ((int64_t)d.lines * g.wn + kSineColumns - 1) / kSineColumns;
@@ -2686,24 +2701,49 @@ void launch_sine_solve(jja_plan* p, const Group& g, cudaStream_t st) {
     launch_smem(p->pdl, sine_kernel(d.kp), dim3(grid), kSineThreads, sine_smem_bytes(d.kp), st, d, in, out, g.w0, g.wn,
                 fast_div(g.wn), p->flow_err);
   };
-  const SineTri& t = p->sine_tri;
-  const unsigned tri = (unsigned)(((int64_t)t.lines * g.wn + kTriColumns - 1) / kTriColumns);
-  lines(p->sine_fwd, p->b, p->z);
-  launch_smem(p->pdl, k_sine_tri, dim3(tri), 2 * kTriColumns, 0, st, t, p->z, g.w0, g.wn, fast_div(g.wn));
-  lines(p->sine_bwd, p->z, p->x);
+  auto chains = [&](const SineTri& t, const double* in, double* out, bool sep) {
+    if (t.segs) {
+      launch_smem(p->pdl, sep ? k_sine_chain<true> : k_sine_chain<false>,
+                  dim3((unsigned)(((int64_t)t.lines * g.wn + 31) / 32)), 32 * t.segs, 0, st, t, in, out, p->W, g.w0, g.wn,
+                  fast_div(g.wn));
+      return;
+    }
+    const unsigned grid = (unsigned)(((int64_t)t.lines * g.wn + kTriColumns - 1) / kTriColumns);
+    launch_smem(p->pdl, sep ? k_sine_tri<true> : k_sine_tri<false>, dim3(grid), 2 * kTriColumns, 0, st, t, in, out, p->W,
+                g.w0, g.wn, fast_div(g.wn));
+  };
+  const SineStrips& S = p->strips;
+  for (const auto& c : p->sine) lines(c.fwd, p->b, p->z);
+  if (!S.seps) {
+    for (const auto& c : p->sine) chains(c.tri, p->z, p->z, false);
+    for (const auto& c : p->sine) lines(c.bwd, p->z, p->x);
+    return;
+  }
+  const int W = p->W;   // such plans step all problems as one chain
+  double* u = p->b;     // the strips' part of b; its separators stay
+  for (const auto& c : p->sine) {
+    chains(c.tri, p->z, u, false);
+    const bool lanes = 32 % W == 0 || W % 32 == 0;
+    const int tw = lanes ? std::min(W, 32) : std::min(W, 256);
+    launch_smem(p->pdl, k_sine_edges, dim3((unsigned)(lanes ? (S.n + 7) / 8 : S.n), (unsigned)c.strips,
+                (unsigned)((W + tw - 1) / tw)), 256, 0, st, (const double*)u, c.es, c.tri.lines / c.strips, c.tri.off,
+                c.tri.s_strip, c.tri.s_n, c.tri.s_c, c.strip0, S.seps + 1, S.n, W, S.edge);
+  }
+  const int64_t ns = (int64_t)S.n * S.seps * W;
+  launch(p->pdl, k_sep_rhs, grid_for(ns, 256), 256, st, S, (const double*)p->b, W, fast_div(W));
+  launch_block_list(p, p->sep_dst, S.rhs, S.hat, S.seps * W, 0, S.seps * W, st);
+  launch(p->pdl, k_sep_solve, grid_for((int64_t)S.n * W, 256), 256, st, S, W, fast_div(W));
+  launch_block_list(p, p->sep_dst, S.hat, S.g, S.seps * W, 0, S.seps * W, st);
+  launch(p->pdl, k_sep_store, grid_for(ns, 256), 256, st, S, p->x, W, fast_div(W));
+  for (const auto& c : p->sine) chains(c.tri, p->z, u, true);
+  for (const auto& c : p->sine) lines(c.bwd, u, p->x);
 }
 
 // x = K^-1 b by products with dense blocks, accumulated into a zeroed x (b is changed); `zeroed`: the
 // face kernel has zeroed it
 void launch_block_solve(jja_plan* p, const Group& g, cudaStream_t st, bool zeroed) {
   if (!zeroed) JJA_CUDA(cudaMemsetAsync(p->x, 0, (size_t)p->Nf * p->W * sizeof(double), st));
-  for (const BlockList& L : p->blocks) {
-    if (!L.n) continue;
-    const int wp = block_width(L.n, g.wn), ty = (g.wn + wp - 1) / wp;
-    const dim3 grid((unsigned)std::max(1, std::min(L.n, kNumSMs / ty)), (unsigned)ty);
-    launch_smem(p->pdl, block_kernel(wp), grid, kBlockThreads, block_smem_bytes(wp), st, L, p->b, p->x, p->W, g.w0, g.wn,
-                p->flow_err);
-  }
+  for (const BlockList& L : p->blocks) launch_block_list(p, L, p->b, p->x, p->W, g.w0, g.wn, st);
 }
 
 // x = K^-1 b for group g: the two triangular sweeps, sine transforms, or dense blocks
@@ -3573,8 +3613,8 @@ int jja_plan_set_sine_solver(jja_plan* p, int mx, int my, const int32_t* grid_fa
     if ((int64_t)mx * my != p->Nf) throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: mx * my != Nf");
     if (!(kappa > 0.0) || !std::isfinite(kappa))
       throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: kappa must be positive and finite");
-    if (std::min(mx, my) > kSineMaxPoints)
-      throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: the shorter side must have at most 128 faces");
+    if ((int64_t)std::max(mx, my) > kSineMaxSide)
+      throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: a side of more than " + std::to_string(kSineMaxSide) + " faces");
     if (p->dst) throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: the plan already solves by sine transforms");
     const int Nf = p->Nf, W = p->W;
     // the tables again with the faces in grid order: cell iy * mx + ix
@@ -3606,58 +3646,221 @@ int jja_plan_set_sine_solver(jja_plan* p, int mx, int my, const int32_t* grid_fa
       }
       fill_ell(ft, Nf);
     }
-    // transforms along x (lines are grid rows) when the rows are the shorter side or both fit and
-    // rows keep the tridiagonal chains' loads contiguous for few problems; else along y
-    const bool along_x = mx <= my || mx <= kSineMaxPoints;
+    // one strip: transforms along x when its side fits, else along y; strips: along the longer side
+    const bool one = std::min(mx, my) <= kSineMaxPoints;
+    auto strips_of = [](int side) { return (side + 1 + kSineMaxPoints) / (kSineMaxPoints + 1); };
+    // strips of one width need half the launches of two widths: that side first, else the longer one
+    const bool even_x = (mx + 1) % strips_of(mx) == 0, even_y = (my + 1) % strips_of(my) == 0;
+    const bool along_x = one ? mx <= kSineMaxPoints : (even_x != even_y ? even_x : mx >= my);
     const int m = along_x ? mx : my, n = along_x ? my : mx;
-    const int kp = (m - m / 2 + 15) / 16 * 16;
-    const int64_t sx = W, sy = (int64_t)mx * W;
-    SineArgs d{};
-    d.m = m;
-    d.kp = kp;
-    d.lines = n;
-    d.s_t = along_x ? sx : sy;
-    d.s_c = along_x ? sy : sx;
-    int e = 0;
-    const long double scale = frexpl(2.0L / ((long double)(m + 1) * kappa), &e);   // in [1/2, 1) 2^e
-    const std::vector<uint16_t> plain = sine_matrix(m, kp, 1.0L), scaled = sine_matrix(m, kp, scale);
-    // the tridiagonal factors, eliminated from either end (the chain is symmetric)
-    SineTri t{};
-    t.n = n;
-    t.lines = m;
-    t.top = n / 2;
-    t.s_n = d.s_c;
-    t.s_c = d.s_t;
-    const int longest = n - t.top;
-    std::vector<double> c((size_t)longest * m), g(2 * (size_t)m);
+    const int64_t sx = W, sy = (int64_t)mx * W, s_t = along_x ? sx : sy, s_n = along_x ? sy : sx;
+    // strips of equal or two neighbouring widths: m + 1 = sum of (width + 1)
+    const int P = one ? 1 : strips_of(m);
+    const int narrow = (m + 1) / P - 1, n_wide = (m + 1) % P;
     const long double pi_l = 3.141592653589793238462643383279502884L;
-    for (int k = 0; k < m; ++k) {
-      const long double s = sinl(pi_l * (k + 1) / (2.0L * (m + 1)));
-      const long double diag = 2.0L + 4.0L * s * s;
-      long double r = 0.0L, ctop = 0.0L;
-      for (int i = 0; i < longest; ++i) {
-        r = 1.0L / (diag - r);
-        c[(size_t)i * m + k] = (double)r;
-        if (i == t.top - 1) ctop = r;
-      }
-      g[k] = (double)(ctop / (1.0L - ctop * r));
-      g[(size_t)m + k] = (double)(r / (1.0L - ctop * r));
-    }
     set_face_tables(p->t, ft, [&](auto* h, size_t n) { return p->up(h, n); });
     p->perm_factor = p->perm;
     p->perm = p->up(grid_face, (size_t)Nf);
-    t.c = p->up(c.data(), c.size());
-    t.g = p->up(g.data(), g.size());
-    d.mat = reinterpret_cast<const unsigned char*>(p->up(plain.data(), plain.size()));
-    d.e_shift = 0;
-    p->sine_fwd = d;
-    d.mat = reinterpret_cast<const unsigned char*>(p->up(scaled.data(), scaled.size()));
-    d.e_shift = e;
-    p->sine_bwd = d;
-    p->sine_tri = t;
-    JJA_CUDA(cudaFuncSetAttribute(sine_kernel(kp), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sine_smem_bytes(kp)));
-    // the step runs as one chain: its kernels fill the GPU (128x128 x 512: 0.477 ms per step, 0.519
-    // as the three concurrent groups that the sweeps' levels want)
+    p->sine.clear();
+    SineStrips S{};
+    S.n = n;
+    S.seps = P - 1;
+    S.s_n = s_n;
+    S.s_x = s_t;
+    S.inv_kappa = 1.0 / kappa;
+    if (P > 1) {
+      const size_t seps = (size_t)S.seps, cells = (size_t)n * seps;
+      S.rhs = p->up<double>(nullptr, cells * W);
+      S.hat = p->up<double>(nullptr, cells * W);
+      S.g = p->up<double>(nullptr, cells * W);
+      S.edge = p->up<double>(nullptr, (size_t)n * P * 2 * W);
+    }
+    for (int cls = 0, strip = 0, x0 = 0; cls < 2; ++cls) {   // the wide strips first
+      const int count = cls ? P - n_wide : n_wide, len = cls ? narrow : narrow + 1;
+      if (!count) continue;
+      const int kp = (len - len / 2 + 15) / 16 * 16;
+      jja_plan::SineClass c;
+      c.strip0 = strip;
+      c.strips = count;
+      SineArgs d{};
+      d.m = len;
+      d.kp = kp;
+      d.lines = n * count;
+      d.s_t = s_t;
+      d.s_c = s_n;
+      d.off = (int64_t)x0 * s_t;
+      d.s_strip = (int64_t)(len + 1) * s_t;
+      d.per_strip = fast_div(n);
+      int e = 0;
+      const long double scale = frexpl(2.0L / ((long double)(len + 1) * kappa), &e);   // in [1/2, 1) 2^e
+      const std::vector<uint16_t> plain = sine_matrix(len, kp, 1.0L), scaled = sine_matrix(len, kp, scale);
+      d.mat = reinterpret_cast<const unsigned char*>(p->up(plain.data(), plain.size()));
+      d.e_shift = 0;
+      c.fwd = d;
+      d.mat = reinterpret_cast<const unsigned char*>(p->up(scaled.data(), scaled.size()));
+      d.e_shift = e;
+      c.bwd = d;
+      // the tridiagonal factors, eliminated from either end (the chain is symmetric)
+      SineTri t{};
+      t.n = n;
+      t.lines = len * count;
+      t.modes = fast_div(len);
+      t.top = n / 2;
+      t.s_n = s_n;
+      t.s_c = s_t;
+      t.off = d.off;
+      t.s_strip = d.s_strip;
+      t.strip0 = strip;
+      t.seps = S.seps;
+      t.sep = S.g;
+      const int longest = n - t.top;
+      std::vector<double> cc((size_t)longest * len), g(2 * (size_t)len), edge(len), es(len);
+      for (int k = 0; k < len; ++k) {
+        const long double s = sinl(pi_l * (k + 1) / (2.0L * (len + 1)));
+        const long double diag = 2.0L + 4.0L * s * s;
+        long double r = 0.0L, ctop = 0.0L;
+        for (int i = 0; i < longest; ++i) {
+          r = 1.0L / (diag - r);
+          cc[(size_t)i * len + k] = (double)r;
+          if (i == t.top - 1) ctop = r;
+        }
+        g[k] = (double)(ctop / (1.0L - ctop * r));
+        g[(size_t)len + k] = (double)(r / (1.0L - ctop * r));
+        const long double sk = sinl(pi_l * (k + 1) / (long double)(len + 1));
+        edge[k] = (double)(kappa * sk);
+        es[k] = (double)(2.0L * sk / ((long double)(len + 1) * kappa));
+      }
+      t.segs = chain_segments(n, (int64_t)t.lines * W);
+      if (t.segs) {
+        t.seg_len = (n + t.segs) / t.segs - 1;                       // segs x (seg_len + 1) >= n + 1
+        t.segs = (n + 1 + t.seg_len) / (t.seg_len + 1);
+        const int L = t.seg_len, last = n - (t.segs - 1) * (L + 1);   // points of the last segment
+        std::vector<double> spike((size_t)L * len), spike_last((size_t)std::max(last, 1) * len),
+            piv((size_t)t.segs * len), cpl(len);
+        std::vector<long double> r(L + 1);
+        for (int k = 0; k < len; ++k) {
+          const long double s = sinl(pi_l * (k + 1) / (2.0L * (len + 1)));
+          const long double diag = 2.0L + 4.0L * s * s;
+          long double q = 0.0L;
+          for (int i = 0; i < L; ++i) r[i] = q = 1.0L / (diag - q);   // pivots of a segment
+          // responses to a unit value beyond a segment's end: products of pivots, mirrored
+          auto fill = [&](std::vector<double>& to, int m) {
+            long double v = 1.0L;
+            for (int i = m - 1; i >= 0; --i) {
+              v *= r[i];
+              to[(size_t)(m - 1 - i) * len + k] = (double)v;
+            }
+            return v;   // through the whole segment
+          };
+          const long double c_full = fill(spike, L);
+          fill(spike_last, last);
+          cpl[k] = (double)c_full;
+          long double prev = 0.0L;
+          for (int b = 0; b + 1 < t.segs; ++b) {
+            const int right = b + 2 < t.segs ? L : last;
+            const long double dd = diag - r[L - 1] - (right ? r[right - 1] : 0.0L) - (b ? c_full * c_full * prev : 0.0L);
+            prev = 1.0L / dd;
+            piv[(size_t)b * len + k] = (double)prev;
+          }
+        }
+        t.spike = p->up(spike.data(), spike.size());
+        t.spike_last = p->up(spike_last.data(), spike_last.size());
+        t.seg_piv = p->up(piv.data(), piv.size());
+        t.seg_cpl = p->up(cpl.data(), cpl.size());
+      }
+      t.c = p->up(cc.data(), cc.size());
+      t.g = p->up(g.data(), g.size());
+      t.edge = p->up(edge.data(), edge.size());
+      c.es = p->up(es.data(), es.size());
+      c.tri = t;
+      JJA_CUDA(cudaFuncSetAttribute(sine_kernel(kp), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sine_smem_bytes(kp)));
+      p->sine.push_back(c);
+      strip += count;
+      x0 += count * (len + 1);
+    }
+    if (P > 1) {
+      // per transverse mode: the strips' corner entries and the pivots across the separators
+      std::vector<double> piv((size_t)n * S.seps), cpl((size_t)n * S.seps);
+      std::vector<int32_t> sep_x;
+      for (int s = 0, x = -1; s < S.seps; ++s) {
+        x += (s < n_wide ? narrow + 1 : narrow) + 1;
+        sep_x.push_back(x);
+      }
+      for (int q = 0; q < n; ++q) {
+        const long double sq = sinl(pi_l * (q + 1) / (2.0L * (n + 1)));
+        const long double diag = 2.0L + 4.0L * sq * sq;
+        long double a[2], c[2];   // strips of width narrow, narrow + 1: corner and opposite corner
+        long double r = 0.0L, prod = 1.0L;
+        for (int i = 1; i <= narrow + 1; ++i) {
+          r = 1.0L / (diag - r);
+          prod *= r;
+          if (i >= narrow) {
+            a[i - narrow] = r;
+            c[i - narrow] = prod;
+          }
+        }
+        auto wide = [&](int strip) { return strip < n_wide ? 1 : 0; };
+        long double prev = 0.0L;
+        for (int s = 0; s < S.seps; ++s) {
+          const long double cs = s ? c[wide(s)] : 0.0L;   // strip s lies between separators s - 1 and s
+          const long double d = diag - a[wide(s)] - a[wide(s + 1)] - cs * cs * prev;
+          prev = 1.0L / d;
+          piv[(size_t)q * S.seps + s] = (double)prev;
+          cpl[(size_t)q * S.seps + s] = (double)c[wide(s + 1)];
+        }
+      }
+      S.piv = p->up(piv.data(), piv.size());
+      S.cpl = p->up(cpl.data(), cpl.size());
+      S.sep_x = p->up(sep_x.data(), sep_x.size());
+      // sqrt(2 / (n + 1)) sin(pi (i + 1) (j + 1) / (n + 1)) as digit blocks
+      std::vector<double> mat((size_t)n * n), sine(2 * (size_t)(n + 1));
+      const long double norm = sqrtl(2.0L / (n + 1));
+      for (int i = 0; i <= (n + 1) / 2; ++i) {
+        const double v = (double)(norm * sinl(pi_l * i / (long double)(n + 1)));
+        sine[i] = sine[n + 1 - i] = v;
+        if (i) sine[n + 1 + i] = sine[2 * (n + 1) - i] = -v;
+      }
+      sine[n + 1] = 0.0;
+      for (int64_t i = 0; i < n; ++i)
+        for (int64_t j = 0; j < n; ++j) mat[i * n + j] = sine[(size_t)(((i + 1) * (j + 1)) % (2 * ((int64_t)n + 1)))];
+      std::vector<BlockUnit> units;
+      std::vector<BlockSource> src;
+      std::vector<int32_t> rows(n);
+      for (int i = 0; i < n; ++i) rows[i] = i;
+      for (int c = 0; c < n; c += kBlockCols)
+        for (int r = 0; r < n; r += kBlockRows) {
+          const int nr = std::min(kBlockRows, n - r), nc = std::min(kBlockCols, n - c);
+          units.push_back({c, nc, r, nr, (int)units.size(), 0});
+          src.push_back({(int64_t)r * n + c, n, 1, nr, nc});
+        }
+      BlockList L{};
+      L.n = (int)units.size();
+      L.units = p->up(units.data(), units.size());
+      L.in_rows = L.out_rows = p->up(rows.data(), rows.size());
+      unsigned char* mats = p->up<unsigned char>(nullptr, (size_t)L.n * kBlockMatBytes);
+      int* e_mat = p->up<int>(nullptr, (size_t)L.n);
+      int64_t ignored = 0;
+      double* store = upload(mat.data(), mat.size(), ignored);
+      BlockSource* d_src = nullptr;
+      try {
+        d_src = upload(src.data(), src.size(), ignored);
+        k_block_digits<<<L.n, 256>>>(store, d_src, mats, e_mat);
+        g_launches++;
+        JJA_CUDA(cudaDeviceSynchronize());
+      } catch (...) {
+        cudaFree(store);
+        cudaFree(d_src);
+        throw;
+      }
+      cudaFree(store);
+      cudaFree(d_src);
+      L.mats = mats;
+      L.e_mat = e_mat;
+      for (int wp : {16, 32, 48, 64})
+        JJA_CUDA(cudaFuncSetAttribute(block_kernel(wp), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem_bytes(wp)));
+      p->sep_dst = L;
+    }
+    p->strips = S;
     one_chain(p);
     p->dst = 2;
   });

@@ -23,7 +23,9 @@
 //
 // Measured (GB300, per step, graph-replayed; the sweeps they replace -> these kernels): 128x128 x
 // 512 problems 1.157 -> 0.669 ms, 101x60 x 24 0.138 -> 0.058 ms; an adjoint run on 64x64 x 64
-// 121 -> 53 ms. A tile (128 columns of 127 faces) takes about 30k cycles: reading and splitting
+// 121 -> 53 ms; 1024x1024 x 8 (8 strips) 2.30 -> 0.92 ms: 84 us per transform, 108 and 158 us for the
+// two passes over the chains (72 and 100 us of FP64 work), 45 us for the edges, 50 us for the
+// separators. A tile (128 columns of 127 faces) takes about 30k cycles: reading and splitting
 // 6k, twice the products 3.8k (3.5k of MMA issue at the multipliers' rate) and the joining 7k.
 // What bounds it: the shifts and logic of splitting and joining (the ALU pipe runs half a warp
 // instruction per clock and scheduler), serialised with the products because one tile's digits and
@@ -34,6 +36,7 @@ namespace {
 constexpr int kMatDigits = 6;                  // 9-bit digits of a matrix entry
 constexpr int kDatDigits = 7;                  // ... of a data value; also the number of accumulators
 constexpr int kSineMaxPoints = 128;            // longest transform (folded length 64)
+constexpr int kSineMaxSide = 4096;             // of the grid (the separators' dense sine matrix: 200 MB of digits)
 constexpr int kSineColumns = 128;              // (line, problem) columns per tile: the MMA's M
 constexpr int kSineThreads = 512;
 // TMEM columns of the 7 accumulators of kp columns each (a power of two is allocated)
@@ -45,16 +48,33 @@ constexpr int64_t kMmaSpinLimit = 1LL << 24;   // try_wait polls; far beyond any
 struct SineArgs {
   int m, kp, lines;
   int64_t s_t, s_c;
+  int64_t off, s_strip;   // first line, and between strips of the grid (see SineStrips)
+  FastDiv per_strip;      // lines of one strip
   int parts;            // blocks a tile of columns is shared by: 1, 2 (odd, even modes) or 2 x mode chunks
   const unsigned char* mat;   // digits of the odd and even half matrices in the MMA operand layout
   int e_shift;          // result exponent offset (the power-of-two part of the scale)
 };
 
 struct SineTri {
-  int n, lines, top;    // points a chain, chains (modes), points of the upper half
-  int64_t s_n, s_c;     // strides along a chain and between chains
-  const double* c;      // c[i * lines + mode]: reciprocal pivots, from either end
-  const double* g;      // per mode: the join at the middle
+  int n, top;           // points a chain, points of the upper half
+  int lines;            // chains: strips x modes
+  FastDiv modes;        // modes per strip
+  int64_t s_n, s_c;     // strides along a chain and between modes
+  int64_t off, s_strip;
+  const double* c;      // c[i * modes + mode]: reciprocal pivots, from either end
+  const double* g;      // per mode: the join at the middle (top, then bottom)
+  // values on the separators beside the strips (null: none): sep[(i * seps + s) * W + w], added to the
+  // right-hand side as edge[mode] times the sum (modes 1, 3, ...) or difference of both sides'
+  const double* sep;
+  const double* edge;
+  int seps, strip0;     // separators of the grid, first strip of this launch
+  // chains in segments (k_sine_chain): `segs` warps of `seg_len` points each (the last one shorter), one
+  // point between neighbours; segs = 0: two halves (k_sine_tri)
+  int segs, seg_len;
+  const double* spike;  // spike[i * modes + mode]: response at point i to the point before the segment
+  const double* spike_last;
+  const double* seg_piv;   // reciprocal pivots across the points between segments
+  const double* seg_cpl;   // per mode: coupling through a whole segment
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -224,8 +244,8 @@ __global__ void __launch_bounds__(kSineThreads, 1) k_sine_lines(SineArgs d, cons
   auto load = [&](int tl) {
     const int64_t c = (int64_t)tl * kSineColumns + col;
     const bool live = c < ncols;
-    const int64_t line = live ? by_wn(c) : 0;
-    const double* src = in + line * d.s_c + (live ? w0 + (c - line * wn) : 0);
+    const int64_t line = live ? by_wn(c) : 0, strip = d.per_strip(line);
+    const double* src = in + d.off + strip * d.s_strip + (line - strip * d.per_strip.d) * d.s_c + (live ? w0 + (c - line * wn) : 0);
 #pragma unroll
     for (int r = 0; r < 2; ++r)
 #pragma unroll
@@ -269,8 +289,8 @@ __global__ void __launch_bounds__(kSineThreads, 1) k_sine_lines(SineArgs d, cons
   for (; tile < tiles; tile += tile_step) {
     const int64_t c = (int64_t)tile * kSineColumns + col;
     const bool live = c < ncols;
-    const int64_t line = live ? by_wn(c) : 0;
-    double* dst = out + line * d.s_c + (live ? w0 + (c - line * wn) : 0);
+    const int64_t line = live ? by_wn(c) : 0, strip = d.per_strip(line);
+    double* dst = out + d.off + strip * d.s_strip + (line - strip * d.per_strip.d) * d.s_c + (live ? w0 + (c - line * wn) : 0);
     uint32_t top = 0;   // the line's largest magnitude (high words without the sign)
 #pragma unroll
     for (int r = 0; r < 2; ++r)
@@ -396,21 +416,41 @@ size_t sine_smem_bytes(int kp) {
   return (size_t)kp * 2 * (2 * kMatDigits * kp + kDatDigits * kSineColumns) + 4 * kSineColumns * sizeof(int) + 64;
 }
 
-// Tridiagonal solve per (mode, problem) in place: (lambda_mode + 2) x_i - x_{i-1} - x_{i+1} = v_i,
-// eliminated from both ends towards the middle by two threads (half the chain each), joined
-// there, and substituted back outwards. 3 FP64 operations per element.
+// Tridiagonal solve per (mode, problem), in -> out (which may be the same array):
+// (lambda_mode + 2) x_i - x_{i-1} - x_{i+1} = v_i, eliminated from both ends towards the middle by two
+// threads (half the chain each), joined there, and substituted back outwards. 3 FP64 operations per
+// element, 5 with values on the separators.
 constexpr int kTriColumns = 64;
-__global__ void __launch_bounds__(2 * kTriColumns) k_sine_tri(SineTri t, double* v, int w0, int wn, FastDiv by_wn) {
+template <bool kSep>
+__global__ void __launch_bounds__(2 * kTriColumns) k_sine_tri(SineTri t, const double* in, double* out, int W, int w0,
+                                                             int wn, FastDiv by_wn) {
   pdl_begin();
   __shared__ double join_z[2][kTriColumns];
   const int side = threadIdx.x / kTriColumns, lc = threadIdx.x - side * kTriColumns;   // 0: from the first point
   const int64_t c = (int64_t)blockIdx.x * kTriColumns + lc, ncols = (int64_t)t.lines * wn;
   const bool live = c < ncols;
-  const int mode = live ? (int)by_wn(c) : 0;
+  const int64_t line = live ? by_wn(c) : 0;
+  const int strip = (int)t.modes(line), modes = (int)t.modes.d, mode = (int)line - strip * modes;
+  const int w = w0 + (live ? (int)(c - line * wn) : 0);
   const int cnt = side ? t.n - t.top : t.top;
   const int64_t step = side ? -t.s_n : t.s_n;
-  double* p0 = v + (int64_t)mode * t.s_c + (live ? w0 + (c - (int64_t)mode * wn) : 0) + (side ? (int64_t)(t.n - 1) * t.s_n : 0);
+  const int64_t base = t.off + strip * t.s_strip + (int64_t)mode * t.s_c + w + (side ? (int64_t)(t.n - 1) * t.s_n : 0);
+  const double* src = in + base;
+  double* dst = out + base;
   const double* ct = t.c + mode;
+  // the separators before and after the strip
+  const int s1 = t.strip0 + strip;
+  const double* sep_l = kSep && s1 > 0 ? t.sep + ((int64_t)(side ? t.n - 1 : 0) * t.seps + s1 - 1) * W + w : nullptr;
+  const double* sep_r = kSep && s1 < t.seps ? t.sep + ((int64_t)(side ? t.n - 1 : 0) * t.seps + s1) * W + w : nullptr;
+  const int64_t sep_step = (side ? -1 : 1) * (int64_t)t.seps * W;
+  const double edge = kSep ? __ldg(t.edge + mode) : 0.0;
+  auto rhs = [&](int i) -> double {
+    const double v = src[(int64_t)i * step];
+    if (!kSep) return v;
+    double s = sep_l ? __ldg(sep_l + i * sep_step) : 0.0;
+    if (sep_r) s += signed_by(__ldg(sep_r + i * sep_step), mode & 1);
+    return fma(edge, s, v);
+  };
   double z = 0.0, cp = 0.0;
   if (live) {
     // z_i = v_i + c_{i-1} z_{i-1}; c_i z_i is kept for the way back
@@ -419,20 +459,20 @@ __global__ void __launch_bounds__(2 * kTriColumns) k_sine_tri(SineTri t, double*
       double x[8], cc[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        x[u] = p0[(int64_t)(i + u) * step];
-        cc[u] = __ldg(ct + (int64_t)(i + u) * t.lines);
+        x[u] = rhs(i + u);
+        cc[u] = __ldg(ct + (int64_t)(i + u) * modes);
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         z = fma(cp, z, x[u]);
         cp = cc[u];
-        p0[(int64_t)(i + u) * step] = cp * z;
+        dst[(int64_t)(i + u) * step] = cp * z;
       }
     }
     for (; i < cnt; ++i) {
-      z = fma(cp, z, p0[(int64_t)i * step]);
-      cp = __ldg(ct + (int64_t)i * t.lines);
-      p0[(int64_t)i * step] = cp * z;
+      z = fma(cp, z, rhs(i));
+      cp = __ldg(ct + (int64_t)i * modes);
+      dst[(int64_t)i * step] = cp * z;
     }
   }
   join_z[side][lc] = cp * z;    // z / pivot of the half's last point
@@ -440,25 +480,283 @@ __global__ void __launch_bounds__(2 * kTriColumns) k_sine_tri(SineTri t, double*
   if (!live || cnt == 0) return;
   // x at the two middle points: x_b = (z_b + c_t z_t) c_b / (1 - c_t c_b), and the same mirrored
   const double other = join_z[side ^ 1][lc];
-  double x = (z + other) * __ldg(t.g + (int64_t)side * t.lines + mode);
-  p0[(int64_t)(cnt - 1) * step] = x;
+  double x = (z + other) * __ldg(t.g + (int64_t)side * modes + mode);
+  dst[(int64_t)(cnt - 1) * step] = x;
   int i = cnt - 2;
   for (; i >= 7; i -= 8) {
     double y[8], cc[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      y[u] = p0[(int64_t)(i - u) * step];
-      cc[u] = __ldg(ct + (int64_t)(i - u) * t.lines);
+      y[u] = dst[(int64_t)(i - u) * step];
+      cc[u] = __ldg(ct + (int64_t)(i - u) * modes);
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       x = fma(cc[u], x, y[u]);
-      p0[(int64_t)(i - u) * step] = x;
+      dst[(int64_t)(i - u) * step] = x;
     }
   }
   for (; i >= 0; --i) {
-    x = fma(__ldg(ct + (int64_t)i * t.lines), x, p0[(int64_t)i * step]);
-    p0[(int64_t)i * step] = x;
+    x = fma(__ldg(ct + (int64_t)i * modes), x, dst[(int64_t)i * step]);
+    dst[(int64_t)i * step] = x;
+  }
+}
+
+// The same with a chain's points split over `segs` warps (lane = column): each eliminates its segment
+// with zero outside values and forms the solution at its ends (one elimination and one dot product),
+// one warp solves for the points between the segments, and each substitutes back with them:
+// 5 FP64 operations per element instead of 3, chains of n / segs instead of n / 2 dependent ones.
+constexpr int kMaxSegs = 16;
+template <bool kSep>
+__global__ void __launch_bounds__(32 * kMaxSegs) k_sine_chain(SineTri t, const double* in, double* out, int W, int w0,
+                                                             int wn, FastDiv by_wn) {
+  pdl_begin();
+  __shared__ double u1[kMaxSegs][32], uL[kMaxSegs][32], mid[kMaxSegs][32];
+  const int seg = threadIdx.x >> 5, lane = threadIdx.x & 31, segs = t.segs, len_full = t.seg_len;
+  const int64_t c = (int64_t)blockIdx.x * 32 + lane, ncols = (int64_t)t.lines * wn;
+  const bool live = c < ncols;
+  const int64_t line = live ? by_wn(c) : 0;
+  const int strip = (int)t.modes(line), modes = (int)t.modes.d, mode = (int)line - strip * modes;
+  const int w = w0 + (live ? (int)(c - line * wn) : 0);
+  const int pos0 = seg * (len_full + 1), len = min(len_full, t.n - pos0);
+  const bool last = seg == segs - 1;
+  const int64_t base = t.off + strip * t.s_strip + (int64_t)mode * t.s_c + w + (int64_t)pos0 * t.s_n;
+  const double* src = in + base;
+  double* dst = out + base;
+  const double* ct = t.c + mode;
+  const double* sp = (last ? t.spike_last : t.spike) + mode;
+  const int s1 = t.strip0 + strip;
+  const double* sep_l = kSep && s1 > 0 ? t.sep + ((int64_t)pos0 * t.seps + s1 - 1) * W + w : nullptr;
+  const double* sep_r = kSep && s1 < t.seps ? t.sep + ((int64_t)pos0 * t.seps + s1) * W + w : nullptr;
+  const int64_t sep_step = (int64_t)t.seps * W;
+  const double edge = kSep ? __ldg(t.edge + mode) : 0.0;
+  auto rhs = [&](int i) -> double {
+    const double v = src[(int64_t)i * t.s_n];
+    if (!kSep) return v;
+    double s = sep_l ? __ldg(sep_l + i * sep_step) : 0.0;
+    if (sep_r) s += signed_by(__ldg(sep_r + i * sep_step), mode & 1);
+    return fma(edge, s, v);
+  };
+  double z = 0.0, first = 0.0, cp = 0.0;
+  if (live) {
+    const double between = last ? 0.0 : rhs(len_full);
+    int i = 0;
+    for (; i + 8 <= len; i += 8) {
+      double x[8], cc[8], ll[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = rhs(i + u);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        cc[u] = __ldg(ct + (int64_t)(i + u) * modes);
+        ll[u] = __ldg(sp + (int64_t)(i + u) * modes);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        z = fma(cp, z, x[u]);
+        cp = cc[u];
+        first = fma(ll[u], x[u], first);
+        dst[(int64_t)(i + u) * t.s_n] = z;
+      }
+    }
+    for (; i < len; ++i) {
+      const double x = rhs(i);
+      z = fma(cp, z, x);
+      cp = __ldg(ct + (int64_t)i * modes);
+      first = fma(__ldg(sp + (int64_t)i * modes), x, first);
+      dst[(int64_t)i * t.s_n] = z;
+    }
+    mid[seg][lane] = between;
+  }
+  u1[seg][lane] = first;
+  uL[seg][lane] = cp * z;
+  __syncthreads();
+  if (seg == 0 && live) {
+    const double cpl = __ldg(t.seg_cpl + mode);
+    double y = 0.0;
+    for (int s = 0; s + 1 < segs; ++s) {
+      y = fma(cpl, y, mid[s][lane] + uL[s][lane] + u1[s + 1][lane]) * __ldg(t.seg_piv + (int64_t)s * modes + mode);
+      mid[s][lane] = y;
+    }
+    for (int s = segs - 3; s >= 0; --s) {
+      y = fma(cpl * __ldg(t.seg_piv + (int64_t)s * modes + mode), y, mid[s][lane]);
+      mid[s][lane] = y;
+    }
+  }
+  __syncthreads();
+  if (!live) return;
+  const double gl = seg ? mid[seg - 1][lane] : 0.0, gr = last ? 0.0 : mid[seg][lane];
+  if (!last) dst[(int64_t)len_full * t.s_n] = gr;
+  double x = gr;
+  int i = len - 1;
+  for (; i >= 7; i -= 8) {
+    double y[8], cc[8], ll[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) y[u] = dst[(int64_t)(i - u) * t.s_n];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      cc[u] = __ldg(ct + (int64_t)(i - u) * modes);
+      ll[u] = __ldg(sp + (int64_t)(i - u) * modes);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      x = (y[u] + x) * cc[u];
+      dst[(int64_t)(i - u) * t.s_n] = fma(ll[u], gl, x);
+    }
+  }
+  for (; i >= 0; --i) {
+    x = (dst[(int64_t)i * t.s_n] + x) * __ldg(ct + (int64_t)i * modes);
+    dst[(int64_t)i * t.s_n] = fma(__ldg(sp + (int64_t)i * modes), gl, x);
+  }
+}
+
+// segments per chain: about 24 warps per SM, at least 8 points each; none for many columns, where the
+// two-sided elimination's fewer operations count
+int chain_segments(int n, int64_t columns) {
+  const int64_t want = 24LL * kNumSMs * 32 / std::max<int64_t>(1, columns);
+  const int segs = (int)std::min<int64_t>(std::min(kMaxSegs, (n + 1) / 9), want);
+  return segs >= 3 ? segs : 0;
+}
+
+// ------------------------------------------------------------------------------------------
+// Arrays whose sides both exceed 128 faces: the longer side is cut into strips of up to 128 grid lines
+// with one grid line (a separator) between neighbours. Per strip the solver above; the separators'
+// values g follow from their own equations, which the sine transform along the chains diagonalises:
+// for every transverse mode q a tridiagonal system over the separators,
+//   (2 + l_q - a_i - a_{i+1}) g_i - c_i g_{i-1} - c_{i+1} g_{i+1} = b_i / kappa + u0_i(last) + u0_{i+1}(first)
+// with a_i, c_i the corner entries of the inverse of strip i's tridiag(-1, 2 + l_q, -1) and u0 the
+// strips' solutions for zero separators. So: transform the strips, solve the chains, form u0 at the
+// strips' edges, transform the separators (a product with the dense sine matrix, jja_block.cuh), solve
+// across them, transform back, solve the chains again with the separators' values, transform back.
+// ------------------------------------------------------------------------------------------
+struct SineStrips {
+  int n = 0, seps = 0;                // points a chain, separators
+  int64_t s_n = 0, s_x = 0;           // strides along a chain and between grid lines
+  const int32_t* sep_x = nullptr;     // grid line of every separator
+  double inv_kappa = 0.0;
+  const double* piv = nullptr;        // (n x seps): reciprocal pivots per transverse mode
+  const double* cpl = nullptr;        // (n x seps): coupling c of strip s + 1 (between separators s and s + 1)
+  double* edge = nullptr;             // n x strips x 2 x W: u0 at the first and last line of every strip
+  double* rhs = nullptr;              // n x seps x W
+  double* hat = nullptr;
+  double* g = nullptr;
+};
+
+// u0 at the edges of the strips of one width: sums of es[mode] z over odd and even modes. A warp sums a
+// (point, strip) over the contiguous modes x problems when the problems divide its lanes or the
+// lanes divide the problems; else a block does, problems x slices of the modes. Grid: (points,
+// strips, tiles of the problems).
+__global__ void __launch_bounds__(256) k_sine_edges(const double* __restrict__ z, const double* __restrict__ es, int modes,
+                                                    int64_t off, int64_t s_strip, int64_t s_n, int64_t s_c, int strip0,
+                                                    int strips, int n, int W, double* __restrict__ edge) {
+  pdl_begin();
+  const int strip = blockIdx.y;
+  const bool lanes = 32 % W == 0 || W % 32 == 0;
+  if (lanes) {
+    const int per = W < 32 ? 32 / W : 1, lane = threadIdx.x & 31;   // modes side by side in a warp
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (i >= n) return;
+    const int k0 = lane / min(W, 32), w = blockIdx.z * 32 + lane % min(W, 32);
+    const double* p = z + off + strip * s_strip + (int64_t)i * s_n + w;
+    double odd = 0.0, even = 0.0;
+    int k = k0;
+    for (; k + 7 * per < modes; k += 8 * per) {
+      double v[8], e[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        v[u] = p[(int64_t)(k + u * per) * s_c];
+        e[u] = __ldg(es + k + u * per);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if ((k + u * per) & 1) even = fma(e[u], v[u], even);
+        else odd = fma(e[u], v[u], odd);
+      }
+    }
+    for (; k < modes; k += per) {
+      const double v = p[(int64_t)k * s_c], e = __ldg(es + k);
+      if (k & 1) even = fma(e, v, even);
+      else odd = fma(e, v, odd);
+    }
+    for (int o = W; o < 32; o <<= 1) {
+      odd += __shfl_xor_sync(0xffffffffu, odd, o);
+      even += __shfl_xor_sync(0xffffffffu, even, o);
+    }
+    if (k0 == 0) {
+      double* e = edge + (((int64_t)i * strips + strip0 + strip) * 2) * W + w;
+      e[0] = odd + even;   // first line
+      e[W] = odd - even;   // last line
+    }
+    return;
+  }
+  __shared__ double part[2][256];
+  const int tw = min(W, 256), slices = 256 / tw, slice = threadIdx.x / tw, w = blockIdx.z * tw + threadIdx.x % tw;
+  const int i = blockIdx.x;
+  double odd = 0.0, even = 0.0;   // modes 1, 3, ... and 2, 4, ...
+  if (slice < slices && w < W) {
+    const double* p = z + off + strip * s_strip + (int64_t)i * s_n + w;
+#pragma unroll 4
+    for (int k = slice; k < modes; k += slices) {
+      const double v = p[(int64_t)k * s_c], e = __ldg(es + k);
+      if (k & 1) even = fma(e, v, even);
+      else odd = fma(e, v, odd);
+    }
+  }
+  part[0][threadIdx.x] = odd;
+  part[1][threadIdx.x] = even;
+  __syncthreads();
+  if (slice == 0 && w < W) {
+    for (int k = 1; k < slices; ++k) {
+      odd += part[0][k * tw + threadIdx.x];
+      even += part[1][k * tw + threadIdx.x];
+    }
+    double* e = edge + (((int64_t)i * strips + strip0 + strip) * 2) * W + w;
+    e[0] = odd + even;
+    e[W] = odd - even;
+  }
+}
+
+// the separators' right-hand sides; the transformed vector is zeroed for the product that follows
+__global__ void __launch_bounds__(256) k_sep_rhs(SineStrips S, const double* __restrict__ b, int W, FastDiv by_W) {
+  pdl_begin();
+  const int64_t n = (int64_t)S.n * S.seps * W;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = by_W(e), w = e - r * W, i = r / S.seps;
+    const int s = (int)(r - i * S.seps);
+    const double* ed = S.edge + ((i * (S.seps + 1) + s) * 2) * W + w;   // strip s, then strip s + 1
+    S.rhs[e] = fma(b[i * S.s_n + (int64_t)__ldg(S.sep_x + s) * S.s_x + w], S.inv_kappa, ed[W] + ed[2 * W]);
+    S.hat[e] = 0.0;
+  }
+}
+
+// across the separators, per transverse mode and problem; zeroes g for the product that follows
+__global__ void __launch_bounds__(256) k_sep_solve(SineStrips S, int W, FastDiv by_W) {
+  pdl_begin();
+  const int64_t n = (int64_t)S.n * W;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t q = by_W(e), w = e - q * W;
+    double* h = S.hat + q * S.seps * W + w;
+    double* g = S.g + q * S.seps * W + w;
+    const double *piv = S.piv + q * S.seps, *cpl = S.cpl + q * S.seps;
+    double y = 0.0;
+    for (int s = 0; s < S.seps; ++s) {   // y_s = (r_s + c_s y_{s-1}) / pivot
+      y = (s ? fma(__ldg(cpl + s - 1), y, h[(int64_t)s * W]) : h[0]) * __ldg(piv + s);
+      h[(int64_t)s * W] = y;
+      g[(int64_t)s * W] = 0.0;
+    }
+    for (int s = S.seps - 2; s >= 0; --s) {
+      y = fma(__ldg(cpl + s) * __ldg(piv + s), y, h[(int64_t)s * W]);
+      h[(int64_t)s * W] = y;
+    }
+  }
+}
+
+// the separators' values into the solution
+__global__ void __launch_bounds__(256) k_sep_store(SineStrips S, double* __restrict__ x, int W, FastDiv by_W) {
+  pdl_begin();
+  const int64_t n = (int64_t)S.n * S.seps * W;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = by_W(e), w = e - r * W, i = r / S.seps;
+    x[i * S.s_n + (int64_t)__ldg(S.sep_x + (int)(r - i * S.seps)) * S.s_x + w] = S.g[e];
   }
 }
 

@@ -183,24 +183,40 @@ def fast_poisson_grid(circuit, K):
     return None if g is None or any(m + 1 > 1024 or (m + 1) & m for m in g[:2]) else g
 
 
-# "auto" uses the sine transforms for at most this many problems and face-problems (W x Nf). Measured
-# on GB300 (device ms per step, transforms / sweeps): 256x256 W = 1 0.066 / 0.158, 128x128 W = 1
-# 0.031 / 0.082, W = 8 0.092 / 0.142, W = 16 0.168 / 0.163, W = 64 0.60 / 0.30; 512x512 W = 1
-# 0.23 / 0.36; 1024x1024 W = 1 0.85 / 0.79, W = 8 6.3 / 2.9; 64x64 W = 64 0.150 / 0.129
+# "auto" uses the radix-2 sine transforms for at most this many problems and face-problems (W x Nf) when
+# the caller tunes the sweeps. Measured on GB300 (device ms per step, transforms / sweeps): 256x256 W = 1
+# 0.066 / 0.158, 128x128 W = 1 0.031 / 0.082, W = 8 0.092 / 0.142, W = 16 0.168 / 0.163, W = 64
+# 0.60 / 0.30; 512x512 W = 1 0.23 / 0.36; 1024x1024 W = 1 0.85 / 0.79, W = 8 6.3 / 2.9; 64x64 W = 64
+# 0.150 / 0.129
 FAST_POISSON_MAX_W = 8
 FAST_POISSON_MAX_WORK = 1 << 18
 
+# Uniform square arrays otherwise (us per step: radix-2 transforms / tensor-core transforms (cut into
+# strips above 128 faces a side) / dense blocks):
+#   33x33    W = 16   - / 28 / 14      W = 64   - / 29 / 20       W = 256  - / 37 / 42
+#   64x64    W = 1   24 / 30 / 22      W = 16  37 / 32 / 28       W = 64  92 / 39 / 43
+#   101x60   W = 1    - / 40 / 22      W = 16   - / 38 / 30       W = 64   - / 51 / 54
+#   110x110  W = 4    - / 43 / 38      W = 16   - / 44 / 54       W = 64   - / 72 / 116
+#   128x128  W = 1   27 / 66 / 49      W = 4   39 / 46 / 53       W = 16 102 / 48 / 65
+#   150x150  W = 1    - / 76 / 76      W = 8    - / 82 / 90       W = 64   - / 167 / 238
+#   256x256  W = 1   44 / 115 / -      W = 4  124 / 103 / -
+# so: dense blocks up to SINE_FROM_WORK face-problems on up to SINE_FROM_FACES faces, tensor-core
+# transforms above, radix-2 transforms for a few problems on power-of-two grids.
+SINE_FROM_WORK = 150000
+SINE_FROM_FACES = 1 << 14
+SINE_MIN_SIDE = 8
+SINE_MAX_SIDE = 4096
 
-# The tensor-core transforms work on tiles of 128 (grid line, problem) columns, one tile per SM at
-# a time, on grids whose shorter side has at most 128 faces (SINE_MAX_SIDE).
-SINE_MAX_SIDE = 128
-SINE_MIN_COLUMNS = 512
+
+def radix2_fits(n_faces, W):
+    """Whether "auto" tries the radix-2 transforms for W problems (the grid permitting)."""
+    return 2048 <= n_faces <= 1 << 17 and W <= (1 if n_faces < 8192 else 4 if n_faces < 1 << 15 else 3)
 
 
 def sine_solver_fits(grid, W):
     """Whether "auto" takes the tensor-core sine transforms for W problems on this poisson_grid."""
     mx, my = grid[:2]
-    return min(mx, my) <= SINE_MAX_SIDE and min(mx, my) >= 8 and max(mx, my) * W >= SINE_MIN_COLUMNS
+    return SINE_MIN_SIDE <= min(mx, my) and max(mx, my) <= SINE_MAX_SIDE
 
 
 # Circuits whose state and inverse fit one SM run whole calls in one launch, a block per problem, while
@@ -409,22 +425,24 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
     ``ordering`` "nd", "mmd" or "auto" (see resolve_ordering); ``nd_leaf`` None: by the step's
     size (see resolve_factor_shape); ``tuning`` the launch shape of the triangular solves (see
     DevicePlan); ``fast_poisson``: solve with sine transforms when the face-space matrix allows it
-    (fast_poisson_grid): True, False, or "auto" (W <= 8 and W x Nf <= 2^18 face-problems; the
-    tensor-core transforms by sine_solver_fits)."""
-    fp = None
+    (fast_poisson_grid): True (radix-2 grids), False (the sweeps), or "auto": unless ``tuning`` asks for
+    sweeps of some shape, whichever of the resident steps (resident_fits), the radix-2 or tensor-core
+    transforms, and the dense blocks (block_leaf) is fastest for the circuit and W."""
+    fp = sine = blocks = None
     matrices = face_matrix(circuit, dt)
-    resident = fast_poisson == "auto" and untuned(tuning) and resident_fits(circuit, W)
-    if fast_poisson is True or (fast_poisson == "auto" and not resident and W <= FAST_POISSON_MAX_W
-                                and W * circuit._Nf() <= FAST_POISSON_MAX_WORK):
+    n_faces = circuit._Nf()
+    auto = fast_poisson == "auto" and untuned(tuning)
+    resident = auto and resident_fits(circuit, W)
+    if fast_poisson is True or (auto and not resident and radix2_fits(n_faces, W)) or \
+            (fast_poisson == "auto" and not auto and W <= FAST_POISSON_MAX_W and W * n_faces <= FAST_POISSON_MAX_WORK):
         fp = fast_poisson_grid(circuit, matrices[1])
-    sine = None
-    if fp is None and not resident and fast_poisson == "auto" and W * circuit._Nf() >= SINE_MIN_COLUMNS and untuned(tuning):
-        sine = poisson_grid(circuit, matrices[1])
-        if sine is not None and not sine_solver_fits(sine, W):
-            sine = None
-    blocks = None
-    if fp is None and sine is None and not resident and fast_poisson == "auto" and untuned(tuning):
-        blocks = block_leaf(circuit, W)
+    if auto and not resident and fp is None:
+        if W * n_faces > SINE_FROM_WORK or n_faces > SINE_FROM_FACES:
+            sine = poisson_grid(circuit, matrices[1])
+            if sine is not None and not sine_solver_fits(sine, W):
+                sine = None
+        if sine is None:
+            blocks = block_leaf(circuit, W)
     if blocks is not None:     # the block solver cuts the tree itself: nested dissection with small leaves
         nd_leaf = 8 if nd_leaf is None else nd_leaf
         ordering = "nd" if ordering == "auto" else ordering

@@ -44,7 +44,9 @@ def _solve(c, b, sine):
 
 
 SIZES = [(2, 2, 1), (2, 9, 3), (3, 4, 2), (18, 33, 7), (33, 34, 128), (34, 17, 129), (64, 64, 5), (66, 65, 33),
-         (96, 97, 40), (98, 99, 2), (128, 128, 3), (129, 128, 65), (129, 300, 2), (300, 129, 2), (101, 60, 24)]
+         (96, 97, 40), (98, 99, 2), (128, 128, 3), (129, 128, 65), (129, 300, 2), (300, 129, 2), (101, 60, 24),
+         # both sides longer than 128 faces: strips of one and two widths, one and several separators
+         (131, 130, 2), (130, 131, 17), (257, 257, 1), (140, 400, 3), (390, 135, 2), (300, 300, 5), (131, 131, 260)]
 
 
 @pytest.mark.gpu
@@ -82,7 +84,7 @@ def test_non_finite_values_stay_in_their_problem():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("nx,ny,W,width", [(33, 25, 24, 3), (40, 130, 9, 4), (25, 30, 300, 3)])
+@pytest.mark.parametrize("nx,ny,W,width", [(60, 70, 64, 3), (40, 130, 40, 4), (25, 30, 300, 3), (150, 140, 3, 3)])
 def test_trajectory_matches_sweeps_and_oracle(nx, ny, W, width):
     c = SquareArray(nx, ny)
     c.set_capacitance(0.4)
