@@ -142,7 +142,9 @@ def poisson_grid(circuit, K):
     mx x my grid of faces: a square array with equal R and C and a uniform self-inductance, whose K
     is kappa times the 5-point Laplacian with Dirichlet boundaries. Checked entry by entry (relative
     1e-12); None otherwise."""
-    # the diagonal and the entries first: most circuits fail there, without their geometry
+    # the entries first: most circuits fail there, without their geometry
+    K = scipy.sparse.csc_matrix(K)
+    Nf = K.shape[0]
     diag = K.diagonal()
     kappa = float(diag[0]) / 4.0
     if not kappa > 0.0:
@@ -150,31 +152,59 @@ def poisson_grid(circuit, K):
     tol = 1e-12 * kappa
     if np.abs(diag - 4.0 * kappa).max() > tol:
         return None
-    Kc = scipy.sparse.coo_matrix(K)
-    off = Kc.row != Kc.col
-    r, c, v = Kc.row[off], Kc.col[off], Kc.data[off]
-    if np.abs(v + kappa).max(initial=0.0) > tol:
+    if np.count_nonzero(np.abs(K.data + kappa) <= tol) != K.nnz - Nf:
         return None
     try:
-        cx, cy = circuit.get_face_centroids()
+        cx, cy = _face_midpoints(circuit)
     except Exception:
         return None
-    Nf = K.shape[0]
-    ux, ix = np.unique(np.round(np.asarray(cx, np.float64), 9), return_inverse=True)
-    uy, iy = np.unique(np.round(np.asarray(cy, np.float64), 9), return_inverse=True)
-    mx, my = len(ux), len(uy)
-    if mx * my != Nf:
+    ix, iy = _grid_index(K, cx), _grid_index(K, cy)
+    if ix is None or iy is None:
         return None
-    grid = np.full(mx * my, -1, np.int64)
-    grid[iy * mx + ix] = np.arange(Nf)
+    mx, my = int(ix.max()) + 1, int(iy.max()) + 1
+    if mx * my != Nf or K.nnz - Nf != 2 * (mx * (my - 1) + my * (mx - 1)):
+        return None
+    cell = iy * mx + ix
+    grid = np.full(Nf, -1, np.int32)
+    grid[cell] = np.arange(Nf, dtype=np.int32)
     if np.any(grid < 0):
         return None
-    neighbour = (np.abs(ix[r] - ix[c]) + np.abs(iy[r] - iy[c])) == 1
-    if not np.all(neighbour):
+    # every off-diagonal entry couples neighbours: the same row one cell on, or one row on
+    r, c = cell[K.indices], np.repeat(cell, np.diff(K.indptr))
+    step = np.abs(r - c)
+    along = (step == 1) & (np.minimum(r, c) % mx != mx - 1)
+    if np.count_nonzero(along | (step == mx) | (step == 0)) != K.nnz:
         return None
-    if np.count_nonzero(np.abs(v) > tol) != 2 * (mx * (my - 1) + my * (mx - 1)):
-        return None
-    return mx, my, np.ascontiguousarray(grid, np.int32), kappa
+    return mx, my, grid, kappa
+
+
+def _grid_index(K, v):
+    """Index of every face along one axis of an equally spaced grid (int32), or None; the spacing is the
+    smallest difference between coupled faces (all faces of a column: 0)."""
+    some = K.indptr[min(K.shape[0], 4096)]
+    d = np.abs(v[K.indices[:some]] - v[np.repeat(np.arange(min(K.shape[0], 4096)), np.diff(K.indptr[:4097]))])
+    d = d[d > 1e-9]
+    lo, h = v.min(), d.min(initial=np.inf)
+    if not np.isfinite(h):
+        return np.zeros(len(v), np.int32) if v.max() - lo <= 1e-9 else None
+    i = np.rint((v - lo) / h)
+    return i.astype(np.int32) if np.abs(v - (lo + i * h)).max() <= 1e-6 * h else None
+
+
+def _face_midpoints(circuit):
+    """Mean of each face's junction midpoints (for a square, its centre), or of its corners where the
+    circuit gives no junction nodes."""
+    try:
+        x, y = (np.asarray(v, np.float64) for v in circuit.get_node_coordinates())
+        n1, n2 = circuit.get_junction_nodes()
+        A = scipy.sparse.csc_matrix(circuit.get_cycle_matrix())
+        faces, per = A.indices, np.diff(A.indptr)
+        count = np.bincount(faces, minlength=A.shape[0])
+        mean = lambda v: np.bincount(faces, np.repeat(0.5 * (v[n1] + v[n2]), per), A.shape[0]) / count
+        return mean(x), mean(y)
+    except Exception:
+        cx, cy = circuit.get_face_centroids()
+        return np.asarray(cx, np.float64), np.asarray(cy, np.float64)
 
 
 def fast_poisson_grid(circuit, K):
