@@ -202,6 +202,12 @@ int jja_plan_set_resident(jja_plan* p, const jja_factor* f);
  * of the Schur complement of the other faces, and the couplings (three launches per solve). 12 bytes per
  * matrix entry; at most 32768 blocks of 128 x 64. jja_solve_static keeps the sweeps. */
 int jja_plan_set_blocks(jja_plan* p, const jja_factor* f, int leaf_faces);
+
+/* Triangular sweeps below, one product above: the faces above the largest subtrees of at most leaf_faces
+ * faces are solved by the inverse of their Schur complement (per tree of the forest) on the tensor
+ * cores between the two sweeps over the subtrees. For large circuits with few problems, whose upper tree
+ * levels are short dependent launches. Level schedule only; jja_solve_static keeps the whole sweeps. */
+int jja_plan_set_top_block(jja_plan* p, const jja_factor* f, int leaf_faces);
 /* Synchronises the device, then reads and clears the plan's device error flags: *flow_timeouts
  * = 1 if a wait of a dataflow sweep ran out of its bound since the last call (the results of
  * those steps are invalid), else 0. Returns JJA_ERR_NONFINITE when a time step of jja_run /

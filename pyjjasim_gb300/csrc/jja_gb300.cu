@@ -40,8 +40,10 @@ struct Error : std::runtime_error {
 #define JJA_CUDA(call)                                                                          \
   do {                                                                                          \
     cudaError_t e_ = (call);                                                                    \
-    if (e_ != cudaSuccess)                                                                      \
+    if (e_ != cudaSuccess) {                                                                    \
+      cudaGetLastError();   /* not left for the next launch's check */                          \
       throw Error(JJA_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));            \
+    }                                                                                           \
   } while (0)
 
 template <class F>
@@ -2455,6 +2457,8 @@ struct jja_plan {
   SineStrips strips{};
   BlockList sep_dst{};               // the dense sine matrix along the separators
   BlockList blocks[3];               // launches of the block solver (jja_plan_set_blocks; dst == 3)
+  Group leaves;                      // the sweeps below the separators' block (jja_plan_set_top_block; dst == 4)
+  jja_solve_tuning tuning{};
   // whole runs of a small circuit in one launch (jja_plan_set_resident; inv null: not)
   ResidentArgs res{};
   int64_t* res_slots = nullptr;      // output slots of a call's steps (phases, then currents)
@@ -2752,6 +2756,13 @@ void launch_face_solve(jja_plan* p, const Group& g, cudaStream_t st, bool zeroed
     launch_block_solve(p, g, st, zeroed);
     return;
   }
+  if (p->dst == 4) {   // sweeps below the separators, their block in the middle (into a zeroed x)
+    if (!zeroed) JJA_CUDA(cudaMemsetAsync(p->x, 0, (size_t)p->Nf * p->W * sizeof(double), st));
+    launch_levels(p, p->leaves, st, true);
+    launch_block_list(p, p->blocks[1], p->b, p->x, p->W, g.w0, g.wn, st);
+    launch_levels(p, p->leaves, st, false);
+    return;
+  }
   if (p->dst == 2) {
     launch_sine_solve(p, g, st);
     return;
@@ -2871,7 +2882,7 @@ StepArgs make_args(jja_plan* p, jja_state* s, const Group& g) {
   a.dt = p->dt;
   a.Isq = (s->Is.ptr && !s->Is.stride_t) ? jja_view{p->isq, p->W, 1, 0} : jja_view{nullptr, 0, 0, 0};
   a.resistive = p->resistive;
-  a.zero_x = p->dst == 3 ? p->x : nullptr;
+  a.zero_x = p->dst >= 3 ? p->x : nullptr;
   a.amp = (s->noise_mode != JJA_NOISE_NONE && s->T.ptr && !s->T.stride_t && !s->T.stride_w) ? p->amp : nullptr;
   return a;
 }
@@ -2984,6 +2995,23 @@ void one_chain(jja_plan* p) {
   p->adj_graphs.clear();
 }
 
+// the work items of a schedule as a group of problems [w0, w0 + wn) of the plan
+void set_group_items(jja_plan* p, Group& g, const Schedule& S, int w0, int wn) {
+  g.w0 = w0;
+  g.wn = wn;
+  g.fwd_ptr = S.fwd_ptr;
+  g.bwd_ptr = S.bwd_ptr;
+  g.level_packed = S.level_packed;
+  g.fwd_items = p->up(S.fi.data(), S.fi.size());
+  g.bwd_items = p->up(S.bi.data(), S.bi.size());
+  g.nz_f = (int)S.zf.size();
+  g.nz_b = (int)S.zb.size();
+  g.zrows_f = p->up(S.zf.data(), S.zf.size());
+  g.zrows_b = p->up(S.zb.data(), S.zb.size());
+  g.d_step = p->up<int64_t>(nullptr, 4);
+  JJA_CUDA(cudaMemset(g.d_step, 0, 4 * sizeof(int64_t)));
+}
+
 // The blocks of jja_plan_set_blocks and how they are computed. Leaves: the largest subtrees of the
 // elimination tree of at most leaf_faces columns (contiguous in the factor's order; every row outside
 // that a leaf touches is an off-diagonal row of its root); leaf_faces = 0: none, one block matrix.
@@ -3019,7 +3047,8 @@ struct BlockSetup {
       }
   }
 
-  BlockSetup(const jja::Factor& F, int leaf_faces) {
+  // top_only: the separators' matrix alone (the leaves stay with the sweeps)
+  BlockSetup(const jja::Factor& F, int leaf_faces, bool top_only = false) {
     const int ns = F.ns;
     std::vector<int> cols(ns), cnt(ns, 1);
     for (int s = 0; s < ns; ++s) cols[s] = F.sn_k[s];
@@ -3061,6 +3090,7 @@ struct BlockSetup {
       }
       trees.erase(std::remove_if(trees.begin(), trees.end(), [](const auto& t) { return t.empty(); }), trees.end());
     }
+    if (top_only) leaves.clear();
     for (Leaf& l : leaves) {
       l.cols_off = (int)lists.size();
       for (int i = 0; i < l.n; ++i) lists.push_back(l.c0 + i);
@@ -3151,6 +3181,122 @@ struct BlockSetup {
     if (longest_top) top_batches.push_back(std::move(top));
   }
 };
+
+// computes the blocks of B on the device from the plan's factor and gives them to the plan
+void make_blocks(jja_plan* p, const jja::Factor& F, const BlockSetup& B) {
+  const int n = p->Nf, ns = F.ns;
+  if (B.n_blocks > kBlocksMax)
+    throw Error(JJA_ERR_ARG, std::to_string(B.n_blocks) + " blocks of the matrix, more than " +
+                                 std::to_string(kBlocksMax));
+  // device scratch of the setup
+  struct Scratch {
+    std::vector<void*> mem;
+    cudaStream_t st = nullptr;
+    ~Scratch() {
+      if (st) cudaStreamDestroy(st);
+      for (void* m : mem) cudaFree(m);
+    }
+  } tmp;
+  int64_t ignored = 0;
+  auto scratch = [&](auto* h, size_t count) {
+    auto* d = upload(h, count, ignored);
+    tmp.mem.push_back((void*)d);
+    return d;
+  };
+  const int64_t nW = (int64_t)n * kBlockCols;
+  double* b = scratch((const double*)nullptr, (size_t)nW);
+  double* z = scratch((const double*)nullptr, (size_t)nW);
+  double* x = scratch((const double*)nullptr, (size_t)nW);
+  double* store = scratch((const double*)nullptr, (size_t)B.store_size);
+  JJA_CUDA(cudaStreamCreateWithFlags(&tmp.st, cudaStreamNonBlocking));
+  cudaStream_t st = tmp.st;
+  JJA_CUDA(cudaDeviceSynchronize());
+  // level sweeps over the supernodes of one part of the tree, 64 columns at a time
+  jja_solve_tuning tu{};
+  tu.subtree_rows = tu.pack_rows = -1;
+  tu.rows_per_lane = tu.rows_per_lane_fwd = 1;
+  constexpr int kW = kBlockCols, kWB = 32;
+  struct Part {
+    Schedule S;
+    int4 *fi, *bi;
+    int32_t *zf, *zb;
+  };
+  auto make_part = [&](const std::vector<char>& skip) {
+    Part P{build_schedule(F, kW, tu, 0, -1, &skip), nullptr, nullptr, nullptr, nullptr};
+    P.fi = scratch(P.S.fi.data(), P.S.fi.size());
+    P.bi = scratch(P.S.bi.data(), P.S.bi.size());
+    P.zf = scratch(P.S.zf.data(), P.S.zf.size());
+    P.zb = scratch(P.S.zb.data(), P.S.zb.size());
+    return P;
+  };
+  auto zero_rows = [&](double* v, const int32_t* rows, size_t count) {
+    if (count)
+      launch(false, k_zero_rows, grid_for((int64_t)count * kW, 256), 256, st, v, rows, (int)count, kW, 0, kW,
+             fast_div(kW), (unsigned*)nullptr, 0);
+  };
+  auto forward = [&](const Part& P) {
+    zero_rows(z, P.zf, P.S.zf.size());
+    for (int l = 0; l < P.S.n_levels; ++l)
+      if (const int m = (int)(P.S.fwd_ptr[l + 1] - P.S.fwd_ptr[l]))
+        launch(false, k_fwd_level<1, false>, (m + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, st, p->F,
+               (const int4*)(P.fi + P.S.fwd_ptr[l]), m, kW, kWB, b, z);
+  };
+  auto backward = [&](const Part& P) {
+    zero_rows(x, P.zb, P.S.zb.size());
+    for (int l = P.S.n_levels - 1; l >= 0; --l)
+      if (const int m = (int)(P.S.bwd_ptr[l + 1] - P.S.bwd_ptr[l]))
+        launch(false, k_bwd_level<1, false>, (m + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, st, p->F,
+               (const int4*)(P.bi + P.S.bwd_ptr[l]), m, kW, kWB, (const double*)z, x);
+  };
+  auto clear = [&](double* v) { JJA_CUDA(cudaMemsetAsync(v, 0, nW * sizeof(double), st)); };
+  std::vector<char> leaf_only(ns), top_only(ns);
+  for (int s = 0; s < ns; ++s) {
+    leaf_only[s] = B.leaf_of[s] < 0;    // skip the separators
+    top_only[s] = B.leaf_of[s] >= 0;    // skip the leaves
+  }
+  int32_t* lists = p->up(B.lists.data(), B.lists.size());
+  const StoreRows* jobs = scratch(B.jobs.data(), B.jobs.size());
+  auto store_rows = [&](const double* v, int first, int count) {
+    if (count)
+      launch(false, k_store_rows, count, 256, st, v, (const int32_t*)lists, (const StoreRows*)(jobs + first), store);
+  };
+  auto run = [&](const std::vector<BlockSetup::Batch>& batches, const Part& P, bool leaves) {
+    for (const BlockSetup::Batch& t : batches) {
+      const int32_t* rows = scratch(t.rows.data(), t.rows.size());
+      const int32_t* pos = scratch(t.pos.data(), t.pos.size());
+      for (const BlockSetup::Chunk& c : t.chunks) {
+        clear(b);
+        launch(false, k_unit_columns, grid_for((int64_t)t.rows.size(), 256), 256, st, b, rows, pos, (int)t.rows.size(),
+               c.c0);
+        forward(P);
+        store_rows(b, c.couple0, c.n_couple);   // the separators' rows of b now hold -G_l^T
+        if (leaves) clear(x);                   // zero at the separators
+        backward(P);
+        store_rows(x, c.own0, c.n_own);
+      }
+    }
+  };
+  if (!B.leaf_batches.empty()) run(B.leaf_batches, make_part(leaf_only), true);
+  run(B.top_batches, make_part(top_only), false);
+  unsigned char* mats = p->up<unsigned char>(nullptr, (size_t)B.n_blocks * kBlockMatBytes);
+  int* e_mat = p->up<int>(nullptr, (size_t)B.n_blocks);
+  BlockSource* src = scratch(B.sources.data(), B.sources.size());
+  if (B.n_blocks)
+    launch(false, k_block_digits, (int)B.n_blocks, 256, st, (const double*)store, (const BlockSource*)src, mats, e_mat);
+  JJA_CUDA(cudaGetLastError());
+  JJA_CUDA(cudaStreamSynchronize(st));
+  for (int k = 0; k < 3; ++k) {
+    BlockList L{};
+    L.n = (int)B.units[k].size();
+    if (L.n) L.units = p->up(B.units[k].data(), B.units[k].size());
+    L.in_rows = L.out_rows = lists;
+    L.mats = mats;
+    L.e_mat = e_mat;
+    p->blocks[k] = L;
+  }
+  for (int wp : {16, 32, 48, 64})
+    JJA_CUDA(cudaFuncSetAttribute(block_kernel(wp), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem_bytes(wp)));
+}
 
 // graph of G fused steps for the state's current buffers (captured on first use, then cached);
 // with several groups the graph forks into their streams and joins back
@@ -3321,6 +3467,7 @@ int jja_plan_create(const jja_plan_desc* d, const jja_factor* fac, jja_plan** ou
     // launch shape of the triangular solves (jja_solve_tuning; 0 = default), validated again
     // by build_schedule
     const jja_solve_tuning& tu = d->tuning;
+    p->tuning = tu;
     p->WB = resolve_rhs_block(d->W, tu);
     p->rows_per_lane = rows_per_lane_of(tu, false, d->W, F.n);
     p->rows_per_lane_fwd = rows_per_lane_of(tu, true, d->W, F.n);
@@ -3388,22 +3535,7 @@ int jja_plan_create(const jja_plan_desc* d, const jja_factor* fac, jja_plan** ou
     const Schedule S = build_schedule(F, d->W, tu);
     check_schedule(S);
     p->n_levels = S.n_levels;
-    auto set_group = [&](Group& g, const Schedule& Sg, int w0, int wn) {
-      g.w0 = w0;
-      g.wn = wn;
-      g.fwd_ptr = Sg.fwd_ptr;
-      g.bwd_ptr = Sg.bwd_ptr;
-      g.level_packed = Sg.level_packed;
-      g.fwd_items = p->up(Sg.fi.data(), Sg.fi.size());
-      g.bwd_items = p->up(Sg.bi.data(), Sg.bi.size());
-      g.nz_f = (int)Sg.zf.size();
-      g.nz_b = (int)Sg.zb.size();
-      g.zrows_f = p->up(Sg.zf.data(), Sg.zf.size());
-      g.zrows_b = p->up(Sg.zb.data(), Sg.zb.size());
-      g.d_step = p->up<int64_t>(nullptr, 4);
-      JJA_CUDA(cudaMemset(g.d_step, 0, 4 * sizeof(int64_t)));
-    };
-    set_group(p->all, S, 0, d->W);
+    set_group_items(p.get(), p->all, S, 0, d->W);
     if (!S.sp_items.empty()) {
       SubPackDev& sp = p->subp;
       sp.items = p->up(S.sp_items.data(), S.sp_items.size());
@@ -3466,7 +3598,7 @@ int jja_plan_create(const jja_plan_desc* d, const jja_factor* fac, jja_plan** ou
           const Schedule Sg = build_schedule(F, d->W, tu, lo, hi);
           if (Sg.n_levels != S.n_levels || Sg.subs.size() != S.subs.size())
             throw Error(JJA_ERR_INTERNAL, "group schedules differ in levels or subtrees");
-          set_group(p->groups[gi], Sg, lo, hi - lo);
+          set_group_items(p.get(), p->groups[gi], Sg, lo, hi - lo);
           if (gi > 0) JJA_CUDA(cudaStreamCreateWithFlags(&p->groups[gi].stream, cudaStreamNonBlocking));
           JJA_CUDA(cudaEventCreateWithFlags(&p->groups[gi].done, cudaEventDisableTiming));
         }
@@ -3869,122 +4001,31 @@ int jja_plan_set_sine_solver(jja_plan* p, int mx, int my, const int32_t* grid_fa
 int jja_plan_set_blocks(jja_plan* p, const jja_factor* fac, int leaf_faces) {
   return guarded([&] {
     if (!p || !fac || leaf_faces < 0) throw Error(JJA_ERR_ARG, "jja_plan_set_blocks: bad arguments");
-    const jja::Factor& F = *fac->f;
-    const int n = p->Nf, ns = F.ns;
-    if (F.n != n) throw Error(JJA_ERR_ARG, "jja_plan_set_blocks: factor order != Nf");
+    if (fac->f->n != p->Nf) throw Error(JJA_ERR_ARG, "jja_plan_set_blocks: factor order != Nf");
     if (p->dst || p->res.inv) throw Error(JJA_ERR_ARG, "jja_plan_set_blocks: the plan already has another solver");
-    BlockSetup B(F, leaf_faces);
-    if (B.n_blocks > kBlocksMax)
-      throw Error(JJA_ERR_ARG, "jja_plan_set_blocks: " + std::to_string(B.n_blocks) + " blocks of the matrix, more than " +
-                                   std::to_string(kBlocksMax));
-    // device scratch of the setup
-    struct Scratch {
-      std::vector<void*> mem;
-      cudaStream_t st = nullptr;
-      ~Scratch() {
-        if (st) cudaStreamDestroy(st);
-        for (void* m : mem) cudaFree(m);
-      }
-    } tmp;
-    int64_t ignored = 0;
-    auto scratch = [&](auto* h, size_t count) {
-      auto* d = upload(h, count, ignored);
-      tmp.mem.push_back((void*)d);
-      return d;
-    };
-    const int64_t nW = (int64_t)n * kBlockCols;
-    double* b = scratch((const double*)nullptr, (size_t)nW);
-    double* z = scratch((const double*)nullptr, (size_t)nW);
-    double* x = scratch((const double*)nullptr, (size_t)nW);
-    double* store = scratch((const double*)nullptr, (size_t)B.store_size);
-    JJA_CUDA(cudaStreamCreateWithFlags(&tmp.st, cudaStreamNonBlocking));
-    cudaStream_t st = tmp.st;
-    JJA_CUDA(cudaDeviceSynchronize());
-    // level sweeps over the supernodes of one part of the tree, 64 columns at a time
-    jja_solve_tuning tu{};
-    tu.subtree_rows = tu.pack_rows = -1;
-    tu.rows_per_lane = tu.rows_per_lane_fwd = 1;
-    constexpr int kW = kBlockCols, kWB = 32;
-    struct Part {
-      Schedule S;
-      int4 *fi, *bi;
-      int32_t *zf, *zb;
-    };
-    auto make_part = [&](const std::vector<char>& skip) {
-      Part P{build_schedule(F, kW, tu, 0, -1, &skip), nullptr, nullptr, nullptr, nullptr};
-      P.fi = scratch(P.S.fi.data(), P.S.fi.size());
-      P.bi = scratch(P.S.bi.data(), P.S.bi.size());
-      P.zf = scratch(P.S.zf.data(), P.S.zf.size());
-      P.zb = scratch(P.S.zb.data(), P.S.zb.size());
-      return P;
-    };
-    auto zero_rows = [&](double* v, const int32_t* rows, size_t count) {
-      if (count)
-        launch(false, k_zero_rows, grid_for((int64_t)count * kW, 256), 256, st, v, rows, (int)count, kW, 0, kW,
-               fast_div(kW), (unsigned*)nullptr, 0);
-    };
-    auto forward = [&](const Part& P) {
-      zero_rows(z, P.zf, P.S.zf.size());
-      for (int l = 0; l < P.S.n_levels; ++l)
-        if (const int m = (int)(P.S.fwd_ptr[l + 1] - P.S.fwd_ptr[l]))
-          launch(false, k_fwd_level<1, false>, (m + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, st, p->F,
-                 (const int4*)(P.fi + P.S.fwd_ptr[l]), m, kW, kWB, b, z);
-    };
-    auto backward = [&](const Part& P) {
-      zero_rows(x, P.zb, P.S.zb.size());
-      for (int l = P.S.n_levels - 1; l >= 0; --l)
-        if (const int m = (int)(P.S.bwd_ptr[l + 1] - P.S.bwd_ptr[l]))
-          launch(false, k_bwd_level<1, false>, (m + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, st, p->F,
-                 (const int4*)(P.bi + P.S.bwd_ptr[l]), m, kW, kWB, (const double*)z, x);
-    };
-    auto clear = [&](double* v) { JJA_CUDA(cudaMemsetAsync(v, 0, nW * sizeof(double), st)); };
-    std::vector<char> leaf_only(ns), top_only(ns);
-    for (int s = 0; s < ns; ++s) {
-      leaf_only[s] = B.leaf_of[s] < 0;    // skip the separators
-      top_only[s] = B.leaf_of[s] >= 0;    // skip the leaves
-    }
-    int32_t* lists = p->up(B.lists.data(), B.lists.size());
-    const StoreRows* jobs = scratch(B.jobs.data(), B.jobs.size());
-    auto store_rows = [&](const double* v, int first, int count) {
-      if (count)
-        launch(false, k_store_rows, count, 256, st, v, (const int32_t*)lists, (const StoreRows*)(jobs + first), store);
-    };
-    auto run = [&](const std::vector<BlockSetup::Batch>& batches, const Part& P, bool leaves) {
-      for (const BlockSetup::Batch& t : batches) {
-        const int32_t* rows = scratch(t.rows.data(), t.rows.size());
-        const int32_t* pos = scratch(t.pos.data(), t.pos.size());
-        for (const BlockSetup::Chunk& c : t.chunks) {
-          clear(b);
-          launch(false, k_unit_columns, grid_for((int64_t)t.rows.size(), 256), 256, st, b, rows, pos, (int)t.rows.size(),
-                 c.c0);
-          forward(P);
-          store_rows(b, c.couple0, c.n_couple);   // the separators' rows of b now hold -G_l^T
-          if (leaves) clear(x);                   // zero at the separators
-          backward(P);
-          store_rows(x, c.own0, c.n_own);
-        }
-      }
-    };
-    if (!B.leaf_batches.empty()) run(B.leaf_batches, make_part(leaf_only), true);
-    run(B.top_batches, make_part(top_only), false);
-    unsigned char* mats = p->up<unsigned char>(nullptr, (size_t)B.n_blocks * kBlockMatBytes);
-    int* e_mat = p->up<int>(nullptr, (size_t)B.n_blocks);
-    BlockSource* src = scratch(B.sources.data(), B.sources.size());
-    launch(false, k_block_digits, (int)B.n_blocks, 256, st, (const double*)store, (const BlockSource*)src, mats, e_mat);
-    JJA_CUDA(cudaStreamSynchronize(st));
-    for (int k = 0; k < 3; ++k) {
-      BlockList L{};
-      L.n = (int)B.units[k].size();
-      if (L.n) L.units = p->up(B.units[k].data(), B.units[k].size());
-      L.in_rows = L.out_rows = lists;
-      L.mats = mats;
-      L.e_mat = e_mat;
-      p->blocks[k] = L;
-    }
-    for (int wp : {16, 32, 48, 64})
-      JJA_CUDA(cudaFuncSetAttribute(block_kernel(wp), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem_bytes(wp)));
+    make_blocks(p, *fac->f, BlockSetup(*fac->f, leaf_faces));
     one_chain(p);
     p->dst = 3;
+  });
+}
+
+int jja_plan_set_top_block(jja_plan* p, const jja_factor* fac, int leaf_faces) {
+  return guarded([&] {
+    if (!p || !fac || leaf_faces < 1) throw Error(JJA_ERR_ARG, "jja_plan_set_top_block: bad arguments");
+    const jja::Factor& F = *fac->f;
+    if (F.n != p->Nf) throw Error(JJA_ERR_ARG, "jja_plan_set_top_block: factor order != Nf");
+    if (p->dst || p->res.inv || p->flow || p->coop)
+      throw Error(JJA_ERR_ARG, "jja_plan_set_top_block: the plan already has another solver or schedule");
+    const BlockSetup B(F, leaf_faces, true);
+    make_blocks(p, F, B);
+    // the sweeps' work items without the separators
+    std::vector<char> top(F.ns);
+    for (int s = 0; s < F.ns; ++s) top[s] = B.leaf_of[s] < 0;
+    const Schedule S = build_schedule(F, p->W, p->tuning, 0, p->W, &top);
+    if (S.n_levels != p->n_levels) throw Error(JJA_ERR_INTERNAL, "leaf schedule differs in levels");
+    set_group_items(p, p->leaves, S, 0, p->W);
+    one_chain(p);
+    p->dst = 4;
   });
 }
 

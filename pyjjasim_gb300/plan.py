@@ -270,9 +270,18 @@ def resident_fits(circuit, W):
 #   honeycomb 31x31 (1830 faces)   W = 1  55 / 17 / 21    W = 24  70 / 27 / 28    W = 96  115 / 63 / 40
 #   triangular 64x48 (11970 faces) W = 1  89 / - / 33     W = 24  145 / - / 61    W = 96  240 / - / 145
 #   triangular 80x80 (25122 faces) W = 1  97 / - / 66     W = 24  188 / - / 111   W = 256 906 / - / 734
-# and with leaves of 384:
-#   square 230x200, R spread (45571) W = 1  141 / 139     W = 4  157 / 154        W = 24  380 / 247
-#   square 300x300, R spread (89401) W = 1  204 / 317     W = 4  254 / 362        W = 24  670 / 588
+# Larger circuits: leaves of 384 while the problems pay for reading the blocks, else sweeps over subtrees
+# with one product for the separators above them (sweeps / leaves of 384 / subtrees of 3072 / of 6144):
+#   square 230x200, R spread (45571)   W = 1  142 / 136 / 114 / 121   W = 16  270 / 193 / 227 / 238
+#   square 300x300, R spread (89401)   W = 1  201 / 317 / 201 / 190   W = 16  419 / 451 / 365 / 373
+#                                                                     W = 64 1213 / 1164 / 985 / 1021
+#   square 500x500, R spread (249001)  W = 1  345 / - / 463 / 343     W = 16  984 / - / 1014 / 897
+#   24 arrays in one union (274672)    W = 1  351 / - / 320 / 312     8 of them (90876) 167 / - / 155 / 151
+# and for many problems, or many small arrays in one union (sweeps / leaves of 256 or 384 / subtrees of 384 /
+# of 768 / of 3072):
+#   triangular 64x48 (11970)           W = 512  745 / 586 / 631 / 642 / 746     W = 2048 2461 / 2485 / 2121 / 2104 / 2326
+#   square 230x200, R spread (45571)   W = 128 1144 / 899 / - / - / 996         W = 512  3220 / 3379 / - / - / 2917
+#   28 arrays (73184)                  W = 1  145 / - / 115 / 129 / 139         60 (151102) 196 / - / 215 / 209 / 198
 INVERSE_MAX_FACES = 2048
 INVERSE_MAX_WORK = 11000    # 128 x 64 blocks of the inverse x problems
 
@@ -282,11 +291,25 @@ def block_leaf(circuit, W):
     n = circuit._Nf()
     if n <= INVERSE_MAX_FACES and -(-n // 128) * -(-n // 64) * W <= INVERSE_MAX_WORK:
         return 0
+    if n * W > 1 << 24:     # as much data as blocks: their products cost what the sweeps cost
+        return None
     if n <= 1 << 15:
         return 256
-    if W >= 8 and n <= 1 << 16 or W >= 24 and n <= 92000:
-        return 384
-    return None
+    return 384 if W >= 8 and n <= 1 << 16 else None
+
+
+def top_leaf(circuit, W):
+    """The subtree size below which the default plan keeps the sweeps when block_leaf takes none (a
+    product solves the faces above), or None."""
+    n = circuit._Nf()
+    tree = n // getattr(circuit, "components", 1)   # a ragged union's circuits are trees of their own
+    if n > 1 << 19:
+        return None
+    if tree < n and tree <= 6144:
+        return 384 if n <= 100_000 else None
+    if tree <= 1 << 17:
+        return 768 if n <= 1 << 15 else 3072 if n <= 1 << 16 else 6144
+    return 6144 if W >= 16 else None
 
 
 def untuned(tuning):
@@ -299,7 +322,7 @@ class DevicePlan:
     """Circuit tables + factor uploaded for W problems (owned C object)."""
 
     def __init__(self, circuit, factor, A, W, dt, stencil_width, stencil, Ic_w=None, tuning=None, fast_poisson=None,
-                 sine=None, resident=False, blocks=None):
+                 sine=None, resident=False, blocks=None, top=None):
         """``tuning``: dict with any of rhs_block, rows_per_lane, target_warps, min_piece (the
         launch shape of the triangular solves; missing or 0 = library default)."""
         Nj, Nf = circuit._Nj(), circuit._Nf()
@@ -347,9 +370,17 @@ class DevicePlan:
         if resident:
             N.check(N.lib().jja_plan_set_resident(h, factor.handle))
             self.resident = True
-        self.blocks = blocks
-        if blocks is not None:
-            N.check(N.lib().jja_plan_set_blocks(h, factor.handle, int(blocks)))
+        self.blocks = self.top = None
+        try:     # a tree whose blocks are too many (or too large for the memory left) keeps the sweeps
+            if blocks is not None:
+                N.check(N.lib().jja_plan_set_blocks(h, factor.handle, int(blocks)))
+                self.blocks = blocks
+            elif top is not None:
+                N.check(N.lib().jja_plan_set_top_block(h, factor.handle, int(top)))
+                self.top = top
+        except N.JJAError as e:
+            if e.code != 1 and "out of memory" not in str(e):
+                raise
         self.device_bytes = N.lib().jja_plan_device_bytes(h)
 
     def solve(self, b_dev, x_dev, stream=0):
@@ -458,7 +489,7 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
     (fast_poisson_grid): True (radix-2 grids), False (the sweeps), or "auto": unless ``tuning`` asks for
     sweeps of some shape, whichever of the resident steps (resident_fits), the radix-2 or tensor-core
     transforms, and the dense blocks (block_leaf) is fastest for the circuit and W."""
-    fp = sine = blocks = None
+    fp = sine = blocks = top = None
     matrices = face_matrix(circuit, dt)
     n_faces = circuit._Nf()
     auto = fast_poisson == "auto" and untuned(tuning)
@@ -473,6 +504,7 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
                 sine = None
         if sine is None:
             blocks = block_leaf(circuit, W)
+            top = top_leaf(circuit, W) if blocks is None else None
     if blocks is not None:     # the block solver cuts the tree itself: nested dissection with small leaves
         nd_leaf = 8 if nd_leaf is None else nd_leaf
         ordering = "nd" if ordering == "auto" else ordering
@@ -484,7 +516,7 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
         Ic_w = np.ascontiguousarray(np.broadcast_to(np.asarray(Ic_w, np.float64), (circuit._Nj(), W)))
     ic = np.asarray(circuit._Ic(), np.float64) if Ic_w is None else Ic_w
     tkey = tuple(int((tuning or {}).get(f, 0)) for f in TUNING_FIELDS)
-    key = (fkey, W, stencil_width, Ic_w is None, tkey, fp is not None, sine is not None, resident, blocks,
+    key = (fkey, W, stencil_width, Ic_w is None, tkey, fp is not None, sine is not None, resident, blocks, top,
            _digest(ic, *coef, Rv, A.indptr, A.indices, A.data))
     with _CACHE_LOCK:
         p = _PLANS.get(key)
@@ -492,7 +524,7 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
             _PLANS.move_to_end(key)
             return p
     p = DevicePlan(circuit, factor, A, W, dt, stencil_width, stencil, Ic_w=Ic_w, tuning=tuning, fast_poisson=fp,
-                   sine=sine, resident=resident, blocks=blocks)
+                   sine=sine, resident=resident, blocks=blocks, top=top)
     with _CACHE_LOCK:
         _PLANS[key] = p
         while len(_PLANS) > MAX_PLANS:

@@ -152,6 +152,7 @@ class RaggedBatch:
                                cut_matrix=scipy.sparse.block_diag(M_blocks, format="csc"),
                                node_x=np.concatenate(xs), node_y=np.concatenate(ys), node1=np.concatenate(n1s),
                                node2=np.concatenate(n2s))
+        self.circuit.components = len(A_blocks)
 
     def _union_source(self, getter_name, timedep_name, rows):
         """Concatenate one source over all (problem, w) copies: array (N, 1, 1) or callable."""

@@ -16,14 +16,19 @@ from pyjjasim_gb300.circuit import HoneycombArray, SquareArray, TriangularArray
 def test_rule():
     assert P.block_leaf(HoneycombArray(24, 24), 61) == 0
     assert P.block_leaf(HoneycombArray(24, 24), 700) == 256
-    assert P.block_leaf(SquareArray(301, 301), 24) == 384 and P.block_leaf(SquareArray(301, 301), 8) is None
+    c = SquareArray(230, 200)
+    assert P.block_leaf(c, 8) == 384 and P.block_leaf(c, 4) is None and P.top_leaf(c, 4) == 3072
+    assert P.block_leaf(c, 512) is None and P.block_leaf(TriangularArray(64, 48), 2048) is None
+    c.components = 20
+    assert P.top_leaf(c, 1) == 384
 
 
-def _solve(c, b, leaf):
+def _solve(c, b, leaf, top=None):
     import torch
     A, K = P.face_matrix(c, 0.05)
     factor, A, _ = P.get_factor(c, 0.05)
-    pl = P.DevicePlan(c, factor, A, b.shape[1], 0.05, 3, ((1.0, -1.0, 0.0), (1.0, -2.0, 1.0)), blocks=leaf)
+    pl = P.DevicePlan(c, factor, A, b.shape[1], 0.05, 3, ((1.0, -1.0, 0.0), (1.0, -2.0, 1.0)), blocks=leaf, top=top)
+    assert (pl.blocks, pl.top) == (leaf, top)
     bd = torch.from_numpy(b).cuda()
     xd = torch.empty_like(bd)
     s = torch.cuda.Stream()
@@ -58,6 +63,24 @@ def test_solve_matches_scipy(lattice, nx, ny, W, leaf):
     y, _ = _solve(c, b, None)
     rx, ry = (np.linalg.norm(K @ v - b, axis=0) / np.maximum(np.linalg.norm(b, axis=0), 1e-300) for v in (x, y))
     print(f"Nf={Nf} W={W}: residual {rx.max():.2e}, sweeps {ry.max():.2e}")
+    assert rx.max() <= max(4.0 * ry.max(), 1e-13)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lattice,nx,ny,W,top", [(SquareArray, 9, 9, 1, 4), (SquareArray, 60, 55, 1, 300),
+                                                 (TriangularArray, 30, 24, 3, 500), (HoneycombArray, 30, 24, 40, 128),
+                                                 (SquareArray, 90, 70, 17, 1000), (SquareArray, 12, 12, 2, 4000), (TriangularArray, 25, 22, 300, 768)])
+def test_top_block_matches_scipy(lattice, nx, ny, W, top):
+    c = lattice(nx, ny)
+    rng = np.random.default_rng(nx * ny + W)
+    c.set_resistance(rng.lognormal(0.0, 0.4, c._Nj()))
+    b = rng.standard_normal((c._Nf(), W)) * 10.0 ** rng.uniform(-12, 12, (1, W))
+    x, K = _solve(c, b, None, top)
+    ref = scipy.sparse.linalg.spsolve(K.tocsc(), b).reshape(x.shape)
+    err = np.abs(x - ref).max(0) / np.maximum(np.abs(ref).max(0), 1e-300)
+    assert float(err.max()) <= 1e-11, err.argmax()
+    y, _ = _solve(c, b, None)
+    rx, ry = (np.linalg.norm(K @ v - b, axis=0) / np.linalg.norm(b, axis=0) for v in (x, y))
     assert rx.max() <= max(4.0 * ry.max(), 1e-13)
 
 
