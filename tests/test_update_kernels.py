@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 from pyjjasim_gb300 import TimeEvolutionProblem, backend
-from pyjjasim_gb300.circuit import HoneycombArray, SquareArray
+from pyjjasim_gb300.circuit import HoneycombArray, SquareArray, TriangularArray
 
 
 @pytest.mark.gpu
@@ -39,3 +39,24 @@ def test_fast_steps_match_general_steps(W, C, T, driven, per_w, flux):
     for x, y in zip(a.history(), b.history()):
         assert float((x - y).abs().max()) <= 1e-12 * max(1.0, float(y.abs().max()))
     assert torch.equal(th[-1], b.theta())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lattice", [TriangularArray, SquareArray, HoneycombArray])
+@pytest.mark.parametrize("W", [1, 34])
+def test_face_sums_of_each_degree(lattice, W):
+    """The fast face kernel (flux constant in time) against the general one (the same flux as a function of time):
+    the same operations in the same order."""
+    import torch
+    c = lattice(14, 11)
+    c.set_resistance(np.random.default_rng(W).uniform(0.8, 1.2, c._Nj()))
+    f = np.random.default_rng(W).uniform(-0.3, 0.3, (c._Nf(), W, 1))
+    out = []
+    for flux in (f, lambda i: f[:, :, 0]):
+        prob = TimeEvolutionProblem(c, time_step=0.05, time_step_count=20, external_flux=flux,
+                                    current_sources=0.3 * np.ones((c._Nj(), W, 1)))
+        sim = backend.GpuSimulation(prob, fast_poisson=False)
+        sim.run(20)
+        sim.synchronize()
+        out.append(sim.theta().clone())
+    assert float((out[0] - out[1]).abs().max()) <= 1e-13
