@@ -46,7 +46,9 @@ def _solve(c, b, sine):
 SIZES = [(2, 2, 1), (2, 9, 3), (3, 4, 2), (18, 33, 7), (33, 34, 128), (34, 17, 129), (64, 64, 5), (66, 65, 33),
          (96, 97, 40), (98, 99, 2), (128, 128, 3), (129, 128, 65), (129, 300, 2), (300, 129, 2), (101, 60, 24),
          # both sides longer than 128 faces: strips of one and two widths, one and several separators
-         (131, 130, 2), (130, 131, 17), (257, 257, 1), (140, 400, 3), (390, 135, 2), (300, 300, 5), (131, 131, 260)]
+         (131, 130, 2), (130, 131, 17), (257, 257, 1), (140, 400, 3), (390, 135, 2), (300, 300, 5), (131, 131, 260),
+         # more tiles than blocks, a last wave of half tiles
+         (128, 128, 160), (40, 35, 610), (20, 33, 1300)]
 
 
 @pytest.mark.gpu
