@@ -124,7 +124,11 @@ __device__ __forceinline__ double philox_normal(uint64_t seed, uint64_t elem, ui
   const float u1 = ((float)(r.x >> 8) + 1.0f) * (1.0f / 16777216.0f);  // (0, 1]
   const float u2 = (float)(r.y >> 8) * (1.0f / 16777216.0f);           // [0, 1)
   const float rad = sqrtf(-2.0f * logf(u1));
-  return (double)(rad * cospif(2.0f * u2));
+  // to double by its bits (the conversion instruction takes the FP64 pipe): 0 or a normal number, since
+  // the nonzero factors are at least 3e-4 and 1e-7
+  const uint32_t n = __float_as_uint(rad * cospif(2.0f * u2)), mag = n & 0x7fffffffu;
+  const uint32_t hi = mag ? (mag >> 3) + (896u << 20) : 0u;
+  return __hiloint2double((int)(hi | (n & 0x80000000u)), (int)(n << 29));
 }
 
 // Programmatic dependent launch: every kernel first lets the next kernel of its stream be
@@ -457,6 +461,15 @@ __host__ __device__ __forceinline__ void fast_sincos(double x, const longlong2* 
   c_out = double_of_fixed62(cos_fixed(r, sc), false);
 }
 
+// sum of e_k th_k over the first N values of the history
+template <int N>
+__device__ __forceinline__ double stencil_sum(const double* e, const double* th) {
+  double v = e[0] * th[0];
+#pragma unroll
+  for (int k = 1; k < N; ++k) v = fma(e[k], th[k], v);
+  return v;
+}
+
 // q(j, w) = x / c0 for the step whose phase history is th[0..] (time_evolution.py:533-558):
 //   x = sqrt(2 T Rv) xi - Is + Ic sin(sum_k e_k th_k) + sum_k c_k th_k
 // evaluated with the coefficients already divided by c0 (Icq = Ic/c0, coefq_k = c_k/c0,
@@ -465,14 +478,15 @@ __host__ __device__ __forceinline__ void fast_sincos(double x, const longlong2* 
 // `step` keys the Philox stream; tt = step - window start indexes time-dependent sources.
 __device__ __forceinline__ double junction_q(const StepArgs& a, const Tables& t, int64_t e, int64_t j, int64_t w,
                                             const double* th, int64_t step, int64_t tt) {
+  // (terms beyond the stencil are left out by branches on its width: an FP64 instruction that a predicate
+  // turns off occupies the pipe like one that runs)
   double arg;
   if (a.width == 3) {
     arg = fma(2.0, th[0], -th[1]);        // 2 th1 - th2 with the reference's single rounding
+  } else if (a.width == 4) {
+    arg = stencil_sum<3>(a.e, th);
   } else {
-    arg = a.e[0] * th[0];
-#pragma unroll
-    for (int k = 1; k < 4; ++k)
-      if (k < a.width - 1) arg = fma(a.e[k], th[k], arg);
+    arg = stencil_sum<4>(a.e, th);
   }
   const double s = fast_sin(arg, t.sincos);
   const double icq = __ldg(t.Icq + (t.ic_per_w ? e : j));
@@ -481,9 +495,15 @@ __device__ __forceinline__ double junction_q(const StepArgs& a, const Tables& t,
     X = fma(icq, s, -th[0]);
   } else {
     X = icq * s;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (k < a.width - 1) X = fma(__ldg(t.coefq + (int64_t)k * a.Nj + j), th[k], X);
+    const double* c = t.coefq + j;
+    X = fma(__ldg(c), th[0], X);
+    X = fma(__ldg(c + a.Nj), th[1], X);
+    if (a.width == 4) {
+      X = fma(__ldg(c + (int64_t)2 * a.Nj), th[2], X);
+    } else if (a.width > 4) {
+      const double c2 = __ldg(c + (int64_t)2 * a.Nj), c3 = __ldg(c + (int64_t)3 * a.Nj);
+      X = fma(c3, th[3], fma(c2, th[2], X));
+    }
   }
   // Is / c0: precomputed when Is does not change with time, else scaled here
   const double isq = a.Isq.ptr ? view_at(a.Isq, j, w) : view_at(a.Is, j, w, tt) * __ldg(t.inv_c0 + j);
@@ -541,6 +561,8 @@ __global__ void k_set_counters(int64_t* __restrict__ d_step, int64_t step, int64
 
 // b(p, w) = sum_j A_pj (q_j - theta_s_j) - 2 pi f_p, p in the factor's face order. Also
 // publishes step + 1 in d_step[1] (read by k_update, which evaluates the next step's q).
+// D: at least the junctions of every face (0: any number, from the CSR lists).
+template <int D>
 __global__ void __launch_bounds__(256) k_face_rhs(StepArgs a, Tables t, const double* __restrict__ q,
                                                   double* __restrict__ b) {
   pdl_begin();
@@ -549,21 +571,21 @@ __global__ void __launch_bounds__(256) k_face_rhs(StepArgs a, Tables t, const do
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t p = a.by_wn(i), w = a.w0 + (i - p * a.wn), e = p * a.W + w;
     double acc = 0.0;
-    if (t.face_deg) {
+    if constexpr (D > 0) {
       // fixed-degree layout: all index loads, then all value loads, then the sum
-      int code[kEllMax];
-      double v[kEllMax];
+      int code[D];
+      double v[D];
 #pragma unroll
-      for (int d = 0; d < kEllMax; ++d) code[d] = d < t.face_deg ? __ldg(t.fj_ell + p * t.face_deg + d) : -1;
+      for (int d = 0; d < D; ++d) code[d] = d < t.face_deg ? __ldg(t.fj_ell + p * t.face_deg + d) : -1;
 #pragma unroll
-      for (int d = 0; d < kEllMax; ++d) {
+      for (int d = 0; d < D; ++d) {
         const int64_t j = code[d] >> 1;
         v[d] = code[d] >= 0 ? q[j * a.W + w] : 0.0;
         if (a.theta_s && code[d] >= 0) v[d] -= a.theta_s[j * a.W + w];
       }
       acc = signed_by(v[0], code[0] & 1);
 #pragma unroll
-      for (int d = 1; d < kEllMax; ++d)
+      for (int d = 1; d < D; ++d)
         if (code[d] >= 0) acc += signed_by(v[d], code[d] & 1);
     } else {
       const int64_t i0 = __ldg(t.fj_ptr + p), i1 = __ldg(t.fj_ptr + p + 1);
@@ -626,11 +648,13 @@ __global__ void __launch_bounds__(256, JJA_UPDATE_MIN_BLOCKS) k_update(StepArgs 
 // current sources, and no noise or Philox noise of an amplitude table; V adjacent problems per
 // thread. The general kernel spends 380 instructions per element, mostly on strided views and
 // 64-bit index arithmetic; this one shares them between the V problems (two 16-byte loads per
-// array). Measured per step: 128x128 x 512 0.301 -> 0.193 ms, 1024x1024 x 8 with C, L and noise
-// 0.721 -> 0.290 ms (there the amplitude table saves the FP64 square root). Bound by the latency of
-// three dependent reads (face numbers, face currents, sine table) at 32 warps per SM, with the FP64
-// pipe 75 % busy; 5 or 6 blocks per SM (fewer registers) and a thread per pair without the grid
-// loop measured the same.
+// array). Measured per step: 128x128 x 512 0.301 -> 0.184 ms, 1024x1024 x 8 with C, L and noise
+// 0.721 -> 0.257 ms (there the amplitude table saves the FP64 square root, the source as the first addend
+// and the noise's conversion by its bits two of nine FP64 operations: 0.290 -> 0.257). Bound by the FP64
+// pipe (73 % busy with 5 operations per element, 80 % with the 9 of before) and the latency of three
+// dependent reads (face numbers, face currents, sine table) at 32 warps per SM; 5 or 6 blocks per SM
+// (fewer registers), a thread per pair without the grid loop, the face numbers read an iteration
+// ahead and a branch around absent sources measured the same or slower.
 template <bool kCap, bool kNoise, int V>
 __global__ void __launch_bounds__(256, V == 1 ? 6 : 4) k_update_fast(StepArgs a, Tables t, double* __restrict__ q,
                                                                     const double* __restrict__ J) {
@@ -668,15 +692,11 @@ __global__ void __launch_bounds__(256, V == 1 ? 6 : 4) k_update_fast(StepArgs a,
       th.v[u] = fma(s, ic0, -qv.v[u]);
       if (non_finite(th.v[u])) *t.nonfinite = 1;
       const double sn = fast_sin(fma(2.0, th.v[u], -h0.v[u]), t.sincos);
-      double X;
-      if (kCap) X = fma(c1, h0.v[u], fma(c0, th.v[u], icq[u] * sn));
-      else X = fma(icq[u], sn, -th.v[u]);
-      if (kNoise) {
-        const double xi = philox_normal(a.seed, (uint64_t)(e + u), (uint64_t)next_step);
-        qn.v[u] = fma(amp, xi, -isq.v[u]) + X;
-      } else {
-        qn.v[u] = a.Isq.ptr ? X - isq.v[u] : X;
-      }
+      double X = fma(icq[u], sn, -isq.v[u]);
+      if (kCap) X = fma(c1, h0.v[u], fma(c0, th.v[u], X));
+      else X -= th.v[u];
+      if (kNoise) X = fma(amp, philox_normal(a.seed, (uint64_t)(e + u), (uint64_t)next_step), X);
+      qn.v[u] = X;
     }
     *reinterpret_cast<Vec*>(a.hout + e) = th;
     *reinterpret_cast<Vec*>(q + e) = qn;
@@ -2804,11 +2824,16 @@ bool pairs_fit(const StepArgs& a) {
   return a.W % 2 == 0 && a.w0 % 2 == 0 && a.wn % 2 == 0 && aligned(a.h[0]) && aligned(a.hout) && aligned(a.th_out);
 }
 
+using FaceKernel = void (*)(StepArgs, Tables, const double*, double*);
+FaceKernel face_rhs_kernel(int deg) {
+  return deg == 0 ? k_face_rhs<0> : deg <= 3 ? k_face_rhs<3> : deg == 4 ? k_face_rhs<4> : k_face_rhs<kEllMax>;
+}
+
 void launch_face_rhs(jja_plan* p, const StepArgs& a, cudaStream_t st) {
   const int64_t nf = (int64_t)p->Nf * a.wn;
   const double* q = p->xj;
   if (!p->t.face_deg || a.theta_s || a.f.stride_t || (int64_t)p->Nf * p->t.face_deg >= INT_MAX) {
-    launch(p->pdl, k_face_rhs, grid_for(nf, 256), 256, st, a, p->t, q, p->b);
+    launch(p->pdl, face_rhs_kernel(p->t.face_deg), grid_for(nf, 256), 256, st, a, p->t, q, p->b);
     return;
   }
   StepArgs f = a;
@@ -4331,7 +4356,7 @@ int jja_adjoint_flux(jja_plan* p, const double* usum, double* gf, void* stream) 
     const int64_t NfW = (int64_t)p->Nf * p->W;
     StepArgs s{};
     s.Nj = p->Nj; s.Nf = p->Nf; s.W = p->W; s.width = p->width; s.w0 = 0; s.wn = p->W; s.by_wn = fast_div(p->W); s.d_step = p->all.d_step;
-    k_face_rhs<<<grid_for(NfW, 256), 256, 0, st>>>(s, p->t, usum, p->b);
+    face_rhs_kernel(p->t.face_deg)<<<grid_for(NfW, 256), 256, 0, st>>>(s, p->t, usum, p->b);
     g_launches++;
     launch_face_solve(p, st);
     k_unpermute_scaled<<<grid_for(NfW, 256), 256, 0, st>>>(p->x, gf, p->perm, p->Nf, p->W, fast_div(p->W), -kTwoPi);

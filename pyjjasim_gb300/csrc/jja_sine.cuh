@@ -21,12 +21,14 @@
 // Even and odd modes see x_j + x_{N-j} and x_j - x_{N-j} (N = m + 1), which halves the products:
 // two contractions of length <= 64 for lines of up to 128 faces.
 //
-// Measured (GB300, per step, graph-replayed; the sweeps they replace -> these kernels): 128x128 x
-// 512 problems 1.157 -> 0.669 ms, 101x60 x 24 0.138 -> 0.058 ms; an adjoint run on 64x64 x 64
-// 121 -> 53 ms; 1024x1024 x 8 (8 strips) 2.30 -> 0.92 ms: 84 us per transform, 108 and 158 us for the
-// two passes over the chains (72 and 100 us of FP64 work), 45 us for the edges, 50 us for the
-// separators. A tile (128 columns of 127 faces) takes about 30k cycles: reading and splitting
-// 6k, twice the products 3.8k (3.5k of MMA issue at the multipliers' rate) and the joining 7k.
+// Measured (GB300, the face solve of a step; the sweeps they replace -> these kernels): 128x128 x
+// 512 problems 850 -> 195 us (70 us per transform, 56 us for the chains: 43 us of FP64 work), 101x60 x
+// 24 178 -> 31 us; an adjoint run on 64x64 x 64 121 -> 48 ms; 1024x1024 x 8 (8 strips) 1976 -> 510 us:
+// 77 us per transform, 108 and 159 us for the two passes over the chains (72 and 100 us of FP64 work),
+// 30 us for the edges, 44 us for the separators. A tile (128 columns of 127 faces) takes about 30k
+// cycles: reading and splitting 6k, twice the products 3.8k (3.5k of MMA issue at the multipliers' rate)
+// and the joining 7k. Overlapping the products with the joins (chunks of modes, two sets of accumulators) was
+// measured and gained nothing: at 16 warps the digit work itself waits on its own latencies.
 // What bounds it: the shifts and logic of splitting and joining (the ALU pipe runs half a warp
 // instruction per clock and scheduler), serialised with the products because one tile's digits and
 // accumulators fill the SM's shared memory and TMEM.
@@ -657,7 +659,8 @@ struct SineStrips {
 // u0 at the edges of the strips of one width: sums of es[mode] z over odd and even modes. A warp sums a
 // (point, strip) over the contiguous modes x problems when the problems divide its lanes or the
 // lanes divide the problems; else a block does, problems x slices of the modes. Grid: (points,
-// strips, tiles of the problems).
+// strips, tiles of the problems). The lanes' sums take no branch on the parity: with one, both sides'
+// FP64 instructions took the pipe (1024x1024 x 8: 44 -> 30 us).
 __global__ void __launch_bounds__(256) k_sine_edges(const double* __restrict__ z, const double* __restrict__ es, int modes,
                                                     int64_t off, int64_t s_strip, int64_t s_n, int64_t s_c, int strip0,
                                                     int strips, int n, int W, double* __restrict__ edge) {
@@ -681,14 +684,19 @@ __global__ void __launch_bounds__(256) k_sine_edges(const double* __restrict__ z
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        if ((k + u * per) & 1) even = fma(e[u], v[u], even);
+        if (u & 1) even = fma(e[u], v[u], even);
         else odd = fma(e[u], v[u], odd);
       }
     }
     for (; k < modes; k += per) {
       const double v = p[(int64_t)k * s_c], e = __ldg(es + k);
-      if (k & 1) even = fma(e, v, even);
+      if (per == 1 && (k & 1)) even = fma(e, v, even);
       else odd = fma(e, v, odd);
+    }
+    if (per > 1) {   // an even number: a lane's modes are all odd or all even, and both sums are one
+      const double sum = odd + even;
+      odd = k0 & 1 ? 0.0 : sum;
+      even = k0 & 1 ? sum : 0.0;
     }
     for (int o = W; o < 32; o <<= 1) {
       odd += __shfl_xor_sync(0xffffffffu, odd, o);
