@@ -17,8 +17,10 @@ Reported (one JSON line):
   adjoint     cost of gradients (checkpointed adjoint) against a forward pass on the disorder
               workload (64 x 64 arrays, W = 64, 5000 steps);
   plain_gpu   the same lattice, one problem per launch (W = 1);
-  roofline    the dominant stage (forward supernodal solve) against the FP64 pipe, with
-              its HBM figures beside it; stage times from CUDA events per stage;
+  roofline    the face solve (tensor-core sine transforms along one axis, tridiagonal solves along
+              the other) against HBM bandwidth, with its tensor-core rate beside it, and the
+              supernodal sweeps of the same batch against the FP64 pipe; stage times from CUDA
+              events per stage;
   cpu_baseline the CPU oracle (numpy/scipy restatement of the reference's loop) on a
               bounded sample of the same workload, timed on this host.
 ``--impl reference`` times the CPU oracle alone on the same workload (reference arm).
@@ -44,6 +46,7 @@ FRUST = 0.25
 DT = 0.05
 METRIC = "junction-steps/s (batched IV sweep, SquareArray(128,128) x 512, FP64)"
 PROFILE_JSON = os.path.join(ROOT, "profiles", "traffic_iv_sweep_128x128_w512.json")
+SOLVE_PROFILE_JSON = os.path.join(ROOT, "profiles", "traffic_face_solve_128x128_w512.json")
 
 
 def config(n_gpus):
@@ -809,35 +812,62 @@ def main():
             "gpu_launches": int(gpu_launches), "clocks": clocks,
             "plan_seconds": t_plan, "factor": fstats}
     if rank == 0:
-        # roofline of the dominant stage (forward supernodal solve; backward is its mirror)
-        nnzL = fstats["nnz_L"]
-        fwd_s = stages["forward"] / 1e3 / args.steps
-        fwd_flops = 2.0 * nnzL * W
-        fwd_bytes = 16.0 * Nf * W + 8.0 * fstats["f_values"]
+        # roofline of the face solve, and of the sweeps it replaces (the solver of non-uniform arrays)
         peaks = measured_peaks()
-        fp64 = fp64_peak_tflops(torch)
-        traffic = None
-        try:
-            with open(PROFILE_JSON) as fh:
-                traffic = json.load(fh).get("forward_sweep_dram_bytes_per_step")
-        except Exception:
-            traffic = None
         hbm_peak = peaks.get("hbm_gbs", 6800.0)
-        line["roofline"] = {
-            "kernel": "forward supernodal solve (k_subtree<fwd> for the bottom subtrees + k_fwd_level for the "
-                      "levels above, one step, all problem groups)",
-            "bound": "fp64", "achieved": fwd_flops / fwd_s / 1e12, "peak": fp64, "unit": "TFLOP/s",
-            "frac": (fwd_flops / fwd_s / 1e12) / fp64,
-            "peak_source": "measured in this run: cuBLAS DGEMM 4096^3 (FP64 has no entry in MEASURED_PEAKS.json)",
-            "traffic": traffic,
-            "algorithmic_flops_per_launch": fwd_flops, "algorithmic_bytes_per_launch": fwd_bytes,
-            "hbm": {"achieved": fwd_bytes / fwd_s / 1e9, "peak": hbm_peak, "unit": "GB/s",
-                    "frac": fwd_bytes / fwd_s / 1e9 / hbm_peak,
-                    "peak_source": "MEASURED_PEAKS.json hbm_gbs" if "hbm_gbs" in peaks else "fallback 6800 GB/s"},
-            "stage_ms_per_step": {k: v / args.steps for k, v in stages.items()},
-            "stage_share": stage_share}
-        # plain GPU path: one problem per launch. (a) The batched path's own solver (supernodal
-        # sweeps) at W = 1 in its fastest launch mode: the batching ratio. (b) The library's
+        hbm_source = "MEASURED_PEAKS.json hbm_gbs" if "hbm_gbs" in peaks else "fallback 6800 GB/s"
+        fp64 = fp64_peak_tflops(torch)
+
+        def profiled(path, key):
+            try:
+                with open(path) as fh:
+                    return json.load(fh).get(key)
+            except Exception:
+                return None
+
+        def sweeps(st, steps):
+            nnzL = fstats["nnz_L"]
+            fwd_s = st["forward"] / 1e3 / steps
+            fwd_flops = 2.0 * nnzL * W
+            fwd_bytes = 16.0 * Nf * W + 8.0 * fstats["f_values"]
+            return {"kernel": "forward supernodal solve (k_subtree<fwd> for the bottom subtrees + k_fwd_level for the "
+                              "levels above, one step, all problem groups)",
+                    "bound": "fp64", "achieved": fwd_flops / fwd_s / 1e12, "peak": fp64, "unit": "TFLOP/s",
+                    "frac": (fwd_flops / fwd_s / 1e12) / fp64,
+                    "peak_source": "measured in this run: cuBLAS DGEMM 4096^3 (FP64 has no entry in MEASURED_PEAKS.json)",
+                    "traffic": profiled(PROFILE_JSON, "forward_sweep_dram_bytes_per_step"),
+                    "algorithmic_flops_per_launch": fwd_flops, "algorithmic_bytes_per_launch": fwd_bytes,
+                    "hbm": {"achieved": fwd_bytes / fwd_s / 1e9, "peak": hbm_peak, "unit": "GB/s",
+                            "frac": fwd_bytes / fwd_s / 1e9 / hbm_peak, "peak_source": hbm_source},
+                    "stage_ms_per_step": {k: v / steps for k, v in st.items()}}
+
+        if sim.plan.sine:
+            sim_sw = GpuSimulation(prob, fast_poisson=False, **factor_opts(args))
+            sim_sw.run(64)
+            k_sw = min(args.steps, 50)
+            sweep_line = sweeps(sim_sw.run_timed(k_sw), k_sw)
+            del sim_sw
+            solve_s = (stages["forward"] + stages["backward"]) / 1e3 / args.steps
+            solve_bytes = 16.0 * Nf * W          # right-hand side in, solution out
+            # digit products executed: 2 transforms of (NY - 1) x W lines, odd and even half matrices of
+            # 64 x 64, 27 products of 9-bit digits
+            solve_flops = 2.0 * 2 * 27 * 64 * 64 * 2 * (NY - 1) * W
+            line["roofline"] = {
+                "kernel": "face solve (k_sine_lines, k_sine_tri, k_sine_lines, one step)",
+                "bound": "hbm", "achieved": solve_bytes / solve_s / 1e9, "peak": hbm_peak, "unit": "GB/s",
+                "frac": solve_bytes / solve_s / 1e9 / hbm_peak, "peak_source": hbm_source,
+                "traffic": profiled(SOLVE_PROFILE_JSON, "face_solve_dram_bytes_per_step"),
+                "algorithmic_bytes_per_launch": solve_bytes,
+                "limited_by": "the integer work of splitting and joining the digits (k_sine_lines) and the FP64 pipe "
+                              "(k_sine_tri), not by memory",
+                "tensor": {"achieved": solve_flops / solve_s / 1e12, "peak": peaks.get("bf16_tflops", 1900.0),
+                           "unit": "TFLOP/s (FP16 in, FP32 out, executed digit products)"},
+                "stage_ms_per_step": {k: v / args.steps for k, v in stages.items()},
+                "stage_share": stage_share, "sweeps": sweep_line}
+        else:
+            line["roofline"] = dict(sweeps(stages, args.steps), stage_share=stage_share)
+        # plain GPU path: one problem per launch. (a) Supernodal sweeps at W = 1 in their fastest launch
+        # mode: the batching ratio. (b) The library's
         # fastest W = 1 path, the sine-transform face solve this uniform square array allows.
         prob1 = make_problem(G, 1, [1.0])
         k1 = max(args.steps, 200)
@@ -858,7 +888,7 @@ def main():
         t_fp = fp_ms["default"] * k1 / 1e3
         fp = Nj * k1 / t_fp
         line["plain_gpu"] = {"value": plain, "unit": "junction-steps/s", "W": 1, "ms_per_step": t1 / k1 * 1e3,
-                             "solver": "supernodal sweeps (the batched path's solver)",
+                             "solver": "supernodal sweeps",
                              "ms_per_step_by_launch_mode": plain_ms, "batched_over_plain": value / world / plain,
                              "fast_poisson": {"value": fp, "ms_per_step": t_fp / k1 * 1e3,
                                               "solver": "sine transforms (uniform square array), the library's "

@@ -488,7 +488,8 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
     DevicePlan); ``fast_poisson``: solve with sine transforms when the face-space matrix allows it
     (fast_poisson_grid): True (radix-2 grids), False (the sweeps), or "auto": unless ``tuning`` asks for
     sweeps of some shape, whichever of the resident steps (resident_fits), the radix-2 or tensor-core
-    transforms, and the dense blocks (block_leaf) is fastest for the circuit and W."""
+    transforms, the dense blocks (block_leaf) and the dense top block (top_leaf) is fastest for the circuit
+    and W."""
     fp = sine = blocks = top = None
     matrices = face_matrix(circuit, dt)
     n_faces = circuit._Nf()

@@ -60,3 +60,24 @@ def test_face_sums_of_each_degree(lattice, W):
         sim.synchronize()
         out.append(sim.theta().clone())
     assert float((out[0] - out[1]).abs().max()) <= 1e-13
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,W,per_face", [(4, 4, 1, True), (16, 32, 1, False), (32, 8, 2, True), (64, 32, 3, True),
+                                              (64, 64, 8, False), (256, 64, 1, True), (32, 32, 9, True)])
+def test_face_sums_in_the_first_transform(nx, ny, W, per_face):
+    """Radix-2 plans form the face sums in their first transform, except in timed runs (and beyond 8 problems): the
+    same operations in the same order."""
+    import torch
+    c = SquareArray(nx, ny)
+    rng = np.random.default_rng(nx + W)
+    f = rng.uniform(-0.3, 0.3, (c._Nf(), W, 1)) if per_face else rng.uniform(-0.3, 0.3, (1, W, 1))
+    prob = TimeEvolutionProblem(c, time_step=0.05, time_step_count=40, external_flux=f,
+                                current_sources=0.4 * np.ones((c._Nj(), W, 1)))
+    a, b = (backend.GpuSimulation(prob, fast_poisson=True) for _ in range(2))
+    assert a.plan.fast_poisson
+    a.run(40)
+    a.synchronize()
+    b.run_timed(40)
+    b.synchronize()
+    assert torch.equal(a.theta(), b.theta())
