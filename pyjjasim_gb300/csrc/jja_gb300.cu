@@ -692,9 +692,9 @@ __global__ void __launch_bounds__(256, V == 1 ? 6 : 4) k_update_fast(StepArgs a,
       th.v[u] = fma(s, ic0, -qv.v[u]);
       if (non_finite(th.v[u])) *t.nonfinite = 1;
       const double sn = fast_sin(fma(2.0, th.v[u], -h0.v[u]), t.sincos);
-      double X = fma(icq[u], sn, -isq.v[u]);
-      if (kCap) X = fma(c1, h0.v[u], fma(c0, th.v[u], X));
-      else X -= th.v[u];
+      double X;
+      if (kCap) X = fma(c1, h0.v[u], fma(c0, th.v[u], fma(icq[u], sn, -isq.v[u])));
+      else X = fma(icq[u], sn, -th.v[u]) - isq.v[u];   // the general kernel's order, at no cost
       if (kNoise) X = fma(amp, philox_normal(a.seed, (uint64_t)(e + u), (uint64_t)next_step), X);
       qn.v[u] = X;
     }
