@@ -113,3 +113,24 @@ def test_trajectory_matches_sweeps_and_oracle(lattice, nx, ny, W, width):
     assert float(np.abs(th - th_s).max()) <= 1e-10 * scale
     assert float(np.abs(th - th_o).max()) <= 1e-9 * scale
     assert float(np.abs(I - I_o).max()) <= 1e-9
+
+
+@pytest.mark.gpu
+def test_too_many_blocks_keep_the_sweeps():
+    """More blocks than the limit (131 x 261 of one inverse): the plan solves by its sweeps, as without blocks."""
+    import torch
+    c = SquareArray(130, 130)
+    c.set_resistance(np.random.default_rng(0).lognormal(0.0, 0.2, c._Nj()))
+    A, K = P.face_matrix(c, 0.05)
+    factor, A, _ = P.get_factor(c, 0.05)
+    pl = P.DevicePlan(c, factor, A, 2, 0.05, 3, ((1.0, -1.0, 0.0), (1.0, -2.0, 1.0)), blocks=0)
+    assert pl.blocks is None
+    b = np.random.default_rng(1).standard_normal((c._Nf(), 2))
+    bd = torch.from_numpy(b).cuda()
+    xd = torch.empty_like(bd)
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    pl.solve(bd.data_ptr(), xd.data_ptr(), s.cuda_stream)
+    s.synchronize()
+    ref = scipy.sparse.linalg.spsolve(K.tocsc(), b)
+    assert np.abs(xd.cpu().numpy() - ref).max() <= 1e-11 * np.abs(ref).max()

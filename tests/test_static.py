@@ -95,6 +95,25 @@ def test_device_factorisation_solves_indefinite_systems(make, L):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,W", [(2, 2, 2), (3, 9, 1), (34, 35, 3), (130, 125, 2)])
+def test_device_factorisation_of_small_and_large_fronts(nx, ny, W):
+    """Fronts of one column, of a warp's 32 columns and more, and (130 x 125) too large for shared memory."""
+    from pyjjasim_gb300.static import get_static_plan
+    c = SquareArray(nx, ny)
+    c.set_inductance(0.1)
+    rng = np.random.default_rng(nx)
+    iq = 1.0 / rng.uniform(0.4, 1.5, (W, c.junction_count()))
+    b = rng.standard_normal((W, c.face_count()))
+    x, err = get_static_plan(c, W).solve(iq, b)
+    assert not err.any()
+    A = scipy.sparse.csr_matrix(c.get_cycle_matrix()).astype(float)
+    for w in range(W):
+        K = (A @ (scipy.sparse.csr_matrix(c._L()) + scipy.sparse.diags(iq[w])) @ A.T).tocsc()
+        ref = np.atleast_1d(scipy.sparse.linalg.spsolve(K, b[w]))
+        assert np.abs(x[w] - ref).max() <= 1e-9 * np.abs(ref).max()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("name", CASES)
 def test_device_newton_matches_reference(name):
     """From the reference's initial guess: same status, iteration count, target flags; residual
