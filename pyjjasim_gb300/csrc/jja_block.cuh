@@ -17,7 +17,7 @@
 // identity (jja_plan_set_blocks).
 //
 // Measured (GB300, us per step with the sweeps -> with these products): honeycomb 24x24 x 61 problems
-// 99 -> 25, triangular 64x48 with spread resistances x 96 240 -> 145, one such array 89 -> 33. A unit
+// 99 -> 24, triangular 64x48 with spread resistances x 96 240 -> 134, one such array 89 -> 33. A unit
 // (128 x 64 block, 64 problems) takes about 12k cycles on its SM: 1.5k reading and splitting the data,
 // 3.5k the products (the multipliers' rate), 7k joining the digits and adding to the result, while
 // the next block's 96 KB arrive. The joining (the ALU pipe) bounds launches of many units, the

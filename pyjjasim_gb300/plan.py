@@ -222,7 +222,8 @@ FAST_POISSON_MAX_W = 8
 FAST_POISSON_MAX_WORK = 1 << 18
 
 # Uniform square arrays otherwise (us per step: radix-2 transforms / tensor-core transforms (cut into
-# strips above 128 faces a side) / dense blocks):
+# strips above 128 faces a side) / dense blocks; the radix-2 steps take 1.6 us less since their first
+# transform forms the face sums):
 #   33x33    W = 16   - / 28 / 14      W = 64   - / 29 / 20       W = 256  - / 37 / 42
 #   64x64    W = 1   24 / 30 / 22      W = 16  37 / 32 / 28       W = 64  92 / 39 / 43
 #   101x60   W = 1    - / 40 / 22      W = 16   - / 38 / 30       W = 64   - / 51 / 54
