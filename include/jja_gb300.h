@@ -196,6 +196,10 @@ int jja_plan_set_sine_solver(jja_plan* p, int mx, int my, const int32_t* grid_fa
  * history buffers keep their places in jja_state over such a call (no rotation). */
 int jja_plan_set_resident(jja_plan* p, const jja_factor* f);
 
+/* 1 when jja_plan_set_resident takes circuits of nf faces and nj junctions at this stencil width (3 to
+ * 5; the phase history lies in shared memory beside the inverse), else 0. */
+int jja_resident_fits(int nf, int nj, int width);
+
 /* Face-space solves by products with dense blocks on the tensor cores (error-free digit products,
  * FP64 results) instead of the triangular sweeps: leaf_faces = 0, the whole inverse (one launch per
  * solve); else the inverses of the largest subtrees of at most leaf_faces faces of the factor's elimination tree,

@@ -106,6 +106,7 @@ SIGNATURES = {
     "jja_plan_device_bytes": (c_int64, [c_void_p]),
     "jja_plan_set_fast_poisson": (c_int, [c_void_p, c_int, c_int, P_i32, c_double]),
     "jja_plan_set_sine_solver": (c_int, [c_void_p, c_int, c_int, P_i32, c_double]),
+    "jja_resident_fits": (c_int, [c_int, c_int, c_int]),
     "jja_plan_set_resident": (c_int, [c_void_p, c_void_p]),
     "jja_plan_set_blocks": (c_int, [c_void_p, c_void_p, c_int]),
     "jja_plan_set_top_block": (c_int, [c_void_p, c_void_p, c_int]),

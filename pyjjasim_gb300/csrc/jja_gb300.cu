@@ -4102,15 +4102,19 @@ int jja_plan_set_top_block(jja_plan* p, const jja_factor* fac, int leaf_faces) {
   });
 }
 
+int jja_resident_fits(int nf, int nj, int width) {
+  return nf >= 1 && nf <= kResMaxFaces && nj >= 1 && nj <= kResMaxJunctions && width >= 3 && width <= 5 &&
+         resident_smem_bytes(nf, nj, width - 1) <= (size_t)227 * 1024;
+}
+
 int jja_plan_set_resident(jja_plan* p, const jja_factor* fac) {
   return guarded([&] {
     if (!p || !fac) throw Error(JJA_ERR_ARG, "jja_plan_set_resident: null argument");
     const jja::Factor& F = *fac->f;
-    const int n = p->Nf, nh = p->width - 1;
+    const int n = p->Nf;
     if (F.n != n) throw Error(JJA_ERR_ARG, "jja_plan_set_resident: factor order != Nf");
     if (p->dst) throw Error(JJA_ERR_ARG, "jja_plan_set_resident: the plan solves by sine transforms");
-    const size_t smem = n <= kResMaxFaces ? resident_smem_bytes(n, p->Nj, nh) : SIZE_MAX;
-    if (p->Nj > kResMaxJunctions || smem > (size_t)227 * 1024)
+    if (!jja_resident_fits(n, p->Nj, p->width))
       throw Error(JJA_ERR_ARG, "jja_plan_set_resident: the circuit does not fit one SM");
     // the inverse, in the factor's face order, column by column in fixed point
     std::vector<double> inv((size_t)n * n, 0.0);   // row-major right-hand sides

@@ -259,9 +259,12 @@ RESIDENT_MAX_JUNCTIONS = 512
 RESIDENT_MAX_W = 512
 
 
-def resident_fits(circuit, W):
-    """Whether the default plan steps W problems of this circuit in one launch per call."""
-    return circuit._Nf() <= RESIDENT_MAX_FACES and circuit._Nj() <= RESIDENT_MAX_JUNCTIONS and W <= RESIDENT_MAX_W
+def resident_fits(circuit, W, stencil_width=3):
+    """Whether the default plan steps W problems of this circuit in one launch per call. The phase history is
+    in shared memory too: with 160 faces and width 5 at most 360 junctions fit, with 158 faces 468."""
+    n_faces, n_junctions = circuit._Nf(), circuit._Nj()
+    return n_faces <= RESIDENT_MAX_FACES and n_junctions <= RESIDENT_MAX_JUNCTIONS and W <= RESIDENT_MAX_W and \
+        bool(N.lib().jja_resident_fits(n_faces, n_junctions, stencil_width))
 
 
 # Other circuits solve by products with dense blocks on the tensor cores: the whole inverse (leaf 0),
@@ -495,7 +498,7 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
     matrices = face_matrix(circuit, dt)
     n_faces = circuit._Nf()
     auto = fast_poisson == "auto" and untuned(tuning)
-    resident = auto and resident_fits(circuit, W)
+    resident = auto and resident_fits(circuit, W, stencil_width)
     if fast_poisson is True or (auto and not resident and radix2_fits(n_faces, W)) or \
             (fast_poisson == "auto" and not auto and W <= FAST_POISSON_MAX_W and W * n_faces <= FAST_POISSON_MAX_WORK):
         fp = fast_poisson_grid(circuit, matrices[1])

@@ -92,3 +92,29 @@ def test_non_finite_phases_are_reported():
     with pytest.raises(N.JJAError):
         sim.synchronize()
     sim.synchronize()   # reported once
+
+
+# faces, junctions, width, fits: both sides of the 227 KB of shared memory, which the history shares
+LIMITS = [(41, 5, 3, True), (41, 5, 4, True), (41, 5, 5, False), (81, 3, 5, False), (54, 4, 5, True), (80, 3, 5, True)]
+
+
+@pytest.mark.parametrize("nx,ny,width,fits", LIMITS)
+def test_rule_counts_the_history(nx, ny, width, fits):
+    for c in (SquareArray(nx, ny), SquareArray(ny, nx)):
+        assert P.resident_fits(c, 1, width) == fits
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,width,fits", LIMITS)
+def test_default_plan_at_the_limit(nx, ny, width, fits):
+    c = SquareArray(nx, ny)
+    c.set_capacitance(0.6)
+    Is = c.current_base(0.0)[:, None, None] * np.linspace(0.4, 1.4, 2)[None, :, None]
+    prob = TimeEvolutionProblem(c, time_step=0.05, time_step_count=30, current_sources=Is, external_flux=0.13,
+                                store_time_steps=[10, 29], stencil_width=width)
+    m = prob.store_time_steps
+    sim = backend.GpuSimulation(prob)
+    assert sim.plan.resident == fits
+    th, _ = backend.time_evolution_core(prob, m, m, sim=sim)
+    th_o, _ = rcsj_oracle.evolve(prob, m, m)
+    assert float(np.abs(th - th_o).max()) <= 1e-9 * max(1.0, float(np.abs(th_o).max()))
