@@ -3753,7 +3753,8 @@ int jja_plan_set_fast_poisson(jja_plan* p, int mx, int my, const int32_t* grid_f
     if (!p || !grid_face || mx < 1 || my < 1) throw Error(JJA_ERR_ARG, "jja_plan_set_fast_poisson: bad arguments");
     if ((int64_t)mx * my != p->Nf) throw Error(JJA_ERR_ARG, "jja_plan_set_fast_poisson: mx * my != Nf");
     if (!(kappa > 0.0)) throw Error(JJA_ERR_ARG, "jja_plan_set_fast_poisson: kappa must be positive");
-    if (p->dst > 1) throw Error(JJA_ERR_ARG, "jja_plan_set_fast_poisson: the plan already has another solver");
+    if (p->dst > 1 || p->res.inv)
+      throw Error(JJA_ERR_ARG, "jja_plan_set_fast_poisson: the plan already has another solver");
     auto log2_of = [](int n) {   // log2(2 n) for n a power of two (n = m + 1), else -1
       if (n < 2 || (n & (n - 1))) return -1;
       int l = 1;
@@ -3820,7 +3821,9 @@ int jja_plan_set_sine_solver(jja_plan* p, int mx, int my, const int32_t* grid_fa
       throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: kappa must be positive and finite");
     if ((int64_t)std::max(mx, my) > kSineMaxSide)
       throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: a side of more than " + std::to_string(kSineMaxSide) + " faces");
-    if (p->dst) throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: the plan already solves by sine transforms");
+    // (the resident steps keep the factor's face order, which this solver replaces in the plan's tables)
+    if (p->dst || p->res.inv)
+      throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: the plan already has another solver");
     const int Nf = p->Nf, W = p->W;
     // the tables again with the faces in grid order: cell iy * mx + ix
     std::vector<int32_t> cell_of(Nf, -1);   // the factor's face -> grid cell
@@ -4113,7 +4116,7 @@ int jja_plan_set_resident(jja_plan* p, const jja_factor* fac) {
     const jja::Factor& F = *fac->f;
     const int n = p->Nf;
     if (F.n != n) throw Error(JJA_ERR_ARG, "jja_plan_set_resident: factor order != Nf");
-    if (p->dst) throw Error(JJA_ERR_ARG, "jja_plan_set_resident: the plan solves by sine transforms");
+    if (p->dst || p->res.inv) throw Error(JJA_ERR_ARG, "jja_plan_set_resident: the plan already has another solver");
     if (!jja_resident_fits(n, p->Nj, p->width))
       throw Error(JJA_ERR_ARG, "jja_plan_set_resident: the circuit does not fit one SM");
     // the inverse, in the factor's face order, column by column in fixed point
