@@ -210,7 +210,8 @@ int jja_plan_set_blocks(jja_plan* p, const jja_factor* f, int leaf_faces);
 /* Triangular sweeps below, one product above: the faces above the largest subtrees of at most leaf_faces
  * faces are solved by the inverse of their Schur complement (per tree of the forest) on the tensor
  * cores between the two sweeps over the subtrees. For large circuits with few problems, whose upper tree
- * levels are short dependent launches. Level schedule only; jja_solve_static keeps the whole sweeps. */
+ * levels are short dependent launches. Level schedule only; leaf_faces at least the subtrees that the
+ * plan's sweeps fuse (jja_solve_tuning.subtree_rows). jja_solve_static keeps the whole sweeps. */
 int jja_plan_set_top_block(jja_plan* p, const jja_factor* f, int leaf_faces);
 /* Synchronises the device, then reads and clears the plan's device error flags: *flow_timeouts
  * = 1 if a wait of a dataflow sweep ran out of its bound since the last call (the results of

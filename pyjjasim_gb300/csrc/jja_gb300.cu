@@ -2179,6 +2179,9 @@ Schedule build_schedule(const jja::Factor& F, int W, const jja_solve_tuning& tu,
     }
   }
   std::vector<std::vector<int>> by_level(S.n_levels);
+  for (int s = 0; skip && s < F.ns; ++s)   // a fused subtree is solved whole
+    if (inside[s] && (*skip)[s])
+      throw Error(JJA_ERR_ARG, "a supernode to be left out of the sweeps lies inside a subtree sweep");
   for (int s = 0; s < F.ns; ++s)
     if (!inside[s] && !(skip && (*skip)[s])) by_level[level[s]].push_back(s);
   auto pack = [](int s, int r0, int r1, int w0, bool partial, int c_lo, int c_hi) {
@@ -4093,12 +4096,12 @@ int jja_plan_set_top_block(jja_plan* p, const jja_factor* fac, int leaf_faces) {
     if (p->dst || p->res.inv || p->flow || p->coop)
       throw Error(JJA_ERR_ARG, "jja_plan_set_top_block: the plan already has another solver or schedule");
     const BlockSetup B(F, leaf_faces, true);
-    make_blocks(p, F, B);
     // the sweeps' work items without the separators
     std::vector<char> top(F.ns);
     for (int s = 0; s < F.ns; ++s) top[s] = B.leaf_of[s] < 0;
     const Schedule S = build_schedule(F, p->W, p->tuning, 0, p->W, &top);
     if (S.n_levels != p->n_levels) throw Error(JJA_ERR_INTERNAL, "leaf schedule differs in levels");
+    make_blocks(p, F, B);
     set_group_items(p, p->leaves, S, 0, p->W);
     one_chain(p);
     p->dst = 4;

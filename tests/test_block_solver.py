@@ -134,3 +134,26 @@ def test_too_many_blocks_keep_the_sweeps():
     s.synchronize()
     ref = scipy.sparse.linalg.spsolve(K.tocsc(), b)
     assert np.abs(xd.cpu().numpy() - ref).max() <= 1e-11 * np.abs(ref).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("top,taken", [(8, False), (16, False), (64, True)])
+def test_top_block_does_not_cut_a_fused_subtree(top, taken):
+    """Supernodes that the sweeps solve inside a fused subtree (up to 32 rows) cannot go to the product."""
+    import torch
+    c = SquareArray(60, 55)
+    c.set_resistance(np.random.default_rng(0).lognormal(0.0, 0.4, c._Nj()))
+    W, tuning = 64, dict(subtree_rows=32)
+    factor, A, _ = P.get_factor(c, 0.05)
+    assert factor.schedule_stats(W, tuning)["n_subtrees"] > 0
+    pl = P.DevicePlan(c, factor, A, W, 0.05, 3, ((1.0, -1.0, 0.0), (1.0, -2.0, 1.0)), tuning=tuning, top=top)
+    assert (pl.top is not None) == taken
+    b = np.random.default_rng(1).standard_normal((c._Nf(), W))
+    bd = torch.from_numpy(b).cuda()
+    xd = torch.empty_like(bd)
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    pl.solve(bd.data_ptr(), xd.data_ptr(), s.cuda_stream)
+    s.synchronize()
+    ref = scipy.sparse.linalg.spsolve(P.face_matrix(c, 0.05)[1].tocsc(), b)
+    assert np.abs(xd.cpu().numpy() - ref).max() <= 1e-11 * np.abs(ref).max()
