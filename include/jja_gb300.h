@@ -28,7 +28,8 @@ typedef enum {
   JJA_ERR_NOT_SPD = 2,    /* face-space matrix is not positive definite */
   JJA_ERR_CUDA = 3,       /* a CUDA runtime call failed */
   JJA_ERR_NONFINITE = 4,  /* a time step produced a NaN or +-inf phase (reported by jja_plan_check) */
-  JJA_ERR_INTERNAL = 5
+  JJA_ERR_INTERNAL = 5,
+  JJA_ERR_UNFIT = 6       /* a solver does not fit the circuit (jja_plan_set_*); the plan keeps its sweeps */
 } jja_status;
 
 typedef struct jja_factor jja_factor;
@@ -181,6 +182,9 @@ int64_t jja_plan_device_bytes(const jja_plan* p);
  * two up to 1024. The caller checks that K has that form. jja_solve_static keeps the sweeps. */
 int jja_plan_set_fast_poisson(jja_plan* p, int mx, int my, const int32_t* grid_face, double kappa);
 
+/* The setters of a solver below leave the plan as it was, with no device memory of theirs, when they fail;
+ * JJA_ERR_UNFIT: this circuit is too large for the solver (or its tree does not match the sweeps'). */
+
 /* The same solve with the sine transforms as tensor-core contractions (error-free digit products, FP64
  * results) along one axis of the grid and tridiagonal solves along the other: K = kappa (4 I - adjacency)
  * on an mx x my grid of faces of any size up to 4096 a side (grids longer than 128 faces both ways are cut
@@ -213,6 +217,11 @@ int jja_plan_set_blocks(jja_plan* p, const jja_factor* f, int leaf_faces);
  * levels are short dependent launches. Level schedule only; leaf_faces at least the subtrees that the
  * plan's sweeps fuse (jja_solve_tuning.subtree_rows). jja_solve_static keeps the whole sweeps. */
 int jja_plan_set_top_block(jja_plan* p, const jja_factor* f, int leaf_faces);
+
+/* For tests: device allocations of the plan beyond `bytes` more fail as they do when memory runs out
+ * (negative: no limit). Nothing is allocated for it. */
+int jja_plan_test_alloc_limit(jja_plan* p, int64_t bytes);
+
 /* Synchronises the device, then reads and clears the plan's device error flags: *flow_timeouts
  * = 1 if a wait of a dataflow sweep ran out of its bound since the last call (the results of
  * those steps are invalid), else 0. Returns JJA_ERR_NONFINITE when a time step of jja_run /

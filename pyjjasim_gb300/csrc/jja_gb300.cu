@@ -2181,7 +2181,7 @@ Schedule build_schedule(const jja::Factor& F, int W, const jja_solve_tuning& tu,
   std::vector<std::vector<int>> by_level(S.n_levels);
   for (int s = 0; skip && s < F.ns; ++s)   // a fused subtree is solved whole
     if (inside[s] && (*skip)[s])
-      throw Error(JJA_ERR_ARG, "a supernode to be left out of the sweeps lies inside a subtree sweep");
+      throw Error(JJA_ERR_UNFIT, "a supernode to be left out of the sweeps lies inside a subtree sweep");
   for (int s = 0; s < F.ns; ++s)
     if (!inside[s] && !(skip && (*skip)[s])) by_level[level[s]].push_back(s);
   auto pack = [](int s, int r0, int r1, int w0, bool partial, int c_lo, int c_hi) {
@@ -2541,8 +2541,15 @@ struct jja_plan {
     if (res_slots) cudaFree(res_slots);
     for (void* p : allocs) cudaFree(p);
   }
+  int64_t alloc_left = -1;               // bytes that may still be allocated (jja_plan_test_alloc_limit); < 0: any
+  void count_alloc(size_t n) {
+    if (alloc_left < 0) return;
+    if ((int64_t)n > alloc_left) throw Error(JJA_ERR_CUDA, "cudaMalloc: out of memory (limit set for a test)");
+    alloc_left -= (int64_t)n;
+  }
   template <class T>
   T* up(const T* h, size_t n) {
+    count_alloc(n * sizeof(T));
     T* d = upload(h, n, bytes);
     allocs.push_back(d);
     return d;
@@ -3057,6 +3064,30 @@ void run_resident(jja_plan* p, jja_state* s, int nsteps, const int64_t* th_slot,
   }
 }
 
+// A solver being set: unless kept, the plan gets its tables back and the memory allocated since is freed.
+struct SolverSetup {
+  jja_plan* p;
+  const size_t n_allocs;
+  const int64_t bytes;
+  const Tables t;
+  int32_t *const perm, *const perm_factor;
+  bool keep = false;
+  explicit SolverSetup(jja_plan* plan)
+      : p(plan), n_allocs(plan->allocs.size()), bytes(plan->bytes), t(plan->t), perm(plan->perm),
+        perm_factor(plan->perm_factor) {}
+  ~SolverSetup() {
+    if (keep) return;
+    cudaDeviceSynchronize();   // setup kernels may still use it
+    for (size_t i = n_allocs; i < p->allocs.size(); ++i) cudaFree(p->allocs[i]);
+    p->allocs.resize(n_allocs);
+    p->bytes = bytes;
+    p->t = t;
+    p->perm = perm;
+    p->perm_factor = perm_factor;
+    p->sine.clear();
+  }
+};
+
 // a plan whose solver changed: its step as one chain, no graphs that bake in the sweeps
 void one_chain(jja_plan* p) {
   for (Group& g : p->groups) {
@@ -3113,6 +3144,10 @@ struct BlockSetup {
   // blocks of a rows x cols matrix at `base` of the store with the given strides
   void add_blocks(int launch, int from, int64_t base, int64_t s_r, int64_t s_c, int out_off, int rows, int in_off,
                   int cols) {
+    const int64_t more = ((int64_t)rows + kBlockRows - 1) / kBlockRows * ((cols + kBlockCols - 1) / kBlockCols);
+    if (n_blocks + more > kBlocksMax)   // before they are listed
+      throw Error(JJA_ERR_UNFIT, std::to_string(n_blocks + more) + " blocks of the matrix or more, above " +
+                                     std::to_string(kBlocksMax));
     for (int c = 0; c < cols; c += kBlockCols)
       for (int r = 0; r < rows; r += kBlockRows) {
         const int nr = std::min(kBlockRows, rows - r), nc = std::min(kBlockCols, cols - c);
@@ -3260,9 +3295,6 @@ struct BlockSetup {
 // computes the blocks of B on the device from the plan's factor and gives them to the plan
 void make_blocks(jja_plan* p, const jja::Factor& F, const BlockSetup& B) {
   const int n = p->Nf, ns = F.ns;
-  if (B.n_blocks > kBlocksMax)
-    throw Error(JJA_ERR_ARG, std::to_string(B.n_blocks) + " blocks of the matrix, more than " +
-                                 std::to_string(kBlocksMax));
   // device scratch of the setup
   struct Scratch {
     std::vector<void*> mem;
@@ -3274,6 +3306,7 @@ void make_blocks(jja_plan* p, const jja::Factor& F, const BlockSetup& B) {
   } tmp;
   int64_t ignored = 0;
   auto scratch = [&](auto* h, size_t count) {
+    p->count_alloc(count * sizeof(*h));
     auto* d = upload(h, count, ignored);
     tmp.mem.push_back((void*)d);
     return d;
@@ -3823,11 +3856,12 @@ int jja_plan_set_sine_solver(jja_plan* p, int mx, int my, const int32_t* grid_fa
     if (!(kappa > 0.0) || !std::isfinite(kappa))
       throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: kappa must be positive and finite");
     if ((int64_t)std::max(mx, my) > kSineMaxSide)
-      throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: a side of more than " + std::to_string(kSineMaxSide) + " faces");
+      throw Error(JJA_ERR_UNFIT, "jja_plan_set_sine_solver: a side of more than " + std::to_string(kSineMaxSide) + " faces");
     // (the resident steps keep the factor's face order, which this solver replaces in the plan's tables)
     if (p->dst || p->res.inv)
       throw Error(JJA_ERR_ARG, "jja_plan_set_sine_solver: the plan already has another solver");
     const int Nf = p->Nf, W = p->W;
+    SolverSetup setup(p);
     // the tables again with the faces in grid order: cell iy * mx + ix
     std::vector<int32_t> cell_of(Nf, -1);   // the factor's face -> grid cell
     for (int c = 0; c < Nf; ++c) {
@@ -4074,6 +4108,7 @@ int jja_plan_set_sine_solver(jja_plan* p, int mx, int my, const int32_t* grid_fa
     p->strips = S;
     one_chain(p);
     p->dst = 2;
+    setup.keep = true;
   });
 }
 
@@ -4082,9 +4117,11 @@ int jja_plan_set_blocks(jja_plan* p, const jja_factor* fac, int leaf_faces) {
     if (!p || !fac || leaf_faces < 0) throw Error(JJA_ERR_ARG, "jja_plan_set_blocks: bad arguments");
     if (fac->f->n != p->Nf) throw Error(JJA_ERR_ARG, "jja_plan_set_blocks: factor order != Nf");
     if (p->dst || p->res.inv) throw Error(JJA_ERR_ARG, "jja_plan_set_blocks: the plan already has another solver");
+    SolverSetup setup(p);
     make_blocks(p, *fac->f, BlockSetup(*fac->f, leaf_faces));
     one_chain(p);
     p->dst = 3;
+    setup.keep = true;
   });
 }
 
@@ -4095,6 +4132,7 @@ int jja_plan_set_top_block(jja_plan* p, const jja_factor* fac, int leaf_faces) {
     if (F.n != p->Nf) throw Error(JJA_ERR_ARG, "jja_plan_set_top_block: factor order != Nf");
     if (p->dst || p->res.inv || p->flow || p->coop)
       throw Error(JJA_ERR_ARG, "jja_plan_set_top_block: the plan already has another solver or schedule");
+    SolverSetup setup(p);
     const BlockSetup B(F, leaf_faces, true);
     // the sweeps' work items without the separators
     std::vector<char> top(F.ns);
@@ -4105,6 +4143,7 @@ int jja_plan_set_top_block(jja_plan* p, const jja_factor* fac, int leaf_faces) {
     set_group_items(p, p->leaves, S, 0, p->W);
     one_chain(p);
     p->dst = 4;
+    setup.keep = true;
   });
 }
 
@@ -4121,7 +4160,8 @@ int jja_plan_set_resident(jja_plan* p, const jja_factor* fac) {
     if (F.n != n) throw Error(JJA_ERR_ARG, "jja_plan_set_resident: factor order != Nf");
     if (p->dst || p->res.inv) throw Error(JJA_ERR_ARG, "jja_plan_set_resident: the plan already has another solver");
     if (!jja_resident_fits(n, p->Nj, p->width))
-      throw Error(JJA_ERR_ARG, "jja_plan_set_resident: the circuit does not fit one SM");
+      throw Error(JJA_ERR_UNFIT, "jja_plan_set_resident: the circuit does not fit one SM");
+    SolverSetup setup(p);
     // the inverse, in the factor's face order, column by column in fixed point
     std::vector<double> inv((size_t)n * n, 0.0);   // row-major right-hand sides
     for (int i = 0; i < n; ++i) inv[(size_t)i * n + i] = 1.0;
@@ -4145,6 +4185,14 @@ int jja_plan_set_resident(jja_plan* p, const jja_factor* fac) {
     g.n = n;
     g.nj = p->Nj;
     p->res = g;
+    setup.keep = true;
+  });
+}
+
+int jja_plan_test_alloc_limit(jja_plan* p, int64_t bytes) {
+  return guarded([&] {
+    if (!p) throw Error(JJA_ERR_ARG, "jja_plan_test_alloc_limit: null plan");
+    p->alloc_left = bytes;
   });
 }
 

@@ -364,26 +364,26 @@ class DevicePlan:
             self._keep["grid"] = grid
             N.check(N.lib().jja_plan_set_fast_poisson(h, int(mx), int(my), N.ptr(grid, ctypes.c_int32), float(kappa)))
             self.fast_poisson = True
-        self.sine = False
-        if sine is not None:
-            mx, my, grid, kappa = sine
-            self._keep["grid"] = grid
-            N.check(N.lib().jja_plan_set_sine_solver(h, int(mx), int(my), N.ptr(grid, ctypes.c_int32), float(kappa)))
-            self.sine = True
-        self.resident = False
-        if resident:
-            N.check(N.lib().jja_plan_set_resident(h, factor.handle))
-            self.resident = True
+        # a solver that is too large for the circuit, or for the memory left, leaves the plan with its sweeps
+        self.sine = self.resident = False
         self.blocks = self.top = None
-        try:     # a tree whose blocks are too many (or too large for the memory left) keeps the sweeps
-            if blocks is not None:
+        try:
+            if sine is not None:
+                mx, my, grid, kappa = sine
+                self._keep["grid"] = grid
+                N.check(N.lib().jja_plan_set_sine_solver(h, int(mx), int(my), N.ptr(grid, ctypes.c_int32), float(kappa)))
+                self.sine = True
+            elif resident:
+                N.check(N.lib().jja_plan_set_resident(h, factor.handle))
+                self.resident = True
+            elif blocks is not None:
                 N.check(N.lib().jja_plan_set_blocks(h, factor.handle, int(blocks)))
                 self.blocks = blocks
             elif top is not None:
                 N.check(N.lib().jja_plan_set_top_block(h, factor.handle, int(top)))
                 self.top = top
         except N.JJAError as e:
-            if e.code != 1 and "out of memory" not in str(e):
+            if e.code != N.ERR_UNFIT and "out of memory" not in str(e):
                 raise
         self.device_bytes = N.lib().jja_plan_device_bytes(h)
 
