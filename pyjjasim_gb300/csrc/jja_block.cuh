@@ -14,7 +14,7 @@
 //     launch 2: x_s = S^-1 b_s
 //     launch 3: x_l -= G_l x_s.
 // The blocks come from the plan's own factor by sweeps over parts of its tree with columns of the
-// identity (jja_plan_set_blocks).
+// identity (jja_plan_set_blocks). Each row of a block has its own scale.
 //
 // Measured (GB300, us per step with the sweeps -> with these products): honeycomb 24x24 x 61 problems
 // 99 -> 24, triangular 64x48 with spread resistances x 96 240 -> 134, one such array 89 -> 33. A unit
@@ -43,7 +43,7 @@ struct BlockList {
   const int32_t* in_rows = nullptr;
   const int32_t* out_rows = nullptr;
   const unsigned char* mats = nullptr;   // per block: digit, 8-column group, row, column
-  const int* e_mat = nullptr;            // per block: |entry| < 2^e
+  const int* e_row = nullptr;            // per block and row of it: |entry| < 2^e
   int n = 0;
 };
 
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_block_apply(BlockList L, d
     const int row = tid & (kBlockRows - 1);
     const bool live = row < now.out_cnt;
     double* dst = (now.from == 1 ? b : x) + (live ? (int64_t)__ldg(L.out_rows + now.out_off + row) * W : 0) + w_lo;
-    const int e_mat = __ldg(L.e_mat + now.mat);
+    const int e_row = __ldg(L.e_row + now.mat * kBlockRows + row);
     const uint32_t lane_base = tmem + ((uint32_t)((tid >> 5) & 3) << 21);
 #pragma unroll 1
     for (int blk = 0; blk < wp / 16; ++blk) {
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_block_apply(BlockList L, d
         if (live && n0 + o < live_w) {
           const int emax = colexp[n0 + o];
           atomicAdd(dst + n0 + o, emax == 0x7ff ? __longlong_as_double((long long)kNaNBits)
-                                                : double_of_fixed(R, emax - 1022 - 1 + e_mat));
+                                                : double_of_fixed(R, emax - 1022 - 1 + e_row));
         }
       }
     }
@@ -246,7 +246,34 @@ struct BlockSource {
   int rows, cols;
 };
 
-// rows of 64 solved columns into the store: dst + i s_i + j for list rows i, columns j < cnt
+// The listed rows (null: all n) of E - K (x + dx), E the columns c0 .. c0 + 63 of the identity as in
+// k_unit_columns (pos null: zero), in twice the working precision (exact products, two-sums): residuals for
+// refining the blocks, and couplings. K by rows in the factor's order.
+struct MatrixRows {
+  const int64_t* ptr = nullptr;
+  const int32_t* idx = nullptr;
+  const double* val = nullptr;
+};
+__global__ void __launch_bounds__(256) k_residual(MatrixRows K, const int32_t* __restrict__ rows,
+                                                  const int32_t* __restrict__ pos, int n, int c0,
+                                                  const double* __restrict__ x, const double* __restrict__ dx,
+                                                  double* __restrict__ out) {
+  const int64_t total = (int64_t)n * kBlockCols;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
+    const int i = (int)(e / kBlockCols), j = (int)(e % kBlockCols), r = rows ? rows[i] : i;
+    double hi = pos && pos[i] == c0 + j ? 1.0 : 0.0, lo = 0.0;
+    for (int64_t k = K.ptr[r]; k < K.ptr[r + 1]; ++k) {
+      const double a = -K.val[k], v = x[(int64_t)K.idx[k] * kBlockCols + j];
+      const double p = a * v, s = hi + p, t = s - hi;
+      lo += ((hi - (s - t)) + (p - t)) + fma(a, v, -p);
+      if (dx) lo = fma(a, dx[(int64_t)K.idx[k] * kBlockCols + j], lo);
+      hi = s;
+    }
+    out[(int64_t)r * kBlockCols + j] = hi + lo;
+  }
+}
+
+// rows of 64 solved columns (x + dx, dx may be null) into the store: dst + i s_i + j for list rows i, columns j < cnt
 struct StoreRows {
   int64_t dst;       // of the list's first row, column c0
   int64_t s_i;       // between rows; columns are s_j apart
@@ -254,44 +281,49 @@ struct StoreRows {
   int first, count;  // rows of the list
   int cols;          // columns in range (cnt - c0 <= 64)
 };
-__global__ void k_store_rows(const double* __restrict__ x, const int32_t* __restrict__ rows,
-                             const StoreRows* __restrict__ jobs, double* __restrict__ store) {
+__global__ void k_store_rows(const double* __restrict__ x, const double* __restrict__ dx,
+                             const int32_t* __restrict__ rows, const StoreRows* __restrict__ jobs,
+                             double* __restrict__ store) {
   const StoreRows J = jobs[blockIdx.x];
   for (int i = threadIdx.x; i < J.count * kBlockCols; i += blockDim.x) {
     const int r = i / kBlockCols, j = i % kBlockCols;
-    if (j < J.cols) store[J.dst + r * J.s_i + j * J.s_j] = x[(int64_t)rows[J.first + r] * kBlockCols + j];
+    const int64_t at = (int64_t)rows[J.first + r] * kBlockCols + j;
+    if (j < J.cols) store[J.dst + r * J.s_i + j * J.s_j] = dx ? x[at] + dx[at] : x[at];
   }
 }
 
-// digits of the blocks, each scaled by its own largest magnitude; one thread block per block
+// digits of the blocks, each row scaled by its own largest magnitude; one thread block per block, a warp
+// per row. (One scale for a block's 128 rows held the rows of small entries to fewer bits: with resistances
+// of a lognormal spread of 3 the phases moved 15 times further from the exact ones.)
 __global__ void __launch_bounds__(256) k_block_digits(const double* __restrict__ store,
                                                       const BlockSource* __restrict__ src,
-                                                      unsigned char* __restrict__ mats, int* __restrict__ e_mat) {
-  __shared__ uint32_t wtop[8];
+                                                      unsigned char* __restrict__ mats, int* __restrict__ e_row) {
   const BlockSource B = src[blockIdx.x];
-  auto entry = [&](int i) {
-    const int r = i / kBlockCols, j = i % kBlockCols;
-    return r < B.rows && j < B.cols ? store[B.base + r * B.s_r + j * B.s_c] : 0.0;
-  };
-  uint32_t top = 0;
-  for (int i = threadIdx.x; i < kBlockRows * kBlockCols; i += blockDim.x)
-    top = max(top, (uint32_t)__double2hiint(entry(i)) * 2u);
-  top = __reduce_max_sync(0xffffffffu, top);
-  if ((threadIdx.x & 31) == 0) wtop[threadIdx.x >> 5] = top;
-  __syncthreads();
-  for (int k = 0; k < 8; ++k) top = max(top, wtop[k]);
-  const int e = max((int)(top >> 21), 64) - 1022;
-  if (threadIdx.x == 0) e_mat[blockIdx.x] = e;
+  const int lane = threadIdx.x & 31;
   __half* m = reinterpret_cast<__half*>(mats + (size_t)blockIdx.x * kBlockMatBytes);
-  for (int i = threadIdx.x; i < kBlockRows * kBlockCols; i += blockDim.x) {
-    const int r = i / kBlockCols, j = i % kBlockCols;
-    uint64_t t = (uint64_t)llrint(scalbn(entry(i), 53 - e));   // 2^53 of the scale
+  for (int r = threadIdx.x >> 5; r < kBlockRows; r += blockDim.x >> 5) {
+    double v[kBlockCols / 32];
+    uint32_t top = 0;
 #pragma unroll
-    for (int d = 0; d < kMatDigits; ++d) t += 256ull << (9 * d);
+    for (int q = 0; q < kBlockCols / 32; ++q) {
+      const int j = lane + 32 * q;
+      v[q] = r < B.rows && j < B.cols ? store[B.base + r * B.s_r + j * B.s_c] : 0.0;
+      top = max(top, (uint32_t)__double2hiint(v[q]) * 2u);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    const int e = max((int)(top >> 21), 64) - 1022;
+    if (lane == 0) e_row[(size_t)blockIdx.x * kBlockRows + r] = e;
 #pragma unroll
-    for (int d = 0; d < kMatDigits; ++d) {
-      const int f9 = (int)((t >> (9 * (kMatDigits - 1 - d))) & (d ? 511 : 1023)) - 256;
-      m[(((size_t)d * (kBlockCols / 8) + j / 8) * kBlockRows + r) * 8 + j % 8] = __float2half((float)f9);
+    for (int q = 0; q < kBlockCols / 32; ++q) {
+      const int j = lane + 32 * q;
+      uint64_t t = (uint64_t)llrint(scalbn(v[q], 53 - e));   // 2^53 of the scale
+#pragma unroll
+      for (int d = 0; d < kMatDigits; ++d) t += 256ull << (9 * d);
+#pragma unroll
+      for (int d = 0; d < kMatDigits; ++d) {
+        const int f9 = (int)((t >> (9 * (kMatDigits - 1 - d))) & (d ? 511 : 1023)) - 256;
+        m[(((size_t)d * (kBlockCols / 8) + j / 8) * kBlockRows + r) * 8 + j % 8] = __float2half((float)f9);
+      }
     }
   }
 }

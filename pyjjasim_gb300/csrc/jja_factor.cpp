@@ -567,6 +567,9 @@ Factor* factor_create(int n, const int64_t* colptr, const int32_t* rowind, const
   }
   F->n_levels = maxlev + 1;
   F->ns = ns;
+  F->mat_ptr.assign(colptr, colptr + n + 1);
+  F->mat_idx.assign(rowind, rowind + colptr[n]);
+  F->mat_val.assign(val, val + colptr[n]);
   return F.release();
 }
 

@@ -26,6 +26,10 @@ struct Factor {
   std::vector<int64_t> sn_valptr;  // ns+1, into fcol
   std::vector<double> fcol;        // F_s blocks, column-major
   std::vector<double> lcol;        // optional: Cholesky columns [L11; L21] (same layout)
+  // the factored matrix itself (both triangles, original order), for residuals
+  std::vector<int64_t> mat_ptr;
+  std::vector<int32_t> mat_idx;
+  std::vector<double> mat_val;
   double factor_flops = 0.0;
   int64_t nnz_L = 0;
 };
