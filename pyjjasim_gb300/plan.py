@@ -316,6 +316,23 @@ def top_leaf(circuit, W):
     return 6144 if W >= 16 else None
 
 
+# Products with explicit inverses (resident steps, dense blocks) are at least as accurate as the sweeps while the
+# junctions' weights in K are within this factor of each other. Error of the phase increments (rms, of the sweeps')
+# at lognormal spreads of the resistances of 1 (factor 200 to 3000) / 2 (1e6) / 3 (1e8): whole inverse of
+# honeycomb 24x24 0.6 / 0.8 / 3.7, leaves of 64x64 0.5 / 0.8 / 6, 10x10 resident 0.4 / 1.0 / 6; one junction of 1e3
+# times the others' resistance on 10x10: 3.3.
+EVEN_WEIGHTS = 256.0
+
+
+def even_weights(circuit, dt):
+    """Whether no junction's weight 1 / (Cv + Rv), nor that plus its inductance, is more than EVEN_WEIGHTS times
+    another's."""
+    w = 1.0 / (np.asarray(circuit._C(), np.float64) / dt ** 2 + 1.0 / (dt * np.asarray(circuit._R(), np.float64)))
+    L = circuit._L()
+    w_L = w + (np.asarray(L.diagonal()) if scipy.sparse.issparse(L) else np.diag(np.asarray(L)))
+    return all(bool(v.min() > 0.0 and v.max() <= EVEN_WEIGHTS * v.min()) for v in (w, w_L))
+
+
 def untuned(tuning):
     """True when ``tuning`` asks for nothing but the level schedule (the library's default)."""
     t = dict(tuning or {})
@@ -493,12 +510,12 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
     (fast_poisson_grid): True (radix-2 grids), False (the sweeps), or "auto": unless ``tuning`` asks for
     sweeps of some shape, whichever of the resident steps (resident_fits), the radix-2 or tensor-core
     transforms, the dense blocks (block_leaf) and the dense top block (top_leaf) is fastest for the circuit
-    and W."""
+    and W (resident steps and blocks for circuits of even_weights only)."""
     fp = sine = blocks = top = None
     matrices = face_matrix(circuit, dt)
     n_faces = circuit._Nf()
     auto = fast_poisson == "auto" and untuned(tuning)
-    resident = auto and resident_fits(circuit, W, stencil_width)
+    resident = auto and resident_fits(circuit, W, stencil_width) and even_weights(circuit, dt)
     if fast_poisson is True or (auto and not resident and radix2_fits(n_faces, W)) or \
             (fast_poisson == "auto" and not auto and W <= FAST_POISSON_MAX_W and W * n_faces <= FAST_POISSON_MAX_WORK):
         fp = fast_poisson_grid(circuit, matrices[1])
@@ -510,6 +527,8 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
         if sine is None:
             blocks = block_leaf(circuit, W)
             top = top_leaf(circuit, W) if blocks is None else None
+            if blocks is not None and not even_weights(circuit, dt):
+                blocks = None
     if blocks is not None:     # the block solver cuts the tree itself: nested dissection with small leaves
         nd_leaf = 8 if nd_leaf is None else nd_leaf
         ordering = "nd" if ordering == "auto" else ordering
