@@ -611,4 +611,37 @@ void factor_solve_host(const Factor& F, double* b, int nrhs) {
     for (int w = 0; w < nrhs; ++w) b[(int64_t)F.perm[i] * nrhs + w] = x[(int64_t)i * nrhs + w];
 }
 
+// K^-1 in the factor's order, row-major, as unevaluated sums hi + lo: the columns by the sweeps above, refined
+// once with residuals in twice the working precision (exact products, two-sums).
+void refined_inverse(const Factor& F, std::vector<double>& hi, std::vector<double>& lo) {
+  const int n = F.n;
+  std::vector<double> x((size_t)n * n, 0.0), r((size_t)n * n);   // original order; column c solves for perm[c]
+  for (int c = 0; c < n; ++c) x[(size_t)F.perm[c] * n + c] = 1.0;
+  factor_solve_host(F, x.data(), n);
+  std::vector<double> s(n), t(n);
+  for (int i = 0; i < n; ++i) {
+    std::fill(s.begin(), s.end(), 0.0);
+    std::fill(t.begin(), t.end(), 0.0);
+    s[F.iperm[i]] = 1.0;
+    for (int64_t q = F.mat_ptr[i]; q < F.mat_ptr[i + 1]; ++q) {   // K is symmetric: its columns are its rows
+      const double a = -F.mat_val[q];
+      const double* v = x.data() + (size_t)F.mat_idx[q] * n;
+      for (int c = 0; c < n; ++c) {
+        const double p = a * v[c], sum = s[c] + p, d = sum - s[c];
+        t[c] += ((s[c] - (sum - d)) + (p - d)) + std::fma(a, v[c], -p);
+        s[c] = sum;
+      }
+    }
+    for (int c = 0; c < n; ++c) r[(size_t)i * n + c] = s[c] + t[c];
+  }
+  factor_solve_host(F, r.data(), n);
+  hi.resize((size_t)n * n);
+  lo.resize((size_t)n * n);
+  for (int i = 0; i < n; ++i)
+    for (int c = 0; c < n; ++c) {
+      hi[(size_t)i * n + c] = x[(size_t)F.perm[i] * n + c];
+      lo[(size_t)i * n + c] = r[(size_t)F.perm[i] * n + c];
+    }
+}
+
 }  // namespace jja

@@ -4221,26 +4221,31 @@ int jja_plan_set_resident(jja_plan* p, const jja_factor* fac) {
     if (!jja_resident_fits(n, p->Nj, p->width))
       throw Error(JJA_ERR_UNFIT, "jja_plan_set_resident: the circuit does not fit one SM");
     SolverSetup setup(p);
-    // the inverse, in the factor's face order, column by column in fixed point
-    std::vector<double> inv((size_t)n * n, 0.0);   // row-major right-hand sides
-    for (int i = 0; i < n; ++i) inv[(size_t)i * n + i] = 1.0;
-    jja::factor_solve_host(F, inv.data(), n);
-    double top = 0.0;
-    for (double v : inv) top = std::max(top, std::fabs(v));
-    if (!(top > 0.0) || !std::isfinite(top)) throw Error(JJA_ERR_NOT_SPD, "jja_plan_set_resident: no finite inverse");
-    int e = 0;
-    std::frexp(top, &e);   // |inv| < 2^e
+    // the inverse, in the factor's face order, column by column in fixed point, a scale per row
+    std::vector<double> hi, lo;
+    jja::refined_inverse(F, hi, lo);
     std::vector<int2> fixed((size_t)n * n);
-    for (int c = 0; c < n; ++c)
-      for (int r = 0; r < n; ++r) {
-        const int64_t v = (int64_t)std::llround(std::ldexp(inv[(size_t)F.perm[r] * n + F.perm[c]], 55 - e));
-        const int lo = (int)((uint32_t)v << (32 - kResHalf)) >> (32 - kResHalf);
-        fixed[(size_t)c * n + r] = make_int2((int)((v - lo) >> kResHalf), lo);
+    std::vector<int> e_row(n);
+    for (int r = 0; r < n; ++r) {
+      double top = 0.0;
+      for (int c = 0; c < n; ++c) {
+        if (!std::isfinite(hi[(size_t)r * n + c]) || !std::isfinite(lo[(size_t)r * n + c]))
+          throw Error(JJA_ERR_NOT_SPD, "jja_plan_set_resident: no finite inverse");
+        top = std::max(top, std::fabs(hi[(size_t)r * n + c]));
       }
+      if (!(top > 0.0)) throw Error(JJA_ERR_NOT_SPD, "jja_plan_set_resident: no finite inverse");
+      std::frexp(top, &e_row[r]);   // |inv| < 2^e
+      for (int c = 0; c < n; ++c) {
+        const int64_t v = (int64_t)std::llround(std::ldexp(hi[(size_t)r * n + c], 55 - e_row[r])) +
+                          (int64_t)std::llround(std::ldexp(lo[(size_t)r * n + c], 55 - e_row[r]));
+        const int half = (int)((uint32_t)v << (32 - kResHalf)) >> (32 - kResHalf);
+        fixed[(size_t)c * n + r] = make_int2((int)((v - half) >> kResHalf), half);
+      }
+    }
     JJA_CUDA(cudaFuncSetAttribute(k_resident, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     ResidentArgs g{};
     g.inv = p->up(fixed.data(), fixed.size());
-    g.e_inv = e;
+    g.e_row = p->up(e_row.data(), e_row.size());
     g.n = n;
     g.nj = p->Nj;
     p->res = g;

@@ -37,5 +37,6 @@ struct Factor {
 Factor* factor_create(int n, const int64_t* colptr, const int32_t* rowind, const double* val,
                       const double* cx, const double* cy, const int32_t* user_perm, const FactorOptions& opt);
 void factor_solve_host(const Factor& F, double* b, int nrhs);
+void refined_inverse(const Factor& F, std::vector<double>& hi, std::vector<double>& lo);
 
 }  // namespace jja

@@ -14,7 +14,13 @@
 // product J = K^-1 b is formed in fixed point: GB300's FP64 pipe does 2 operations per clock and
 // SM, so the n^2 multiply-adds of one 10x10 array would take 1.7 us; 28-bit halves of 56-bit
 // integers multiplied and summed in 64 bits (3 integer multiply-adds per product) take a tenth of
-// that, with an absolute error of 2^-55 max|K^-1| max|b| per term, below an FP64 dot product's.
+// that. The inverse is refined once on the host (residuals in twice the working precision). With
+// 2^e > the largest |K^-1| of the row and 2^f > the largest |b|: the entries of K^-1 are off by at most
+// 2^(e-56), b by 2^(f-56), and the product of two lower halves, which is left out, is below 2^(e+f-56), so a
+// term is off by at most 3 2^(e+f-56) and usually by a tenth of that. Phase increments against long double,
+// error of the Cholesky sweeps' (rms, equal resistances / lognormal spread of 0.4 / of 1): 10x10 0.47 / 0.46 /
+// 0.38, 13x13 0.53 / 0.45 / 0.43; with one scale for the whole inverse, not refined, and b cut instead of
+// rounded 1.09 / 1.13 / 1.44 and 1.10 / 1.09 / 1.60.
 
 namespace {
 
@@ -25,8 +31,8 @@ constexpr int kResChunk = 8192;         // steps per launch (tens of millisecond
 constexpr int kResHalf = 28;            // bits of the lower half of a fixed-point number
 
 struct ResidentArgs {
-  const int2* inv;     // K^-1 by columns, fixed point: (upper, lower half), value = (hi 2^28 + lo) 2^(e_inv - 55)
-  int e_inv;
+  const int2* inv;     // K^-1 by columns, fixed point: (upper, lower half), value = (hi 2^28 + lo) 2^(e - 55)
+  const int* e_row;    // per row: e
   int n, nj, nsteps;
   int64_t step0, src_t0;
   const int64_t* th_slots;   // per step: output slot or -1 (null: none; unused with store_all)
@@ -40,9 +46,9 @@ __host__ __device__ inline size_t resident_smem_bytes(int n, int nj, int nh) {
                                             sizeof(double) + 32 * sizeof(uint32_t);
 }
 
-// x 2^(55 - E) in halves of 28 bits, E = emax - 1022 (see fixed_of)
+// x 2^(55 - E), rounded, in halves of 28 bits, E = emax - 1022 (see fixed_of)
 __device__ __forceinline__ int2 resident_halves(double x, int emax) {
-  const int64_t v = fixed_of(x, emax) >> (61 - 55);
+  const int64_t v = (fixed_of(x, emax) + (1 << 5)) >> (61 - 55);
   const int lo = (int)((uint32_t)v << (32 - kResHalf)) >> (32 - kResHalf);
   return make_int2((int)((v - lo) >> kResHalf), lo);
 }
@@ -82,6 +88,7 @@ __global__ void __launch_bounds__(kResThreads, 2) k_resident(StepArgs a, Tables 
   __syncthreads();
   const int row = tid % rows, slice = tid / rows;
   const int c_lo = slice * per, c_hi = min(n, c_lo + per);
+  const int e_row = tid < n ? __ldg(g.e_row + tid) : 0;
   bool diverged = false;
   for (int i = 0; i < g.nsteps; ++i) {
     const int64_t step = g.step0 + i, tt = step - g.src_t0;
@@ -136,7 +143,7 @@ __global__ void __launch_bounds__(kResThreads, 2) k_resident(StepArgs a, Tables 
         cross += part[(k * n + tid) * 2 + 1];
       }
       const int64_t R = hi + ((cross + (1ll << (kResHalf - 1))) >> kResHalf);   // 2^-54 units
-      J[tid] = emax == 0x7ff ? __longlong_as_double((long long)kNaNBits) : double_of_fixed(R, g.e_inv + emax - 1022 - 1);
+      J[tid] = emax == 0x7ff ? __longlong_as_double((long long)kNaNBits) : double_of_fixed(R, e_row + emax - 1022 - 1);
     }
     __syncthreads();
     const int64_t th_slot = a.store_all ? g.slot0 + i : (g.th_slots ? __ldg(g.th_slots + i) : -1);
