@@ -168,7 +168,11 @@ typedef struct {
 } jja_plan_desc;
 
 /* Uploads the circuit tables and the factor to the current CUDA device and allocates the
- * face-space work vectors for W problems (cudaMalloc). The factor may be destroyed after. */
+ * face-space work vectors for W problems (cudaMalloc). The factor may be destroyed after.
+ * A plan may be used from several threads and streams: calls that work in its vectors (jja_run,
+ * jja_run_timed, jja_solve, jja_solve_static, jja_adjoint_*) follow one another, a call on another stream
+ * waiting on the device for the end of the last one. Inside a stream capture the caller orders them. The
+ * static scratch of jja_solve_static is one per device, for one call at a time. */
 int jja_plan_create(const jja_plan_desc* desc, const jja_factor* f, jja_plan** out);
 void jja_plan_destroy(jja_plan* p);
 /* Bytes of device memory held by the plan (tables + factor + work vectors). */

@@ -2538,9 +2538,15 @@ struct jja_plan {
       if (g.done) cudaEventDestroy(g.done);
     }
     if (fork) cudaEventDestroy(fork);
+    if (used) cudaEventDestroy(used);
     if (res_slots) cudaFree(res_slots);
     for (void* p : allocs) cudaFree(p);
   }
+  // calls on the plan are ordered (PlanUse): the last one's end and its stream
+  std::mutex use;
+  cudaEvent_t used = nullptr;
+  cudaStream_t used_on = nullptr;
+  bool was_used = false;
   int64_t alloc_left = -1;               // bytes that may still be allocated (jja_plan_test_alloc_limit); < 0: any
   void count_alloc(size_t n) {
     if (alloc_left < 0) return;
@@ -2557,6 +2563,29 @@ struct jja_plan {
 };
 
 namespace {
+
+// A call that uses the plan's work vectors (face and junction vectors, source tables, output slots, counters):
+// simulations of one cached plan share them, each from its own stream and maybe thread. The calls follow one
+// another: threads by the mutex, streams by an event at each call's end that a call on another stream waits for.
+// (Every call starts from its caller's state, so any order is right.) A call that is being captured is left to
+// its capturer.
+struct PlanUse {
+  jja_plan* p;
+  cudaStream_t st;
+  std::lock_guard<std::mutex> lock;
+  bool captured;
+  PlanUse(jja_plan* plan, cudaStream_t stream) : p(plan), st(stream), lock(plan->use) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    JJA_CUDA(cudaStreamIsCapturing(st, &cap));
+    captured = cap != cudaStreamCaptureStatusNone;
+    if (!captured && p->was_used && p->used_on != st) JJA_CUDA(cudaStreamWaitEvent(st, p->used, 0));
+  }
+  ~PlanUse() {
+    if (captured || cudaEventRecord(p->used, st) != cudaSuccess) return;
+    p->used_on = st;
+    p->was_used = true;
+  }
+};
 
 // Launch with programmatic stream serialisation (the kernel overlaps its launch with the tail
 // of the previous kernel of the stream; it synchronises itself in pdl_begin), or plainly.
@@ -3834,6 +3863,7 @@ int jja_plan_create(const jja_plan_desc* d, const jja_factor* fac, jja_plan** ou
     p->xj = p->up<double>(nullptr, NjW);
     p->isq = p->up<double>(nullptr, NjW);
     p->amp = p->up<double>(nullptr, Nj);
+    JJA_CUDA(cudaEventCreateWithFlags(&p->used, cudaEventDisableTiming));
     JJA_CUDA(cudaDeviceSynchronize());
     *out = p.release();
   });
@@ -4310,6 +4340,7 @@ int jja_solve(jja_plan* p, const double* b, double* x, void* stream) {
   return guarded([&] {
     if (!p || !b || !x) throw Error(JJA_ERR_ARG, "jja_solve: null argument");
     cudaStream_t st = (cudaStream_t)stream;
+    PlanUse use(p, st);
     const int64_t NfW = (int64_t)p->Nf * p->W;
     k_permute_rows<<<grid_for(NfW, 256), 256, 0, st>>>(b, p->b, p->perm, p->Nf, p->W, fast_div(p->W), 1);
     g_launches++;
@@ -4403,6 +4434,7 @@ int jja_solve_static(jja_plan* p, const double* b, double* x, void* stream) {
                                    " exceeds the static scratch limit of " +
                                    std::to_string(kStaticScratchDoubles / 2) + " (32 MiB for two work vectors)");
     cudaStream_t st = (cudaStream_t)stream;
+    PlanUse use(p, st);
     double* bx = static_scratch_for_current_device(st);   // permuted right-hand side, later the solution
     double* z = bx + NfW;                                // forward-substitution result
     const int32_t* perm = p->perm_factor ? p->perm_factor : p->perm;   // the sweeps' face order
@@ -4438,6 +4470,7 @@ int jja_adjoint_step(jja_plan* p, const jja_adjoint_args* g, void* stream) {
       throw Error(JJA_ERR_ARG, "jja_adjoint_step: missing buffer");
     if ((g->mu_p1 && !g->cos_p1) || (g->mu_p2 && !g->cos_p2))
       throw Error(JJA_ERR_ARG, "jja_adjoint_step: mu of a later step given without its cos(phi)");
+    PlanUse use(p, (cudaStream_t)stream);
     AdjArgs a{};
     a.Nj = p->Nj; a.W = p->W; a.by_W = fast_div(p->W); a.G = g->G;
     a.th_m1 = g->th_m1; a.th_m2 = g->th_m2;
@@ -4458,6 +4491,7 @@ int jja_adjoint_segment(jja_plan* p, const jja_adjoint_segment_args* g, void* st
     if (!g->usum || !g->musum || !g->gIc) throw Error(JJA_ERR_ARG, "jja_adjoint_segment: missing accumulator");
     const int64_t NjW = (int64_t)p->Nj * p->W;
     cudaStream_t st = (cudaStream_t)stream;
+    PlanUse use(p, st);
     auto walk = [&]() {
       for (int64_t i = g->L - 1; i >= 0; --i) {    // steps s0 + L - 1 down to s0
         const int64_t n = g->s0 + i;
@@ -4517,6 +4551,7 @@ int jja_adjoint_flux(jja_plan* p, const double* usum, double* gf, void* stream) 
   return guarded([&] {
     if (!p || !usum || !gf) throw Error(JJA_ERR_ARG, "jja_adjoint_flux: null argument");
     cudaStream_t st = (cudaStream_t)stream;
+    PlanUse use(p, st);
     const int64_t NfW = (int64_t)p->Nf * p->W;
     StepArgs s{};
     s.Nj = p->Nj; s.Nf = p->Nf; s.W = p->W; s.width = p->width; s.w0 = 0; s.wn = p->W; s.by_wn = fast_div(p->W); s.d_step = p->all.d_step;
@@ -4576,6 +4611,7 @@ int jja_run(jja_plan* p, jja_state* s, int nsteps, const int64_t* th_slot, const
     if (nsteps == 0) return;
     check_window(s, nsteps, "jja_run");
     cudaStream_t st = (cudaStream_t)stream;
+    PlanUse use(p, st);
     const std::vector<Group*> gs = step_groups(p);
     set_counters(p, s, st);
     launch_scale_sources(p, s, st);
@@ -4645,6 +4681,7 @@ int jja_run_timed(jja_plan* p, jja_state* s, int nsteps, double* stage_ms, void*
     if (s->noise_mode == JJA_NOISE_BUFFER) throw Error(JJA_ERR_ARG, "jja_run_timed: host noise buffer not supported");
     check_window(s, nsteps, "jja_run_timed");
     cudaStream_t st = (cudaStream_t)stream;
+    PlanUse use(p, st);
     set_counters(p, s, st);
     std::vector<cudaEvent_t> ev(1 + 5 * (size_t)nsteps);
     for (auto& e : ev) JJA_CUDA(cudaEventCreate(&e));
