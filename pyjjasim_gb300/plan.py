@@ -158,9 +158,9 @@ def poisson_grid(circuit, K):
         cx, cy = _face_midpoints(circuit)
     except Exception:
         return None
-    ix, iy = _grid_index(K, cx), _grid_index(K, cy)
-    if ix is None or iy is None:
+    if not (np.isfinite(cx).all() and np.isfinite(cy).all()):
         return None
+    ix, iy = _grid_index(K, cx), _grid_index(K, cy)
     mx, my = int(ix.max()) + 1, int(iy.max()) + 1
     if mx * my != Nf or K.nnz - Nf != 2 * (mx * (my - 1) + my * (mx - 1)):
         return None
@@ -179,16 +179,17 @@ def poisson_grid(circuit, K):
 
 
 def _grid_index(K, v):
-    """Index of every face along one axis of an equally spaced grid (int32), or None; the spacing is the
-    smallest difference between coupled faces (all faces of a column: 0)."""
+    """Index of every face along one axis (int32): on an equally spaced grid from the spacing, the smallest
+    difference between coupled faces (without a sort), else by rank."""
     some = K.indptr[min(K.shape[0], 4096)]
     d = np.abs(v[K.indices[:some]] - v[np.repeat(np.arange(min(K.shape[0], 4096)), np.diff(K.indptr[:4097]))])
     d = d[d > 1e-9]
     lo, h = v.min(), d.min(initial=np.inf)
-    if not np.isfinite(h):
-        return np.zeros(len(v), np.int32) if v.max() - lo <= 1e-9 else None
-    i = np.rint((v - lo) / h)
-    return i.astype(np.int32) if np.abs(v - (lo + i * h)).max() <= 1e-6 * h else None
+    if np.isfinite(h):
+        i = np.rint((v - lo) / h)
+        if np.abs(v - (lo + i * h)).max() <= 1e-6 * h:
+            return i.astype(np.int32)
+    return np.unique(np.round(v, 9), return_inverse=True)[1].astype(np.int32)
 
 
 def _face_midpoints(circuit):

@@ -91,3 +91,29 @@ def test_plan_uses_the_transforms_by_default_for_single_arrays():
     assert sim.plan.fast_poisson
     sim = backend.GpuSimulation(_problem(SquareArray(10, 10), 1, 10))
     assert not sim.plan.fast_poisson
+
+
+def _graded(nx, ny):
+    """A square array drawn on a graded grid: the same circuit, node coordinates at unequal distances."""
+    from pyjjasim_gb300.circuit import Circuit
+    a = SquareArray(nx, ny)
+    x, y = (np.asarray(v, float) for v in a.get_node_coordinates())
+    n1, n2 = a.get_junction_nodes()
+    return Circuit(a.get_cycle_matrix(), node_x=x ** 1.5, node_y=np.exp(0.05 * y), node1=n1, node2=n2,
+                   cut_matrix=a.get_cut_matrix())
+
+
+@pytest.mark.parametrize("nx,ny", [(64, 64), (32, 64), (33, 17), (2, 5)])
+def test_recognises_a_graded_square_array(nx, ny):
+    c = _graded(nx, ny)
+    K = P.face_matrix(c, 0.05)[1]
+    mx, my, grid, kappa = P.poisson_grid(c, K)
+    assert (mx, my) == (nx - 1, ny - 1)
+    # the matrix in grid order is the 5-point Laplacian's
+    Kg = K[grid][:, grid].toarray()
+    lap = 4.0 * np.eye(mx * my)
+    for k in range(mx * my):
+        for m in ([k + 1] if k % mx < mx - 1 else []) + ([k + mx] if k + mx < mx * my else []):
+            lap[k, m] = lap[m, k] = -1.0
+    np.testing.assert_allclose(Kg, kappa * lap, rtol=1e-12, atol=1e-14 * kappa)
+    assert (P.fast_poisson_grid(c, K) is not None) == (nx % 32 == 0)
