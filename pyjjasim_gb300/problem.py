@@ -382,7 +382,7 @@ class TimeEvolutionResult:
         if stored is None or len(sel) == 0:
             return self._select(select_time_points, self.get_circuit()._Nj(), func)
         # one time-major copy, returned as the (Nj, W, T) view
-        return stored.transpose(2, 0, 1)[self._time_point_index(sel)].transpose(1, 2, 0)
+        return stored.transpose(2, 0, 1)[self._time_point_index(sel)].astype(np.double, copy=False).transpose(1, 2, 0)
 
     def get_theta(self, select_time_points=None):
         return self._select_stored(select_time_points, self.theta, self._th)

@@ -63,3 +63,18 @@ def test_problem_validation():
     assert p.get_problem_count() == 7 and p._Is_is_timedep
     with pytest.raises(ValueError):       # the GPU core is the only backend: no CPU fallback
         p.compute(backend="numpy")
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.int64])
+def test_getters_return_double_precision(dtype):
+    """Results made from stored arrays of any type give float64 arrays of their own, of all or of some steps."""
+    from pyjjasim_gb300.problem import TimeEvolutionResult
+    c = SquareArray(3, 3)
+    p = TimeEvolutionProblem(c, time_step_count=4, store_current=True, store_voltage=True)
+    stored = (100 * np.random.default_rng(0).standard_normal((c._Nj(), 1, 4))).astype(dtype)
+    r = TimeEvolutionResult(p, stored, stored, stored)
+    for get in (r.get_theta, r.get_current, r.get_voltage):
+        for select, part in ((None, stored), ([1, 3], stored[:, :, [1, 3]])):
+            got = get(select)
+            assert got.dtype == np.float64 and not np.shares_memory(got, stored)
+            np.testing.assert_array_equal(got, part.astype(np.float64))
