@@ -159,9 +159,16 @@ def _store_cache(path, cache):
     os.replace(tmp, path)
 
 
+# Raised when the default plan's solvers change: an entry holds what was fastest beside the default of its
+# time (a shape of the sweeps chosen before the transforms and blocks came would keep them out: on 512 problems of
+# 128x128 2.6 times the default's time per step).
+SOLVERS = 2
+
+
 def cache_key(device_name, circuit, dt, W, stencil_width, nd_leaf=8):
     A, K = P.face_matrix(circuit, dt)
-    return f"{device_name}|K={P._digest(K.indptr, K.indices, K.data)}|W={W}|width={stencil_width}|leaf={nd_leaf}"
+    return (f"{device_name}|K={P._digest(K.indptr, K.indices, K.data)}|W={W}|width={stencil_width}|leaf={nd_leaf}"
+            f"|solvers={SOLVERS}")
 
 
 def autotune(circuit, dt, W, stencil_width=3, nd_leaf=8, steps=64, use_cache=True, device=None, measure=None,

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from pyjjasim_gb300 import autotune as AT
+from pyjjasim_gb300 import plan as P
 from pyjjasim_gb300.circuit import SquareArray
 
 
@@ -106,3 +107,19 @@ def test_autotune_on_gpu(tmp_path, monkeypatch):
     assert set(opts) == {"ordering", "relax", "tuning"}
     entry, = json.loads((tmp_path / "tune.json").read_text()).values()
     assert entry["seconds_per_step"] <= entry["default_seconds_per_step"]
+
+
+def test_entries_of_other_solvers_are_not_taken(tmp_path, monkeypatch):
+    """A tuning cached beside other default solvers is measured again: with the default the fastest, it stays."""
+    path = tmp_path / "tuning.json"
+    monkeypatch.setenv(AT.CACHE_ENV, str(path))
+    c = SquareArray(12, 12)
+    sweeps = dict(AT.DEFAULT, rows_per_lane=2, relax=[0, 0.0])
+    now = AT.cache_key("fake-gpu", c, 0.05, 4, 3)
+    assert now.endswith(f"|solvers={AT.SOLVERS}")
+    older = now[:now.rindex("|solvers=")]
+    path.write_text(json.dumps({k: {"best": sweeps} for k in (older, older + f"|solvers={AT.SOLVERS - 1}")}))
+    opts = AT.autotune(c, 0.05, 4, measure=lambda cfg: 1.0 if cfg == AT.DEFAULT else 2.0, device_name="fake-gpu")
+    assert opts == AT.to_options(AT.DEFAULT) and P.untuned(opts["tuning"])
+    path.write_text(json.dumps({now: {"best": sweeps}}))
+    assert AT.autotune(c, 0.05, 4, device_name="fake-gpu", measure=lambda cfg: 1.0) == AT.to_options(sweeps)
