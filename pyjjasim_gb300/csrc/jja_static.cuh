@@ -536,7 +536,7 @@ int jja_static_create(const jja_static_desc* d, const jja_factor* fac, jja_stati
     const FaceTables ft = face_tables(Nj, Nf, d->a_rowptr, d->a_col, d->a_val, F.perm);
     set_face_tables(sp->t, ft, [&](auto* h, size_t n) { return sp->up(h, n); });
     {
-      const std::vector<longlong2> tab = build_sin_table();
+      const std::vector<longlong2>& tab = sin_table();
       sp->t.sincos = sp->up(tab.data(), tab.size());
     }
     sp->perm = sp->up(F.perm.data(), F.perm.size());

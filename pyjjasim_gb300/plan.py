@@ -12,6 +12,7 @@ import ctypes
 import hashlib
 import threading
 from collections import OrderedDict
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import scipy.sparse
@@ -20,8 +21,12 @@ from . import _native as N
 
 _FACTORS = OrderedDict()
 _PLANS = OrderedDict()
+_ROUTES = OrderedDict()   # what was asked for -> key of its plan: a kept plan is found without choosing its solver
+_GRIDS = OrderedDict()    # digest of K -> poisson_grid
 MAX_FACTORS = 4
 MAX_PLANS = 4
+MAX_ROUTES = 64
+MAX_GRIDS = 8
 _CACHE_LOCK = threading.Lock()   # the caches are shared by host threads (ragged parts build in parallel);
                                  # the lock covers lookups and insertions, not the factorisations
 
@@ -34,12 +39,26 @@ TUNING_FIELDS = ("rhs_block", "rows_per_lane", "target_warps", "min_piece", "sch
 SCHEDULES = {"levels": 1, "dataflow": 2, "cooperative": 3}
 
 
+_DIGEST_PIECE = 4 << 20   # bytes hashed by one thread (hashlib lets go of the interpreter); 1024x1024: 250 -> 40 ms
+
+
 def _digest(*arrays):
+    """Digest of the arrays' types, shapes and contents, in pieces of a fixed size (large ones by several threads)."""
     h = hashlib.blake2b(digest_size=16)
+    pieces = []
     for a in arrays:
         a = np.ascontiguousarray(a)
         h.update(str(a.dtype).encode() + str(a.shape).encode())
-        h.update(a.view(np.uint8).ravel() if a.size else b"")
+        flat = a.view(np.uint8).ravel() if a.size else np.empty(0, np.uint8)
+        pieces += [flat[k:k + _DIGEST_PIECE] for k in range(0, len(flat), _DIGEST_PIECE)]
+    one = lambda piece: hashlib.blake2b(piece, digest_size=16).digest()
+    if len(pieces) > len(arrays):
+        with ThreadPoolExecutor(8) as pool:
+            parts = list(pool.map(one, pieces))
+    else:
+        parts = map(one, pieces)
+    for part in parts:
+        h.update(part)
     return h.hexdigest()
 
 
@@ -154,6 +173,9 @@ def poisson_grid(circuit, K):
         return None
     if np.count_nonzero(np.abs(K.data + kappa) <= tol) != K.nnz - Nf:
         return None
+    grid = _numbered_grid(circuit, K)
+    if grid is not None:
+        return grid + (kappa,)
     try:
         cx, cy = _face_midpoints(circuit)
     except Exception:
@@ -176,6 +198,57 @@ def poisson_grid(circuit, K):
     if np.count_nonzero(along | (step == mx) | (step == 0)) != K.nnz:
         return None
     return mx, my, grid, kappa
+
+
+def _numbered_grid(circuit, K):
+    """(mx, my, grid_face) when the faces are numbered line by line (as SquareArray numbers them), from the
+    pattern of K alone but for the two faces that tell x from y; else None. 1024x1024: 110 -> 20 ms."""
+    Nf = K.shape[0]
+    first = K.indices[:K.indptr[1]]     # sorted: face 0, the next one of its line, the next line's
+    if not (len(first) == 3 and first[0] == 0 and first[1] == 1):
+        return None
+    m = int(first[2])
+    lines = Nf // m
+    if m < 2 or lines * m != Nf or K.nnz - Nf != 2 * (lines * (m - 1) + (lines - 1) * m):
+        return None
+    i = np.arange(Nf, dtype=K.indices.dtype)
+    at = np.empty((Nf, 5), K.indices.dtype)
+    there = np.ones((Nf, 5), bool)
+    for k, step in enumerate((-m, -1, 0, 1, m)):
+        np.add(i, K.indices.dtype.type(step), out=at[:, k])
+    there[:m, 0] = there[-m:, 4] = False
+    there[::m, 1] = there[m - 1::m, 3] = False
+    count = np.full(Nf, 5, K.indptr.dtype)
+    count[:m] -= 1
+    count[-m:] -= 1
+    count[::m] -= 1
+    count[m - 1::m] -= 1
+    if not (np.array_equal(np.diff(K.indptr), count) and np.array_equal(at[there], K.indices)):
+        return None
+    try:
+        x, y = (np.asarray(v, np.float64) for v in circuit.get_node_coordinates())
+        n1, n2 = circuit.get_junction_nodes()
+        A = scipy.sparse.csc_matrix(circuit.get_cycle_matrix())
+
+        def middle(f):   # mean of the junction midpoints of face f
+            j = np.searchsorted(A.indptr, np.flatnonzero(A.indices == f), side="right") - 1
+            return 0.5 * np.array([(v[n1[j]] + v[n2[j]]).mean() for v in (x, y)])
+
+        along, across = middle(1) - middle(0), middle(m) - middle(0)
+    except Exception:    # no node coordinates
+        return None
+    cell = np.arange(Nf, dtype=np.int32).reshape(lines, m)
+    for axis in (0, 1):   # the lines along x, or along y
+        if abs(along[axis]) > 1e-9 and abs(along[1 - axis]) <= 1e-9 and \
+                abs(across[1 - axis]) > 1e-9 and abs(across[axis]) <= 1e-9:
+            if along[axis] < 0.0:
+                cell = cell[:, ::-1]
+            if across[1 - axis] < 0.0:
+                cell = cell[::-1]
+            if axis == 0:
+                return m, lines, np.ascontiguousarray(cell).ravel()
+            return lines, m, np.ascontiguousarray(cell.T).ravel()
+    return None
 
 
 def _grid_index(K, v):
@@ -208,9 +281,25 @@ def _face_midpoints(circuit):
         return np.asarray(cx, np.float64), np.asarray(cy, np.float64)
 
 
-def fast_poisson_grid(circuit, K):
-    """``poisson_grid`` for the radix-2 transforms: mx + 1 and my + 1 powers of two, up to 1024."""
+def _kept_grid(circuit, K, digest):
+    """poisson_grid, kept by the digest of K (a grid holds for every circuit with that K; that none was found may
+    be for want of coordinates, and is not kept)."""
+    with _CACHE_LOCK:
+        if digest in _GRIDS:
+            _GRIDS.move_to_end(digest)
+            return _GRIDS[digest]
     g = poisson_grid(circuit, K)
+    if g is not None:
+        with _CACHE_LOCK:
+            _GRIDS[digest] = g
+            while len(_GRIDS) > MAX_GRIDS:
+                _GRIDS.popitem(last=False)
+    return g
+
+
+def fast_poisson_grid(circuit, K, digest=None):
+    """``poisson_grid`` for the radix-2 transforms: mx + 1 and my + 1 powers of two, up to 1024."""
+    g = poisson_grid(circuit, K) if digest is None else _kept_grid(circuit, K, digest)
     return None if g is None or any(m + 1 > 1024 or (m + 1) & m for m in g[:2]) else g
 
 
@@ -245,8 +334,8 @@ def radix2_fits(n_faces, W):
     return 2048 <= n_faces <= 1 << 17 and W <= (1 if n_faces < 8192 else 4 if n_faces < 1 << 15 else 3)
 
 
-def sine_solver_fits(grid, W):
-    """Whether "auto" takes the tensor-core sine transforms for W problems on this poisson_grid."""
+def sine_solver_fits(grid):
+    """Whether "auto" takes the tensor-core sine transforms on this poisson_grid (for any number of problems)."""
     mx, my = grid[:2]
     return SINE_MIN_SIDE <= min(mx, my) and max(mx, my) <= SINE_MAX_SIDE
 
@@ -484,10 +573,10 @@ def fill_reducing_order(K, ordering, circuit=None):
     raise ValueError(f"ordering must be 'nd' or 'mmd', not {ordering!r}")
 
 
-def get_factor(circuit, dt, nd_leaf=8, ordering="nd", relax=(-1, -1.0), matrices=None):
-    """(factor, A, cache key); ``matrices``: face_matrix(circuit, dt) when the caller has it."""
+def get_factor(circuit, dt, nd_leaf=8, ordering="nd", relax=(-1, -1.0), matrices=None, digest=None):
+    """(factor, A, cache key); ``matrices``: face_matrix(circuit, dt), ``digest``: of its K, when the caller has them."""
     A, K = face_matrix(circuit, dt) if matrices is None else matrices
-    key = (_digest(K.indptr, K.indices, K.data), nd_leaf, ordering, tuple(relax))
+    key = (_digest(K.indptr, K.indices, K.data) if digest is None else digest, nd_leaf, ordering, tuple(relax))
     with _CACHE_LOCK:
         hit = _FACTORS.get(key)
         if hit is not None:
@@ -512,18 +601,31 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
     sweeps of some shape, whichever of the resident steps (resident_fits), the radix-2 or tensor-core
     transforms, the dense blocks (block_leaf) and the dense top block (top_leaf) is fastest for the circuit
     and W (resident steps and blocks for circuits of even_weights only)."""
-    fp = sine = blocks = top = None
-    matrices = face_matrix(circuit, dt)
+    matrices = A, K = face_matrix(circuit, dt)
+    digest = _digest(K.indptr, K.indices, K.data)
     n_faces = circuit._Nf()
+    Rv, Cv, coef = coefficients(circuit, dt, stencil)
+    if Ic_w is not None:
+        Ic_w = np.ascontiguousarray(np.broadcast_to(np.asarray(Ic_w, np.float64), (circuit._Nj(), W)))
+    ic = np.asarray(circuit._Ic(), np.float64) if Ic_w is None else Ic_w
+    tkey = tuple(int((tuning or {}).get(f, 0)) for f in TUNING_FIELDS)
+    tables = (W, stencil_width, Ic_w is None, tkey, _digest(ic, *coef, Rv, A.indptr, A.indices, A.data))
+    asked = (digest, nd_leaf, ordering, tuple(relax), fast_poisson, getattr(circuit, "components", 1)) + tables
+    with _CACHE_LOCK:
+        p = _PLANS.get(_ROUTES.get(asked))
+        if p is not None:
+            _PLANS.move_to_end(_ROUTES[asked])
+            return p
+    fp = sine = blocks = top = None
     auto = fast_poisson == "auto" and untuned(tuning)
     resident = auto and resident_fits(circuit, W, stencil_width) and even_weights(circuit, dt)
     if fast_poisson is True or (auto and not resident and radix2_fits(n_faces, W)) or \
             (fast_poisson == "auto" and not auto and W <= FAST_POISSON_MAX_W and W * n_faces <= FAST_POISSON_MAX_WORK):
-        fp = fast_poisson_grid(circuit, matrices[1])
+        fp = fast_poisson_grid(circuit, K, digest)
     if auto and not resident and fp is None:
         if W * n_faces > SINE_FROM_WORK or n_faces > SINE_FROM_FACES:
-            sine = poisson_grid(circuit, matrices[1])
-            if sine is not None and not sine_solver_fits(sine, W):
+            sine = _kept_grid(circuit, K, digest)
+            if sine is not None and not sine_solver_fits(sine):
                 sine = None
         if sine is None:
             blocks = block_leaf(circuit, W)
@@ -533,31 +635,30 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
     if blocks is not None:     # the block solver cuts the tree itself: nested dissection with small leaves
         nd_leaf = 8 if nd_leaf is None else nd_leaf
         ordering = "nd" if ordering == "auto" else ordering
-    ordering = resolve_ordering(ordering, W, circuit._Nf())
-    nd_leaf, relax = resolve_factor_shape(nd_leaf, relax, ordering, W, circuit._Nf())
-    factor, A, fkey = get_factor(circuit, dt, nd_leaf, ordering=ordering, relax=relax, matrices=matrices)
-    Rv, Cv, coef = coefficients(circuit, dt, stencil)
-    if Ic_w is not None:
-        Ic_w = np.ascontiguousarray(np.broadcast_to(np.asarray(Ic_w, np.float64), (circuit._Nj(), W)))
-    ic = np.asarray(circuit._Ic(), np.float64) if Ic_w is None else Ic_w
-    tkey = tuple(int((tuning or {}).get(f, 0)) for f in TUNING_FIELDS)
-    key = (fkey, W, stencil_width, Ic_w is None, tkey, fp is not None, sine is not None, resident, blocks, top,
-           _digest(ic, *coef, Rv, A.indptr, A.indices, A.data))
+    ordering = resolve_ordering(ordering, W, n_faces)
+    nd_leaf, relax = resolve_factor_shape(nd_leaf, relax, ordering, W, n_faces)
+    factor, A, fkey = get_factor(circuit, dt, nd_leaf, ordering=ordering, relax=relax, matrices=matrices, digest=digest)
+    key = (fkey, fp is not None, sine is not None, resident, blocks, top) + tables
     with _CACHE_LOCK:
         p = _PLANS.get(key)
         if p is not None:
             _PLANS.move_to_end(key)
-            return p
-    p = DevicePlan(circuit, factor, A, W, dt, stencil_width, stencil, Ic_w=Ic_w, tuning=tuning, fast_poisson=fp,
-                   sine=sine, resident=resident, blocks=blocks, top=top)
+    if p is None:
+        p = DevicePlan(circuit, factor, A, W, dt, stencil_width, stencil, Ic_w=Ic_w, tuning=tuning, fast_poisson=fp,
+                       sine=sine, resident=resident, blocks=blocks, top=top)
     with _CACHE_LOCK:
         _PLANS[key] = p
+        _ROUTES[asked] = key
         while len(_PLANS) > MAX_PLANS:
             _PLANS.popitem(last=False)
+        while len(_ROUTES) > MAX_ROUTES:
+            _ROUTES.popitem(last=False)
     return p
 
 
 def clear_cache():
     with _CACHE_LOCK:
         _PLANS.clear()
+        _ROUTES.clear()
         _FACTORS.clear()
+        _GRIDS.clear()
