@@ -323,10 +323,16 @@ FAST_POISSON_MAX_WORK = 1 << 18
 #   256x256  W = 1   44 / 115 / -      W = 4  124 / 103 / -
 # so: dense blocks up to SINE_FROM_WORK face-problems on up to SINE_FROM_FACES faces, tensor-core
 # transforms above, radix-2 transforms for a few problems on power-of-two grids.
+# The sums of blocks (of the separators between strips too) are added atomically in any order, as the sweeps' split
+# dot products are; the transforms repeat bit for bit. So power-of-two grids within FAST_POISSON_MAX_WORK keep
+# transforms there, also where the others take less time (radix-2 / others: 32x32 W = 1 20 / 10, W = 8 22 / 12; 64x64
+# W = 8 25 / 24; 256x256 W = 4 119 / 100; 512x512 W = 1 133 / 150); from 8192 faces in one strip, where radix2_fits
+# ends, the tensor-core ones (128x128 W = 8 60 / 48).
 SINE_FROM_WORK = 150000
 SINE_FROM_FACES = 1 << 14
 SINE_MIN_SIDE = 8
 SINE_MAX_SIDE = 4096
+SINE_ONE_STRIP = 128     # a side up to which no strips are cut
 
 
 def radix2_fits(n_faces, W):
@@ -632,6 +638,13 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
             top = top_leaf(circuit, W) if blocks is None else None
             if blocks is not None and not even_weights(circuit, dt):
                 blocks = None
+        repeats = sine is not None and min(sine[:2]) <= SINE_ONE_STRIP
+        if not repeats and W <= FAST_POISSON_MAX_W and W * n_faces <= FAST_POISSON_MAX_WORK:
+            grid = fast_poisson_grid(circuit, K, digest)
+            if grid is not None:
+                blocks = top = None
+                strips = min(grid[:2]) > SINE_ONE_STRIP
+                fp, sine = (grid, None) if strips or n_faces < 8192 else (None, grid)
     if blocks is not None:     # the block solver cuts the tree itself: nested dissection with small leaves
         nd_leaf = 8 if nd_leaf is None else nd_leaf
         ordering = "nd" if ordering == "auto" else ordering

@@ -1,4 +1,4 @@
-"""Which solver the default plan takes, where that is decided by accuracy."""
+"""Which solver the default plan takes, where accuracy or repeatability decides."""
 import numpy as np
 import pytest
 
@@ -44,3 +44,38 @@ def test_uneven_circuits_keep_the_sweeps(make, even):
     assert (sim.plan.resident or sim.plan.blocks is not None) == even and not sim.plan.sine and sim.plan.top is None
     if not even:
         assert backend.GpuSimulation(prob, fast_poisson=False).plan is sim.plan
+
+
+# nodes, problems, solver: power-of-two grids of few problems had the radix-2 transforms, whose runs repeat bit for bit
+REPEATS = [(16, 16, 1, "fast_poisson"), (32, 32, 1, "fast_poisson"), (32, 32, 8, "fast_poisson"),
+           (64, 32, 3, "fast_poisson"), (64, 64, 2, "fast_poisson"), (64, 64, 8, "fast_poisson"),
+           (256, 256, 4, "fast_poisson"), (512, 512, 1, "fast_poisson"), (128, 128, 8, "sine"), (10, 10, 8, "resident")]
+
+
+@pytest.mark.parametrize("nx,ny,W,solver", REPEATS)
+def test_power_of_two_grids_of_few_problems_take_what_repeats(monkeypatch, nx, ny, W, solver):
+    asked = {}
+    monkeypatch.setattr(P, "HostFactor", lambda *a, **k: None)
+    monkeypatch.setattr(P, "DevicePlan", lambda *a, **k: asked.update(k))
+    P.clear_cache()
+    P.get_plan(SquareArray(nx, ny), 0.05, W, 3, ((1.0, -1.0, 0.0), (1.0, -2.0, 1.0)))
+    P.clear_cache()
+    assert [k for k in ("fast_poisson", "sine", "resident", "blocks", "top") if asked[k] not in (None, False)] == [solver]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,W,solver", REPEATS)
+def test_their_runs_repeat_bit_for_bit(nx, ny, W, solver):
+    import torch
+    base = np.zeros((nx - 1) * ny + nx * (ny - 1))
+    base[:(nx - 1) * ny] = 1.0
+    prob = TimeEvolutionProblem(SquareArray(nx, ny), time_step=0.05, time_step_count=30, external_flux=0.1,
+                                current_sources=base[:, None, None] * np.linspace(0.3, 1.5, W)[None, :, None])
+    sim = backend.GpuSimulation(prob)
+    start, first = [h.clone() for h in sim.history()], None
+    for _ in range(4):
+        sim.set_history(start, 0)
+        sim.run(30)
+        sim.synchronize()
+        first = sim.theta().clone() if first is None else first
+        assert torch.equal(sim.theta(), first)
