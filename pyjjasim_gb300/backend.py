@@ -229,12 +229,12 @@ class GpuSimulation:
                 from .autotune import autotune
                 opts = autotune(c, stage.dt, self.W, self.width, nd_leaf=nd_leaf, device=self.dev.index)
                 ordering, relax, tuning = opts["ordering"], opts["relax"], opts["tuning"]
-            self.ordering = P.resolve_ordering(ordering, self.W, self.Nf)
             self.relax, self.tuning = tuple(relax), dict(tuning or {})
             self.stream = stream if stream is not None else torch.cuda.Stream(device=self.dev)
             self.plan = P.get_plan(c, stage.dt, self.W, self.width, stage.stencil, nd_leaf=nd_leaf,
                                    ordering=ordering, relax=relax, Ic_w=Ic, tuning=tuning,
                                    fast_poisson=fast_poisson)
+            self.ordering = self.plan.ordering
             self.hist0, self.hist0_zero = stage.hist0, stage.hist0_zero
             self.hist = []
             with torch.cuda.stream(self.stream):

@@ -659,6 +659,7 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
     if p is None:
         p = DevicePlan(circuit, factor, A, W, dt, stencil_width, stencil, Ic_w=Ic_w, tuning=tuning, fast_poisson=fp,
                        sine=sine, resident=resident, blocks=blocks, top=top)
+        p.ordering = ordering     # the order its factor has
     with _CACHE_LOCK:
         _PLANS[key] = p
         _ROUTES[asked] = key

@@ -114,3 +114,15 @@ def test_digests_tell_contents_types_and_shapes_apart(monkeypatch):
         d = P._digest(*other)
         assert d not in seen
         seen.add(d)
+
+
+@pytest.mark.parametrize("make,W,ordering,want", [
+    (lambda: HoneycombArray(24, 24), 4096, "auto", "nd"),     # blocks, with more work than minimum degree is taken from
+    (lambda: HoneycombArray(24, 24), 4096, "mmd", "mmd"), (lambda: SquareArray(90, 90), 600, "auto", "mmd"),
+    (lambda: SquareArray(9, 9), 1, "auto", "nd")])
+def test_a_plan_says_the_order_of_its_factor(counted, monkeypatch, make, W, ordering, want):
+    got = []
+    order = P.fill_reducing_order
+    monkeypatch.setattr(P, "fill_reducing_order", lambda K, o, c=None: got.append(o) or order(K, o, c))
+    p = P.get_plan(make(), 0.05, W, 3, STENCIL, ordering=ordering)
+    assert p.ordering == want and got == [want]

@@ -1,4 +1,6 @@
 """Which solver the default plan takes, where accuracy or repeatability decides."""
+import types
+
 import numpy as np
 import pytest
 
@@ -56,7 +58,7 @@ REPEATS = [(16, 16, 1, "fast_poisson"), (32, 32, 1, "fast_poisson"), (32, 32, 8,
 def test_power_of_two_grids_of_few_problems_take_what_repeats(monkeypatch, nx, ny, W, solver):
     asked = {}
     monkeypatch.setattr(P, "HostFactor", lambda *a, **k: None)
-    monkeypatch.setattr(P, "DevicePlan", lambda *a, **k: asked.update(k))
+    monkeypatch.setattr(P, "DevicePlan", lambda *a, **k: types.SimpleNamespace(asked=asked.update(k)))
     P.clear_cache()
     P.get_plan(SquareArray(nx, ny), 0.05, W, 3, ((1.0, -1.0, 0.0), (1.0, -2.0, 1.0)))
     P.clear_cache()
