@@ -398,16 +398,34 @@ def block_leaf(circuit, W):
     return 384 if W >= 8 and n <= 1 << 16 else None
 
 
+# Unions of many trees: the smallest subtrees whose separators' blocks (12 bytes an entry, read once a step; entries as
+# the sum of the trees' squared sizes) fit the L2 cache. Larger sums spill: sweeps / subtrees of 384 / 768 / 1536 / 3072 /
+# 6144, us per step of one problem, at a sum of
+#   3.9e8  148 / 105 / 115 / 125 / 135 / 143      6.1e8  151 / 170 / 132 / 134 / 144 / 145
+#   8.6e8  158 / 181 / 135 / 135 / 144 / 152      1.1e9  144 / 187 / 118 / 124 / 131 / 131
+#   1.36e9 161 / 202 / 165 / 131 / 138 / 146      2.5e9  180 / 230 / 236 / 223 / 184 / 179
+# Beyond the table subtrees of 6144 gain from some 160000 faces (250558 faces 338 -> 319) and nothing below.
+UNION_LEAVES = ((384, 5.5e8), (768, 1.15e9), (1536, 1.4e9))
+UNION_LARGE = 160_000
+
+
+def tree_sizes(circuit):
+    """Faces of the trees of the circuit's elimination forest: of a ragged union its circuits', else one tree."""
+    n = circuit._Nf()
+    components = getattr(circuit, "components", 1)
+    return getattr(circuit, "tree_faces", None) or (n // components,) * components
+
+
 def top_leaf(circuit, W):
     """The subtree size below which the default plan keeps the sweeps when block_leaf takes none (a
     product solves the faces above), or None."""
-    n = circuit._Nf()
-    tree = n // getattr(circuit, "components", 1)   # a ragged union's circuits are trees of their own
+    n, trees = circuit._Nf(), tree_sizes(circuit)
     if n > 1 << 19:
         return None
-    if tree < n and tree <= 6144:
-        return 384 if n <= 100_000 else None
-    if tree <= 1 << 17:
+    if len(trees) > 1 and max(trees) <= 1 << 17:
+        squares = sum(t * t for t in trees)
+        return next((leaf for leaf, most in UNION_LEAVES if squares <= most), 6144 if n > UNION_LARGE else None)
+    if max(trees) <= 1 << 17:
         return 768 if n <= 1 << 15 else 3072 if n <= 1 << 16 else 6144
     return 6144 if W >= 16 else None
 
@@ -616,7 +634,7 @@ def get_plan(circuit, dt, W, stencil_width, stencil, nd_leaf=None, ordering="aut
     ic = np.asarray(circuit._Ic(), np.float64) if Ic_w is None else Ic_w
     tkey = tuple(int((tuning or {}).get(f, 0)) for f in TUNING_FIELDS)
     tables = (W, stencil_width, Ic_w is None, tkey, _digest(ic, *coef, Rv, A.indptr, A.indices, A.data))
-    asked = (digest, nd_leaf, ordering, tuple(relax), fast_poisson, getattr(circuit, "components", 1)) + tables
+    asked = (digest, nd_leaf, ordering, tuple(relax), fast_poisson, tree_sizes(circuit)) + tables
     with _CACHE_LOCK:
         p = _PLANS.get(_ROUTES.get(asked))
         if p is not None:

@@ -153,6 +153,7 @@ class RaggedBatch:
                                node_x=np.concatenate(xs), node_y=np.concatenate(ys), node1=np.concatenate(n1s),
                                node2=np.concatenate(n2s))
         self.circuit.components = len(A_blocks)
+        self.circuit.tree_faces = tuple(int(A.shape[0]) for A in A_blocks)
 
     def _union_source(self, getter_name, timedep_name, rows):
         """Concatenate one source over all (problem, w) copies: array (N, 1, 1) or callable."""

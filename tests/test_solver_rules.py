@@ -81,3 +81,29 @@ def test_their_runs_repeat_bit_for_bit(nx, ny, W, solver):
         sim.synchronize()
         first = sim.theta().clone() if first is None else first
         assert torch.equal(sim.theta(), first)
+
+
+@pytest.mark.parametrize("trees,leaf", [
+    ([3353] * 12, 384), ([14520] + [5006] * 10, 384),                         # sums of squares below 5.5e8
+    ([14520, 14520] + [3949] * 9, 768), ([17030, 15000, 12000] + [2635] * 15, 768), ([23256, 16000] + [6157] * 5, 768),
+    ([29756, 15000] + [3277] * 10, 1536), ([27060, 25000, 20000] + [5539] * 10, None), ([11444] * 24, 6144),
+    ([200_000, 30_000], None)])                                               # a tree above 2^17: by its size alone
+def test_a_unions_top_block_by_its_trees(trees, leaf):
+    """The separators' blocks of a union are read once a step: the rule keeps them within the L2 cache, whatever
+    the trees' mean (one large lattice among small ones counts by its square)."""
+    class Union:
+        components, tree_faces = len(trees), tuple(trees)
+
+        def _Nf(self):
+            return sum(trees)
+
+    assert P.top_leaf(Union(), 1) == leaf
+
+
+def test_a_ragged_batch_says_its_trees():
+    from pyjjasim_gb300.ragged import RaggedBatch
+    circuits = [SquareArray(4, 5), HoneycombArray(3, 3), SquareArray(7, 3)]
+    Is = [np.zeros((c._Nj(), 2, 1)) for c in circuits]
+    probs = [TimeEvolutionProblem(c, time_step=0.05, time_step_count=3, current_sources=i) for c, i in zip(circuits, Is)]
+    u = RaggedBatch(probs).circuit
+    assert sorted(P.tree_sizes(u)) == sorted(2 * [c._Nf() for c in circuits]) and sum(P.tree_sizes(u)) == u._Nf()
