@@ -409,6 +409,17 @@ UNION_LEAVES = ((384, 5.5e8), (768, 1.15e9), (1536, 1.4e9))
 UNION_LARGE = 160_000
 
 
+# One tree and few problems, likewise (sweeps / 3072 / 6144 / 12288 / 24576, us per step):
+#   45369 faces  W = 1 136 / 113 / 120 / 128 / 136                     53536  W = 1 144 / 172 / 117 / 122 / 131
+#   56355        W = 2 146 / 179 / 160 / 125 /  -   W = 4 192 / 183 / 174 / 162
+#   65025        W = 1 148 / 187 / 151 / 125 / 134  W = 7 242 / 218 / 207 / 215 / 226
+#   68121        W = 1 148 / 200 / 155 / 153 / 136  W = 7 249 / 230 / 218 / 222 / 226
+#   89401        W = 1 182 / 197 / 189 / 187 / 175  W = 7 295 / 253 / 250 / 262 / 270
+#   128881       W = 1 275 / 243 / 236 / 234 / 243  W = 16 583 / 516 / 514 / 524 / 542
+#   358801       W = 16 1348 / 1425 / 1240 / 1212   488601  W = 16 1862 / - / 1967 / 1722   W = 48 6502 / - / 5792
+SINGLE_LEAVES = ((46_000, 3072), (54_000, 6144), (66_000, 12288), (100_000, 24576))
+
+
 def tree_sizes(circuit):
     """Faces of the trees of the circuit's elimination forest: of a ragged union its circuits', else one tree."""
     n = circuit._Nf()
@@ -425,9 +436,13 @@ def top_leaf(circuit, W):
     if len(trees) > 1 and max(trees) <= 1 << 17:
         squares = sum(t * t for t in trees)
         return next((leaf for leaf, most in UNION_LEAVES if squares <= most), 6144 if n > UNION_LARGE else None)
+    if n <= 1 << 15:
+        return 768
+    if n <= 100_000 and W < 8:
+        return next(leaf for most, leaf in SINGLE_LEAVES if n <= most) if n <= 66_000 or W < 4 else 6144
     if max(trees) <= 1 << 17:
-        return 768 if n <= 1 << 15 else 3072 if n <= 1 << 16 else 6144
-    return 6144 if W >= 16 else None
+        return 3072 if n <= 1 << 16 else 6144
+    return 6144 if W >= (16 if n <= 400_000 else 32) else None
 
 
 # Products with explicit inverses (resident steps, dense blocks) are at least as accurate as the sweeps while the

@@ -192,3 +192,15 @@ def test_phase_increments_are_as_accurate_as_the_sweeps(lattice, nx, ny, leaf, t
     rms = [float(np.sqrt((((A.T @ (v - exact).astype(np.float64)) / c0) ** 2).mean())) for v in (x, y)]
     print(f"increments: {rms[0]:.2e}, sweeps {rms[1]:.2e}")
     assert rms[0] <= 1.05 * rms[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,W,top", [(262, 262, 2, 24576), (240, 235, 3, 12288)])
+def test_top_block_over_large_subtrees(nx, ny, W, top):
+    c = SquareArray(nx, ny)
+    rng = np.random.default_rng(nx)
+    c.set_resistance(rng.lognormal(0.0, 0.2, c._Nj()))
+    b = rng.standard_normal((c._Nf(), W))
+    x, K = _solve(c, b, None, top)
+    ref = scipy.sparse.linalg.spsolve(K.tocsc(), b)
+    assert np.abs(x - ref).max() <= 1e-11 * np.abs(ref).max()

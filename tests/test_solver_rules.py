@@ -107,3 +107,15 @@ def test_a_ragged_batch_says_its_trees():
     probs = [TimeEvolutionProblem(c, time_step=0.05, time_step_count=3, current_sources=i) for c, i in zip(circuits, Is)]
     u = RaggedBatch(probs).circuit
     assert sorted(P.tree_sizes(u)) == sorted(2 * [c._Nf() for c in circuits]) and sum(P.tree_sizes(u)) == u._Nf()
+
+
+@pytest.mark.parametrize("n,W,leaf", [
+    (32768, 1, 768), (32769, 1, 3072), (46000, 7, 3072), (46001, 1, 6144), (54000, 7, 6144), (54001, 2, 12288), (66000, 7, 12288),
+    (66001, 1, 24576), (100000, 3, 24576), (66001, 4, 6144), (100001, 1, 6144), (1 << 17, 1, 6144), (60000, 512, 3072),
+    (200000, 8, None), (200000, 16, 6144), (400001, 16, None), (400001, 32, 6144), ((1 << 19) + 1, 64, None)])
+def test_a_single_trees_top_block(n, W, leaf):
+    class One:
+        def _Nf(self):
+            return n
+
+    assert P.top_leaf(One(), W) == leaf
