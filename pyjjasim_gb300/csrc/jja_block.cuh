@@ -16,6 +16,9 @@
 // The blocks come from the plan's own factor by sweeps over parts of its tree with columns of the
 // identity (jja_plan_set_blocks). Each row of a block has its own scale.
 //
+// The products of the blocks side by side are added atomically, in any order: runs repeat to rounding, not bit for
+// bit, as with the sweeps' split dot products.
+//
 // Measured (GB300, us per step with the sweeps -> with these products): honeycomb 24x24 x 61 problems
 // 99 -> 24, triangular 64x48 with spread resistances x 96 240 -> 134, one such array 89 -> 33. A unit
 // (128 x 64 block, 64 problems) takes about 12k cycles on its SM: 1.5k reading and splitting the data,
@@ -27,7 +30,6 @@ namespace {
 
 constexpr int kBlockRows = 128, kBlockCols = 64;
 constexpr int kBlockThreads = 512;
-constexpr int kDenseMaxFaces = 4096;      // the whole inverse: 12 bytes per entry
 constexpr int kBlocksMax = 1 << 15;       // blocks of a plan: 3 GB of digits
 constexpr int kBlockMatBytes = kMatDigits * kBlockRows * kBlockCols * 2;   // 96 KB of digits per block
 

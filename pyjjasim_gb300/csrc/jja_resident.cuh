@@ -6,7 +6,7 @@
 // hundred FP64 operations (SquareArray(10,10): 15.6 us a step replayed from graphs, 40 us when
 // every step is stored and the launches are issued one by one).
 //
-// Measured: 10x10, one problem, 2000 steps with every step stored, 81 -> 24 ms per call, 3.4 us a
+// Measured: 10x10, one problem, 2000 steps with every step stored, 81 -> 11 ms per call, 3.2 us a
 // step; 64 problems 24.8 -> 3.2 us, 512 problems 25.7 -> 8.2 us a step (64 registers per thread:
 // two blocks per SM; one block measured 12.1).
 //
@@ -25,9 +25,9 @@
 namespace {
 
 constexpr int kResMaxFaces = 160;       // K^-1 in shared memory: 8 bytes x 160^2 = 200 KB
-constexpr int kResMaxJunctions = 1024;
+constexpr int kResMaxJunctions = 1024;  // two a thread; the default plan's rule stops at 512
 constexpr int kResThreads = 512;
-constexpr int kResChunk = 8192;         // steps per launch (tens of milliseconds at most)
+constexpr int kResChunk = 8192;         // steps per launch (26 ms for one 10x10 array, 160 ms for 512 of 13x13)
 constexpr int kResHalf = 28;            // bits of the lower half of a fixed-point number
 
 struct ResidentArgs {

@@ -23,7 +23,8 @@
 //
 // Measured (GB300, the face solve of a step; the sweeps they replace -> these kernels): 128x128 x
 // 512 problems 850 -> 195 us (70 us per transform, 56 us for the chains: 43 us of FP64 work), 101x60 x
-// 24 178 -> 31 us; an adjoint run on 64x64 x 64 121 -> 48 ms; 1024x1024 x 8 (8 strips) 1976 -> 510 us:
+// 24 178 -> 31 us; an adjoint run on 64x64 x 64 121 -> 46 ms (critical currents that the
+// plan has not seen: 181 -> 52); 1024x1024 x 8 (8 strips) 1976 -> 510 us:
 // 77 us per transform, 108 and 159 us for the two passes over the chains (72 and 100 us of FP64 work),
 // 30 us for the edges, 44 us for the separators. A tile (128 columns of 127 faces) takes about 30k
 // cycles: reading and splitting 6k, twice the products 3.8k (3.5k of MMA issue at the multipliers' rate)

@@ -674,7 +674,9 @@ int jja_static_create(const jja_static_desc* d, const jja_factor* fac, jja_stati
         if (ci < 4) {
           L.smem = (size_t)nfmax * nfmax * sizeof(double);
           // warps hide the latency of shared memory and of the FP64 pipe: top fronts of 64x64 (94 rows), two
-          // launches, 420 -> 344 us with 16 warps instead of 8; 64 problems 15.1 -> 14.6 ms
+          // launches, 420 -> 344 us with 16 warps instead of 8. Whole solves in ms, 2 / 4 / 8 warps (lines at 32 and 64
+          // rows) -> these: 64x64 x 64 14.9 -> 14.3, x 1 5.3 -> 4.9, 40x40 x 8 3.7 -> 3.4, 72x50 x 16 6.5 -> 6.1, 100x100 x 4
+          // 13.4 -> 12.1, triangular 40x30 x 16 6.95 -> 6.87, honeycomb 24x24 x 32 45.8 -> 45.8
           L.threads = nfmax <= 32 ? 64 : (nfmax <= 48 ? 128 : (nfmax <= 72 ? 256 : 512));
         }
         gmax = std::max(gmax, L.gl_total);

@@ -347,9 +347,10 @@ def sine_solver_fits(grid):
 
 
 # Circuits whose state and inverse fit one SM run whole calls in one launch, a block per problem, while
-# the problems need at most a few rounds of blocks. Measured on GB300 (us per step, one launch per call /
-# launches per step): 5x5 nodes W = 1 2.4 / 12.2; 10x10 W = 64 3.2 / 24.8, W = 512 8.2 / 25.7, W = 1024
-# 14.5 / 27.0; 13x13 W = 152 5.0 / 25.5, W = 512 19.4 / 27.2, W = 1024 34.1 / 32.6
+# the problems need few rounds of blocks (304 a round). Measured on GB300 (us per step, one launch per call /
+# dense inverse / sweeps): 5x5 nodes W = 1 2.3 / 8.6 / 11.6, W = 512 5.3 / 11.4 / 15.8; 10x10 W = 64 3.2 / 10.9 / 19.3,
+# W = 512 8.1 / 12.5 / 39.4, W = 1024 14.5 / 13.3 / 41.4; 13x13 W = 152 5.0 / 11.8 / 31.3, W = 304 10.0 / 12.6 / 57.4,
+# W = 512 19.4 / 14.8 / 58.8: the largest circuits are past the crossing with the dense inverse there, the others not
 RESIDENT_MAX_FACES = 160
 RESIDENT_MAX_JUNCTIONS = 512
 RESIDENT_MAX_W = 512

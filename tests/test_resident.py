@@ -1,8 +1,7 @@
 """Whole runs of small circuits in one launch (jja_plan_set_resident) against the oracle and the sweeps.
 
 The trajectory bars are those of the other paths (1e-9 relative against the oracle, 1e-10 between
-solvers): one face-space product is off by at most n 2^-55 of max|K^-1| max|b|, below an FP64 dot
-product's bound for n <= 160 terms."""
+solvers); the product's error bound stands in csrc/jja_resident.cuh, its size beside the sweeps' is tested here."""
 import numpy as np
 import pytest
 
@@ -154,3 +153,28 @@ def test_steps_are_as_accurate_as_the_sweeps(lattice, nx, ny, sigma):
         rms.append(float(np.sqrt(((sim.theta().cpu().numpy() - exact) ** 2).mean())))
     print(f"step: {rms[0]:.2e}, sweeps {rms[1]:.2e}")
     assert rms[0] <= rms[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("steps", [50, 60000])
+def test_output_slots_are_read_before_the_call_returns(steps):
+    """The caller may reuse its slot arrays at once, also while earlier steps are still running."""
+    import torch
+    c = SquareArray(4, 4)
+    prob = TimeEvolutionProblem(c, time_step=0.05, time_step_count=200000, external_flux=0.1,
+                                current_sources=0.5 * c.current_base(0.0)[:, None, None])
+    want = None
+    for overwrite in (False, True):
+        sim = backend.GpuSimulation(prob)
+        assert sim.plan.resident
+        out = torch.zeros((5, c._Nj(), 1), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        slots = np.full(steps, -1, np.int64)
+        slots[::steps // 5] = np.arange(5)
+        sim.run(100000)          # a quarter of a second of steps before them
+        sim.run(steps, th_slot=slots, th_dev=out)
+        if overwrite:
+            slots[:] = -1
+        sim.synchronize()
+        want = out.clone() if want is None else want
+        assert torch.equal(out, want) and float(out.abs().min(dim=1).values.max()) > 0.0
