@@ -166,6 +166,10 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_block_apply(BlockList L, d
       __syncwarp();
     }
     const BlockUnit now = U;
+    const int row = tid & (kBlockRows - 1);   // of the join; where it goes is read ahead of the wait
+    const bool live = row < now.out_cnt;
+    double* dst = (now.from == 1 ? b : x) + (live ? (int64_t)__ldg(L.out_rows + now.out_off + row) * W : 0) + w_lo;
+    const int e_row = __ldg(L.e_row + now.mat * kBlockRows + row);
     if (u + (int)gridDim.x < L.n) {
       U = L.units[u + gridDim.x];
       load(U);
@@ -177,10 +181,6 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_block_apply(BlockList L, d
       bulk_load(smem_addr(mat), L.mats + (size_t)U.mat * kBlockMatBytes, kBlockMatBytes, smem_addr(mbar + 1));
     phase ^= 1u;
     // join (see k_sine_lines); warp quadrant = 32 rows, quarter of the problems per group of 4 warps
-    const int row = tid & (kBlockRows - 1);
-    const bool live = row < now.out_cnt;
-    double* dst = (now.from == 1 ? b : x) + (live ? (int64_t)__ldg(L.out_rows + now.out_off + row) * W : 0) + w_lo;
-    const int e_row = __ldg(L.e_row + now.mat * kBlockRows + row);
     const uint32_t lane_base = tmem + ((uint32_t)((tid >> 5) & 3) << 21);
 #pragma unroll 1
     for (int blk = 0; blk < wp / 16; ++blk) {
