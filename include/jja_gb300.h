@@ -222,6 +222,11 @@ int jja_plan_set_blocks(jja_plan* p, const jja_factor* f, int leaf_faces);
  * plan's sweeps fuse (jja_solve_tuning.subtree_rows). jja_solve_static keeps the whole sweeps. */
 int jja_plan_set_top_block(jja_plan* p, const jja_factor* f, int leaf_faces);
 
+/* For tests: polls after which a wait for copies or products in the tensor-core kernels gives up (negative: the
+ * default). With 0 every such wait does: the kernels report it (jja_plan_check), wait for what is in flight and end.
+ * Steps that were captured before keep their limit. */
+int jja_plan_test_product_wait_limit(jja_plan* p, int polls);
+
 /* For tests: device allocations of the plan beyond `bytes` more fail as they do when memory runs out
  * (negative: no limit). Nothing is allocated for it. */
 int jja_plan_test_alloc_limit(jja_plan* p, int64_t bytes);

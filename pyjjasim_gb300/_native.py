@@ -111,6 +111,7 @@ SIGNATURES = {
     "jja_plan_set_blocks": (c_int, [c_void_p, c_void_p, c_int]),
     "jja_plan_set_top_block": (c_int, [c_void_p, c_void_p, c_int]),
     "jja_plan_check": (c_int, [c_void_p, ctypes.POINTER(c_int)]),
+    "jja_plan_test_product_wait_limit": (c_int, [c_void_p, c_int]),
     "jja_plan_test_alloc_limit": (c_int, [c_void_p, c_int64]),
     "jja_plan_test_wait_limit": (c_int, [c_void_p, c_void_p]),
     "jja_run": (c_int, [c_void_p, ctypes.POINTER(State), c_int, P_i64, P_i64, c_int, c_void_p]),

@@ -46,7 +46,7 @@ struct BlockList {
   const int32_t* out_rows = nullptr;
   const unsigned char* mats = nullptr;   // per block: digit, 8-column group, row, column
   const int* e_row = nullptr;            // per block and row of it: |entry| < 2^e
-  int n = 0;
+  int n = 0, spin = kMmaSpinLimit;
 };
 
 __host__ __device__ __forceinline__ uint32_t block_tmem_cols(int wp) { return wp <= 16 ? 128 : (wp <= 32 ? 256 : 512); }
@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_block_apply(BlockList L, d
     *gave_up = 0;
     if (u < L.n) bulk_load(smem_addr(mat), L.mats + (size_t)L.units[u].mat * kBlockMatBytes, kBlockMatBytes, smem_addr(mbar + 1));
   }
+  int copies = u < L.n ? 1 : 0, batches = 0;   // of blocks, started by thread 0; of products, by warp 0
   BlockUnit U{};
   if (u < L.n) {
     U = L.units[u];
@@ -112,7 +113,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_block_apply(BlockList L, d
   const uint32_t tmem = *tmem_slot;
   uint32_t phase = 0;
   auto wait = [&](uint64_t* bar, uint32_t parity) {
-    if (!*gave_up && !mbar_wait(smem_addr(bar), parity)) {
+    if (!*gave_up && !mbar_wait(smem_addr(bar), parity, L.spin)) {
       *gave_up = 1;
       atomicExch(err, 1);
     }
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_block_apply(BlockList L, d
     for (int e = 0; e < 8; ++e) top = max(top, (uint32_t)__double2hiint(A[e]) * 2u);
     if (kg < groups) colmax[kg * wp + dw] = top;
     __syncthreads();
+    if (*gave_up) break;   // the same for all: no wait lies between the last barrier and this one
     if (kg < groups) {
 #pragma unroll
       for (int k = 0; k < groups; ++k) top = max(top, colmax[k * wp + dw]);
@@ -146,7 +148,9 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_block_apply(BlockList L, d
       tmem_fence_after();
       constexpr uint32_t lbo_a = kBlockRows * 16, lbo_b = kDatDigits * wp * 16;
       const uint64_t a0 = mma_desc(smem_addr(mat), lbo_a, 128), b0 = mma_desc(smem_addr(dat), lbo_b, 128);
-      if (elect_one()) {
+      const bool go = !__any_sync(0xffffffffu, *gave_up);
+      batches += go;
+      if (elect_one() && go) {
         // block digit i times the data digits [j0, j0 + nj): accumulators i + j0 ...
         auto mma = [&](int i, int j0, int nj, int ks) {
           mma_f16(tmem + (uint32_t)((i + j0) * wp), a0 + (uint32_t)((i * groups + 2 * ks) * lbo_a >> 4),
@@ -177,15 +181,18 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_block_apply(BlockList L, d
     wait(mbar, phase);
     __syncwarp();
     tmem_fence_after();
-    if (tid == 0 && u + (int)gridDim.x < L.n)   // every product has read the block
+    const bool ok = !__any_sync(0xffffffffu, *gave_up);
+    if (tid == 0 && u + (int)gridDim.x < L.n && ok) {   // every product has read the block
       bulk_load(smem_addr(mat), L.mats + (size_t)U.mat * kBlockMatBytes, kBlockMatBytes, smem_addr(mbar + 1));
+      ++copies;
+    }
     phase ^= 1u;
     // join (see k_sine_lines); warp quadrant = 32 rows, quarter of the problems per group of 4 warps
     const uint32_t lane_base = tmem + ((uint32_t)((tid >> 5) & 3) << 21);
 #pragma unroll 1
     for (int blk = 0; blk < wp / 16; ++blk) {
       const int n0 = (tid >> 7) * (wp / 4) + blk * 4;
-      if (n0 >= live_w) break;   // the same for the whole warp
+      if (n0 >= live_w || !ok) break;   // the same for the whole warp
       float P[kDatDigits][4];
       tmem_load_digits(lane_base + (uint32_t)n0, (uint32_t)wp, P);
 #pragma unroll
@@ -203,6 +210,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_block_apply(BlockList L, d
       }
     }
   }
+  if (tid == 0 && *gave_up) mbar_drain(mbar, copies, batches);
   tmem_fence_before();
   __syncthreads();
   if (tid < 32) {

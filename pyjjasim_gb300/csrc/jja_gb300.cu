@@ -4296,6 +4296,16 @@ int jja_plan_test_alloc_limit(jja_plan* p, int64_t bytes) {
   });
 }
 
+int jja_plan_test_product_wait_limit(jja_plan* p, int polls) {
+  return guarded([&] {
+    if (!p) throw Error(JJA_ERR_ARG, "jja_plan_test_product_wait_limit: null plan");
+    const int spin = polls < 0 ? kMmaSpinLimit : polls;
+    for (auto& c : p->sine) c.fwd.spin = c.bwd.spin = spin;
+    for (BlockList& L : p->blocks) L.spin = spin;
+    p->sep_dst.spin = spin;
+  });
+}
+
 int jja_plan_test_wait_limit(jja_plan* p, void* stream) {
   return guarded([&] {
     if (!p) throw Error(JJA_ERR_ARG, "jja_plan_test_wait_limit: null plan");

@@ -44,7 +44,7 @@ constexpr int kSineColumns = 128;              // (line, problem) columns per ti
 constexpr int kSineThreads = 512;
 // TMEM columns of the 7 accumulators of kp columns each (a power of two is allocated)
 __host__ __device__ __forceinline__ uint32_t sine_tmem_cols(int kp) { return kp <= 16 ? 128 : (kp <= 32 ? 256 : 512); }
-constexpr int64_t kMmaSpinLimit = 1LL << 24;   // try_wait polls; far beyond any MMA batch (~3 us)
+constexpr int kMmaSpinLimit = 1 << 24;   // try_wait polls; far beyond any MMA batch (~3 us)
 
 // one transform direction: m points a line, `lines` lines, element (line, t, w) at
 // line * s_c + t * s_t + w; half lengths padded to kp (a multiple of 16)
@@ -56,6 +56,7 @@ struct SineArgs {
   int parts;            // blocks a tile of columns is shared by: 1, 2 (odd, even modes) or 2 x mode chunks
   const unsigned char* mat;   // digits of the odd and even half matrices in the MMA operand layout
   int e_shift;          // result exponent offset (the power-of-two part of the scale)
+  int spin = kMmaSpinLimit;
 };
 
 struct SineTri {
@@ -110,9 +111,10 @@ __device__ __forceinline__ bool elect_one() {
   return one != 0;
 }
 
-// bounded wait for the mbarrier's phase; false when the bound ran out
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
-  for (int64_t i = 0; i < kMmaSpinLimit; ++i) {
+// bounded wait for the mbarrier's phase; false when the bound ran out. A kernel whose wait ran out reports it,
+// starts no further copies or products, and waits again (drain) for those in flight before it gives its memory back.
+__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, int limit) {
+  for (int i = 0; i < limit; ++i) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -205,6 +207,12 @@ __device__ __forceinline__ void digits_of(const int64_t* X, uint4* out) {
   }
 }
 
+// before a kernel whose wait ran out ends: the last of its copies (counted on mbar[1]) and batches of products (mbar[0])
+__device__ __forceinline__ void mbar_drain(uint64_t* mbar, int copies, int batches) {
+  if (copies) mbar_wait(smem_addr(mbar + 1), (uint32_t)(copies - 1) & 1u, kMmaSpinLimit);
+  if (batches) mbar_wait(smem_addr(mbar), (uint32_t)(batches - 1) & 1u, kMmaSpinLimit);
+}
+
 // `bytes` (a multiple of 16) from global to shared memory, counted on the mbarrier
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
@@ -287,11 +295,12 @@ __global__ void __launch_bounds__(kSineThreads, 1) k_sine_lines(SineArgs d, cons
   const uint32_t tmem = *tmem_slot;
   uint32_t phase = 0;
   auto wait = [&](uint64_t* bar, uint32_t parity) {
-    if (!*gave_up && !mbar_wait(smem_addr(bar), parity)) {
+    if (!*gave_up && !mbar_wait(smem_addr(bar), parity, d.spin)) {
       *gave_up = 1;
       atomicExch(err, 1);
     }
   };
+  int batches = 0;                   // of products, started by warp 0
   if (tid == 0) wait(mbar + 1, 0);   // only the MMA issuer reads the matrix
   __syncwarp();
   while (tile < tiles) {
@@ -314,6 +323,7 @@ __global__ void __launch_bounds__(kSineThreads, 1) k_sine_lines(SineArgs d, cons
         top = max(top, max((uint32_t)(A[r][e] >> 32) * 2u, (uint32_t)(B[r][e] >> 32) * 2u));
     colmax[q4 * kSineColumns + col] = top;
     __syncthreads();
+    if (*gave_up) break;   // the same for all: no wait lies between the last barrier and this one
 #pragma unroll
     for (int q = 0; q < 4; ++q) top = max(top, colmax[q * kSineColumns + col]);
     const int emax = max((int)(top >> 21), 64);
@@ -352,7 +362,9 @@ __global__ void __launch_bounds__(kSineThreads, 1) k_sine_lines(SineArgs d, cons
         constexpr uint32_t lbo_a = kSineColumns * 16, lbo_b = kMatDigits * kp * 16;
         const uint64_t a0 = mma_desc(smem_addr(dat), lbo_a, 128);
         const uint64_t b0 = mma_desc(smem_addr(mat) + (uint32_t)parity * mat_bytes, lbo_b, 128);
-        if (elect_one()) {
+        const bool go = !__any_sync(0xffffffffu, *gave_up);
+        batches += go;
+        if (elect_one() && go) {
           auto mma = [&](int j, int i0, int ni, int ks, bool add) {
             mma_f16(tmem + (uint32_t)((i0 + j) * kp), a0 + (uint32_t)((j * groups + 2 * ks) * lbo_a >> 4),
                     b0 + (uint32_t)((2 * ks * lbo_b + i0 * kp * 16) >> 4), mma_idesc(ni * kp), add ? 1u : 0u);
@@ -384,6 +396,7 @@ __global__ void __launch_bounds__(kSineThreads, 1) k_sine_lines(SineArgs d, cons
       // 2^-54 of the line's scale. Warp quadrant = 32 columns, q4 = a quarter of the modes
       const uint32_t lane_base = tmem + ((uint32_t)((tid >> 5) & 3) << 21);
       const int count = parity ? half : m - half;
+      if (__any_sync(0xffffffffu, *gave_up)) continue;
       for (int blk = 0; blk < (nc >> 4); ++blk) {
         const int n0 = q4 * (nc >> 2) + blk * 4;
         float P[kDatDigits][4];
@@ -405,6 +418,7 @@ __global__ void __launch_bounds__(kSineThreads, 1) k_sine_lines(SineArgs d, cons
     }
     tile = next;
   }
+  if (tid == 0 && *gave_up) mbar_drain(mbar, 1, batches);
   tmem_fence_before();
   __syncthreads();
   if (tid < 32) {

@@ -42,3 +42,33 @@ def test_infinite_initial_phase_is_reported():
     with pytest.raises(N.JJAError) as e:
         _problem(c, Is, config_at_minus_1=th, config_at_minus_2=th).compute(use_graph=True)
     assert e.value.code == 4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("solver", ["sine", "strips", "blocks", "top"])
+def test_a_product_wait_that_runs_out_is_reported(solver):
+    """Waits for copies and products in the tensor-core kernels, made to give up at once: the kernels report it, wait for
+    what they have in flight and end, and the plan then solves as before."""
+    import torch
+    from pyjjasim_gb300 import plan as P
+    c = SquareArray(150, 140) if solver == "strips" else SquareArray(40, 30)
+    factor, A, _ = P.get_factor(c, 0.05)
+    option = {"blocks": dict(blocks=128), "top": dict(top=300)}.get(
+        solver, dict(sine=P.poisson_grid(c, P.face_matrix(c, 0.05)[1])))
+    W = 20
+    pl = P.DevicePlan(c, factor, A, W, 0.05, 3, ((1.0, -1.0, 0.0), (1.0, -2.0, 1.0)), **option)
+    b = torch.from_numpy(np.random.default_rng(2).standard_normal((c._Nf(), W))).cuda()
+    x = torch.empty_like(b)
+    want = factor.solve_host(b.cpu().numpy())
+    torch.cuda.synchronize()
+    for polls in (-1, 0, -1):
+        N.check(N.lib().jja_plan_test_product_wait_limit(pl.handle, polls))
+        pl.solve(b.data_ptr(), x.data_ptr(), 0)
+        torch.cuda.synchronize()
+        if polls == 0:
+            with pytest.raises(N.JJAError) as e:
+                pl.check()
+            assert e.value.code == 5 and "ran out" in str(e.value)
+        else:
+            pl.check()
+            assert np.abs(x.cpu().numpy() - want).max() <= 1e-11 * np.abs(want).max()
