@@ -399,16 +399,17 @@ def block_leaf(circuit, W):
     return 384 if W >= 8 and n <= 1 << 16 else None
 
 
-# Unions of many trees: the smallest subtrees whose separators' blocks (12 bytes an entry, read once a step; entries as
-# the sum of the trees' squared sizes) fit the L2 cache. Larger sums spill: sweeps / subtrees of 384 / 768 / 1536 / 3072 /
-# 6144, us per step of one problem, at a sum of
-#   3.9e8  148 / 105 / 115 / 125 / 135 / 143      6.1e8  151 / 170 / 132 / 134 / 144 / 145
-#   8.6e8  158 / 181 / 135 / 135 / 144 / 152      1.1e9  144 / 187 / 118 / 124 / 131 / 131
-#   1.36e9 161 / 202 / 165 / 131 / 138 / 146      2.5e9  180 / 230 / 236 / 223 / 184 / 179
-# Beyond the table subtrees of 6144 gain from some 160000 faces (250558 faces 338 -> 319) and nothing below.
-UNION_LEAVES = ((384, 5.5e8), (768, 1.15e9), (1536, 1.4e9))
-UNION_LARGE = 160_000
-
+# Unions of many trees: the smallest subtrees with which a step's data stay within the L2 cache: some 0.77 kB a face
+# (the sweeps' factor and vectors) and the separators' blocks, 12 bytes an entry or 85 MB x 384 / leaf per 1e9 of the
+# trees' squared sizes. us per step of one problem, sweeps / 384 / 768 / 1536 / 3072 / 6144 / 12288 (the sum of squares):
+#   35636 faces (0.54e9) 148 / 98 / 106 / 115 / 126 / 134 / 143      64600 (0.70e9) 157 / 154 / 125 / 133 / 134 / 143 / 152
+#   61929 (1.45e9) 156 / 192 / 175 / 126 / 134 / 142 / 152            82859 (1.98e9) 158 / 196 / 192 / 175 / 135 / 153 / 155
+#   103317 (1.81e9) 168 / 224 / 221 / 191 / 158 / 152 / 168           111999 (1.42e9) 189 / 228 / 225 / 186 / 172 / 186 / 170
+# Where none does, a product still pays for large trees (126470 faces, mean 9033: 212 / - / - / 228 / 214 / 197 / 188; 263822,
+# mean 10147: 345 / - / - / 310 / 332 / 331 / 329), not for small ones (118320, mean 4732: 168 / - / - / 191 / 181 / 188 / 199).
+UNION_LEAVES = (384, 768, 1536, 3072, 6144, 12288)
+UNION_CACHE = 90.0       # MB
+UNION_LARGE_TREES = 6144
 
 # One tree and few problems, likewise (sweeps / 3072 / 6144 / 12288 / 24576, us per step):
 #   45369 faces  W = 1 136 / 113 / 120 / 128 / 136                     53536  W = 1 144 / 172 / 117 / 122 / 131
@@ -436,7 +437,10 @@ def top_leaf(circuit, W):
         return None
     if len(trees) > 1 and max(trees) <= 1 << 17:
         squares = sum(t * t for t in trees)
-        return next((leaf for leaf, most in UNION_LEAVES if squares <= most), 6144 if n > UNION_LARGE else None)
+        for leaf in UNION_LEAVES:
+            if 0.77e-3 * n + 85e-9 * squares * 384 / leaf <= UNION_CACHE:
+                return leaf
+        return None if n // len(trees) <= UNION_LARGE_TREES else 12288 if n < 150_000 else 6144
     if n <= 1 << 15:
         return 768
     if n <= 100_000 and W < 8:

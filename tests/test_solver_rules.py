@@ -84,10 +84,10 @@ def test_their_runs_repeat_bit_for_bit(nx, ny, W, solver):
 
 
 @pytest.mark.parametrize("trees,leaf", [
-    ([3353] * 12, 384), ([14520] + [5006] * 10, 384),                         # sums of squares below 5.5e8
-    ([14520, 14520] + [3949] * 9, 768), ([17030, 15000, 12000] + [2635] * 15, 768), ([23256, 16000] + [6157] * 5, 768),
-    ([29756, 15000] + [3277] * 10, 1536), ([27060, 25000, 20000] + [5539] * 10, None), ([11444] * 24, 6144),
-    ([200_000, 30_000], None)])                                               # a tree above 2^17: by its size alone
+    ([3353] * 12, 384), ([14520] + [5006] * 10, 384), ([14520, 14520] + [3949] * 9, 768),   # equal means, larger squares
+    ([34782] + [3878] * 7, 1536), ([34782, 20000] + [4679] * 6, 3072), ([29756, 25000] + [4856] * 10, 6144),
+    ([25122, 20000] + [2675] * 25, 12288), ([14520] * 4 + [2868] * 21, None), ([34782, 30000] + [5140] * 12, 12288),
+    ([11444] * 24, 6144), ([200_000, 30_000], None)])                                       # a tree above 2^17: by its size alone
 def test_a_unions_top_block_by_its_trees(trees, leaf):
     """The separators' blocks of a union are read once a step: the rule keeps them within the L2 cache, whatever
     the trees' mean (one large lattice among small ones counts by its square)."""
